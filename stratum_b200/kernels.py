@@ -375,9 +375,20 @@ def linear_simple(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
         raise KernelError(f"linear: epilogue {epilogue} writes {want}, out is {out.dtype}")
     f = _fn("linear_simple", "stratum_linear_simple",
             [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-             c_void_p])
+             c_void_p, c_void_p])
+    scratch = _linear_simple_scratch(x, 1, M, N, K)
     _check(f(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), dtype_code(x.dtype), epilogue, M, N, K, x.stride(0),
-             out.stride(0), act, _stream()), "linear_simple")
+             out.stride(0), act, _ptr(scratch), _stream()), "linear_simple")
+
+
+def _linear_simple_scratch(x: torch.Tensor, heads: int, M: int, N: int, K: int) -> Optional[torch.Tensor]:
+    """What a float32 product of more rows than tiles adds its segments' sums through (None: it needs nothing)."""
+    if x.dtype != torch.float32:
+        return None
+    f = build.load("linear_simple").stratum_linear_simple_scratch
+    f.restype = ctypes.c_longlong
+    floats = f(heads, M, N, K)
+    return torch.empty(floats, dtype=torch.float32, device=x.device) if floats else None
 
 
 def linear_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, x_step: int, o_step: int) -> None:
@@ -389,9 +400,10 @@ def linear_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, x_step: in
     heads, N, Kd = w.shape
     f = _fn("linear_simple", "stratum_linear_heads",
             [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-             c_void_p])
+             c_void_p, c_void_p])
+    scratch = _linear_simple_scratch(x, heads, x.shape[0], N, Kd)
     _check(f(_ptr(x), _ptr(w), _ptr(out), dtype_code(x.dtype), EPI_STORE, heads, x.shape[0], N, Kd, x.stride(0),
-             out.stride(0), x_step, o_step, _stream()), "linear_heads")
+             out.stride(0), x_step, o_step, _ptr(scratch), _stream()), "linear_heads")
 
 
 def head_gemm_ok(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, x_step: int, o_step: int) -> bool:

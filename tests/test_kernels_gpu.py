@@ -130,6 +130,49 @@ def test_linear_simple(dtype, M, N, K_):
     assert torch.equal(one[0], out32[M - 1])
 
 
+@pytest.mark.parametrize("N,K_", [(130, 2048), (2048 + 5, 260), (70, 2051), (257, 2100)])
+def test_linear_simple_float32_sums_have_one_order(N, K_):
+    """Rows alone, few rows, tiles of 32 and of 64 rows, whole and cut along k, rows that no 16-byte copy can start on:
+    a row's sums are the same bits in all of them, and as near to 64 bits as sqrt(K) roundings are."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(N + K_)
+    x = dev(rng.standard_normal((301, K_)))
+    w = dev(rng.standard_normal((N, K_)) * 0.1)
+    b = dev(rng.standard_normal(N))
+    ref = P.linear(as64(x), as64(w), as64(b))
+    want = torch.empty(301, N, device="cuda")
+    K.linear_simple(x, w, b, want, K.EPI_STORE)
+    assert rel_err(as64(want), ref) < 2e-6
+    assert np.linalg.norm(as64(want) - ref) / np.linalg.norm(ref) < 2.0 ** -24 * math.sqrt(K_ / 2) * 0.5
+    pitched = torch.zeros(301, K_ + 3, device="cuda")
+    pitched[:, :K_] = x
+    for rows in (1, 2, 3, 8, 9, 32, 33, 64, 65, 300):
+        for start in (0, 301 - rows):
+            out = torch.empty(rows, N, device="cuda")
+            K.linear_simple(x[start:start + rows].contiguous(), w, b, out, K.EPI_STORE)
+            assert torch.equal(out, want[start:start + rows]), (rows, start)
+            K.linear_simple(pitched[start:start + rows, :K_], w, b, out, K.EPI_STORE_F32)
+            assert torch.equal(out, want[start:start + rows]), (rows, start)
+            base = torch.ones(rows, N + 2, device="cuda")
+            K.linear_simple(x[start:start + rows].contiguous(), w, None, base[:, :N], K.EPI_ADD_F32)
+            plain = torch.empty(rows, N, device="cuda")
+            K.linear_simple(x[start:start + rows].contiguous(), w, None, plain, K.EPI_STORE)
+            assert torch.equal(base[:, :N], 1.0 + plain) and torch.equal(base[:, N:], torch.ones(rows, 2, device="cuda"))
+
+
+@pytest.mark.parametrize("rows", [1, 5, 20, 70])
+def test_linear_heads_float32(rows):
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(rows)
+    x = dev(rng.standard_normal((rows, 3 * 600)))
+    w = dev(rng.standard_normal((3, 40, 300)) * 0.1)
+    out = torch.empty(rows, 3 * 50, device="cuda")
+    K.linear_heads(x, w, out, 600, 50)
+    for j in range(3):
+        ref = as64(x[:, 600 * j:600 * j + 300]) @ as64(w[j]).T
+        assert rel_err(as64(out[:, 50 * j:50 * j + 40]), ref) < 2e-6
+
+
 @pytest.mark.parametrize("M", [1, 5, 8, 13, 16, 32])
 @pytest.mark.parametrize("N,K_", [(48, 64), (1000, 200), (4096 + 16, 4096), (2 * 177, 96)])
 def test_gemm_skinny(M, N, K_):
