@@ -434,6 +434,37 @@ def test_attention_simple(dtype, n_q, n_kv, hd):
     assert rel_err(as64(out), c["ref"]) < (3e-6 if dtype == "float32" else 8e-3)
 
 
+@pytest.mark.parametrize("n_q,n_kv,hd,window", [(8, 2, 64, 0), (6, 2, 64, 100), (3, 3, 128, 0), (8, 1, 128, 70),
+                                                (12, 1, 64, 0)])
+def test_attention_simple_float32_by_pages(n_q, n_kv, hd, window):
+    """Heads of 64 and 128 in float32: tiles of rows and one token a cluster give the same bits, at the edges of pages,
+    with a window, over several sequences in one tile; nothing that lies behind a token's position reaches it."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(hd + n_q)
+    before, new = [0, 63, 64, 700, 130], [130, 1, 65, 3, 40]
+    c = _attention_case(rng, before, new, n_q, n_kv, hd, "float32", window=window)
+    args = (n_q, n_kv, hd, 64, window, 1.0 / math.sqrt(hd))
+    out = torch.zeros(c["T"], n_q * hd, device="cuda")
+    K.attention_simple(c["qkv"], c["kc"], c["vc"], c["pos"], c["seq"], c["table"], out, *args)
+    assert rel_err(as64(out), c["ref"]) < 3e-6
+    # a few tokens at a time, with a padding token among them
+    for rows in ([0], [62, 63, 64, 65], [129, 130, 131], list(range(186, 200)), list(range(199, 216))):
+        pick = torch.tensor(rows + [0], device="cuda")
+        seq = c["seq"][pick].clone()
+        seq[-1] = -1
+        few = torch.zeros(len(rows) + 1, n_q * hd, device="cuda")
+        K.attention_simple(c["qkv"][pick].contiguous(), c["kc"], c["vc"], c["pos"][pick].contiguous(), seq, c["table"],
+                           few, *args)
+        assert torch.equal(few[:-1], out[pick[:-1]]) and not few[-1].any(), rows
+    # the last sequence's last key and value become NaN: only its last token sees them
+    last, page = before[-1] + new[-1] - 1, int(c["table"][4, (before[-1] + new[-1] - 1) // 64])
+    c["kc"][page, :, last % 64:] = float("nan")
+    c["vc"][page, :, last % 64:] = float("nan")
+    again = torch.zeros_like(out)
+    K.attention_simple(c["qkv"], c["kc"], c["vc"], c["pos"], c["seq"], c["table"], again, *args)
+    assert torch.equal(again[:-1], out[:-1]) and bool(torch.isnan(again[-1]).all())
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_attention_finds_one_far_key_among_hundreds(dtype):
     """Scale one query and one key so that a single far score dominates: the output must be that key's value."""
