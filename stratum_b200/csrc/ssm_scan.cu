@@ -83,6 +83,72 @@ __global__ void __launch_bounds__(SS_PREP_THREADS) ssm_prep_kernel(const SsmScan
   out[c] = ss_silu(acc);
 }
 
+// Short convolutions of four taps over 16-byte aligned rows (every configuration so far): a thread takes four channels
+// through SS_PREP_TOKENS tokens with the last three inputs in registers, so an input is read once from L2 by 16-byte
+// loads instead of four times by 4-byte ones.  The sums are those of the kernel above, in its order.  2,000 tokens of
+// 10,240 channels (164 MB in and out) take 59 us; a thread per channel and token, which was bound by its instructions
+// (83 % of the issue slots), took 156.
+#define SS_PREP_TOKENS 8
+__global__ void __launch_bounds__(SS_PREP_THREADS) ssm_prep4_kernel(const SsmScan P) {
+  pdl_trigger();
+  pdl_wait();                // the projection and the state are the work of kernels before this one: ld_fresh
+  const int inner = P.n_heads * P.vdim, C = inner + 2 * P.n_groups * P.n_state;
+  const int item = blockIdx.y * SS_PREP_THREADS + threadIdx.x;      // four channels, or behind the channels a head
+  const int t0 = blockIdx.x * SS_PREP_TOKENS, t1 = min(P.n_tokens, t0 + SS_PREP_TOKENS);
+  if (item >= C / 4 + P.n_heads) return;
+  if (item >= C / 4) {
+    const int h = item - C / 4;
+    const float bias = P.dt_bias[h], rate = -expf(P.a_log[h]);
+    for (int t = t0; t < t1; t++) {
+      float* out = P.act + (size_t)t * P.lda;
+      const float z = ld_fresh(P.proj + (size_t)t * P.ld + inner + C + h) + bias;
+      const float dt = z > 20.f ? z : log1pf(expf(z));
+      out[C + h] = dt;
+      out[C + P.n_heads + h] = expf(rate * dt);
+    }
+    return;
+  }
+  const int c = 4 * item;
+  const float* in = P.proj + inner + c;
+  float w[4][4];             // [channel][tap]
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    const float4 v = *reinterpret_cast<const float4*>(P.conv_w + 4 * (size_t)(c + e));
+    w[e][0] = v.x; w[e][1] = v.y; w[e][2] = v.z; w[e][3] = v.w;
+  }
+  const float4 bias = *reinterpret_cast<const float4*>(P.conv_b + c);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 x[SS_PREP_TOKENS + 3];              // rows t0 - 3 .. t1 - 1, whoever's they are
+#pragma unroll
+  for (int i = 0; i < SS_PREP_TOKENS + 3; i++) {
+    const int t = t0 - 3 + i;
+    x[i] = t >= 0 && t < t1 ? ld_fresh(reinterpret_cast<const float4*>(in + (size_t)t * P.ld)) : zero;
+  }
+#pragma unroll
+  for (int k = 0; k < SS_PREP_TOKENS; k++) {
+    const int t = t0 + k;
+    if (t >= t1) break;
+    const int seq = P.token_seq[t], pos = P.token_pos[t];
+    const int in_step = seq >= 0 ? t - P.seq_start[seq] : 0;
+    float4 acc = bias;
+#pragma unroll
+    for (int i = 3; i >= 0; i--) {                   // oldest input first: one fixed order
+      float4 v = x[k + 3 - i];
+      if (i > in_step)                               // it came with an earlier step, or never
+        v = seq >= 0 && pos - i >= 0
+                ? ld_fresh(reinterpret_cast<const float4*>(P.state + (size_t)P.seq_slot[seq] * P.state_stride +
+                                                           (size_t)inner * P.n_state + (size_t)(3 - (i - in_step)) * C + c))
+                : zero;
+      acc.x = fmaf(w[0][3 - i], v.x, acc.x);
+      acc.y = fmaf(w[1][3 - i], v.y, acc.y);
+      acc.z = fmaf(w[2][3 - i], v.z, acc.z);
+      acc.w = fmaf(w[3][3 - i], v.w, acc.w);
+    }
+    *reinterpret_cast<float4*>(P.act + (size_t)t * P.lda + c) =
+        make_float4(ss_silu(acc.x), ss_silu(acc.y), ss_silu(acc.z), ss_silu(acc.w));
+  }
+}
+
 // ---------------------------------------------------------------- the recurrence
 #define SS_THREADS 128
 #define SS_HELD 16            // entries of S that a lane holds: R rows of Q columns
@@ -292,6 +358,157 @@ __global__ void __launch_bounds__(SS_THREADS) ssm_recur_kernel(const SsmScan P) 
   }
 }
 
+// States of 33 to 128 rows (in fours) and columns in eights: a warp by itself takes eight columns, 16 lanes four of them, a
+// lane R rows of its four (rows 64 i + 4 part ..: what 16 lanes read of B and C lies side by side).  It stages its own
+// tokens and adds its own read-outs, so no warp waits for another, and a lane's R x 4 entries share one load of B and C.
+// One sequence of 2,000 tokens, 128 heads of 64 columns and 128 rows: 443 us, against 708 with the block form above (whose
+// blocks met twice in eight tokens, and whose lanes held half as many entries, for twice the loads); six sequences of 1,000
+// tokens on 64 heads: 786 us a layer with prep and finish, 1,211.  What bounds it is the latency of dependent FMA at seven
+// warps an SM (the FMA pipes are 48 % busy); one, two or four warps a block measure the same.
+#define SW_CHUNK 8
+#define SW_WARPS 2
+template <int R, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) ssm_recur_warp_kernel(const SsmScan P) {
+  constexpr int NP = 64 * (R / 4), G = R / 4, TOKEN = 2 * NP + 8, GROUP_PITCH = 68;
+  struct Warp {
+    float in[2][SW_CHUNK][TOKEN];                    // B [NP] | C [NP] | x [8]
+    float dd[2][SW_CHUNK][2];                        // dt, decay
+    float part[SW_CHUNK][2][GROUP_PITCH];
+  };
+  extern __shared__ __align__(16) float sw_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane & 15, grp = lane >> 4;
+  Warp& sm = reinterpret_cast<Warp*>(sw_smem)[warp];
+  pdl_trigger();             // (launched the ordinary way itself: it starts when prep is done)
+  const int seq = blockIdx.z, h = blockIdx.y, tile = blockIdx.x * WARPS + warp;
+  const int N = P.n_state, V = P.vdim, inner = P.n_heads * V, GN = P.n_groups * N, C = inner + 2 * GN;
+  const int r0 = P.seq_start[seq], r1 = P.seq_start[seq + 1];
+  if (r0 >= r1 || tile * 8 >= V) return;
+  if (P.token_seq[r0] < 0) {                         // rows of no sequence: nothing is kept, the output is zero
+    for (int i = lane; i < (r1 - r0) * 8; i += 32) P.y_raw[(size_t)(r0 + i / 8) * inner + (size_t)h * V + tile * 8 + i % 8] = 0.f;
+    return;
+  }
+  float* slot = P.state + (size_t)P.seq_slot[seq] * P.state_stride;
+  if (P.write_state && P.taps > 1) {                 // the convolution's tail, as above: the warps of a sequence share it
+    float* tail = slot + (size_t)inner * N;
+    const int keep = P.taps - 1, n_new = r1 - r0, n_warps = P.n_heads * (V / 8);
+    const int per = (C + n_warps - 1) / n_warps, me = h * (V / 8) + tile, c_end = min(C, (me + 1) * per);
+    for (int c = me * per + lane; c < c_end; c += 32)
+      for (int i = 0; i < keep; i++) {
+        const int back = keep - i;
+        tail[(size_t)i * C + c] = back <= n_new ? P.proj[(size_t)(r1 - back) * P.ld + inner + c] : tail[(size_t)(i + n_new) * C + c];
+      }
+  }
+  const int g = h / (P.n_heads / P.n_groups);
+  const float d_skip = P.d_skip[h];
+  const int j0 = tile * 8 + grp * 4;
+  float* Sg = slot + ((size_t)h * V + j0) * N + 4 * part;
+  float2 S[4][R / 2];
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int i = 0; i < G; i++) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (64 * i + 4 * part < N) v = *reinterpret_cast<const float4*>(Sg + (size_t)q * N + 64 * i);
+      S[q][2 * i] = make_float2(v.x, v.y);
+      S[q][2 * i + 1] = make_float2(v.z, v.w);
+    }
+  if (N < NP)                                        // rows beyond n_state stay zero: nothing below writes them
+    for (int i = lane; i < 2 * SW_CHUNK * TOKEN; i += 32) (&sm.in[0][0][0])[i] = 0.f;
+  __syncwarp();
+  const float* act = P.act + inner + (size_t)g * N;
+  auto stage = [&](int buf, int c0) {
+    const int n_here = min(SW_CHUNK, r1 - c0);
+    const float* a = act + (size_t)c0 * P.lda + 4 * part;
+#pragma unroll
+    for (int tok = 0; tok < SW_CHUNK; tok++)         // half a warp B, half a warp C
+      if (tok < n_here)
+#pragma unroll
+        for (int i = 0; i < G; i++)
+          if (64 * i + 4 * part < N)
+            ss_copy16(&sm.in[buf][tok][grp * NP + 64 * i + 4 * part], a + (size_t)tok * P.lda + grp * GN + 64 * i);
+    if (lane < 2 * n_here)
+      ss_copy16(&sm.in[buf][lane >> 1][2 * NP + 4 * (lane & 1)],
+                P.act + (size_t)(c0 + (lane >> 1)) * P.lda + (size_t)h * V + tile * 8 + 4 * (lane & 1));
+    if (lane < 2 * n_here)
+      ss_copy4(&sm.dd[buf][lane >> 1][lane & 1], P.act + (size_t)(c0 + (lane >> 1)) * P.lda + C + (lane & 1) * P.n_heads + h);
+    ss_commit();
+  };
+  stage(0, r0);
+  int buf = 0;
+  for (int c0 = r0; c0 < r1; c0 += SW_CHUNK, buf ^= 1) {
+    ss_wait_all();
+    __syncwarp();                                    // this chunk has landed, and the other buffer is free again
+    if (c0 + SW_CHUNK < r1) stage(buf ^ 1, c0 + SW_CHUNK);
+    const int n_here = min(SW_CHUNK, r1 - c0);
+    auto token = [&](int tok) {                      // one token of the chunk: the state moves on, partials out
+      const float* in = sm.in[buf][tok];
+      float4 b4[G], c4[G];
+#pragma unroll
+      for (int i = 0; i < G; i++) {
+        b4[i] = *reinterpret_cast<const float4*>(in + 64 * i + 4 * part);
+        c4[i] = *reinterpret_cast<const float4*>(in + NP + 64 * i + 4 * part);
+      }
+      const float4 x4 = *reinterpret_cast<const float4*>(in + 2 * NP + 4 * grp);
+      const float2 dd = *reinterpret_cast<const float2*>(sm.dd[buf][tok]);
+      const float2 dk = make_float2(dd.y, dd.y);
+      const float xq[4] = {x4.x, x4.y, x4.z, x4.w};
+      float y[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const float dtx = dd.x * xq[q];
+        const float2 uu = make_float2(dtx, dtx);
+        float2 a0 = make_float2(0.f, 0.f), a1 = a0;
+#pragma unroll
+        for (int i = 0; i < G; i++) {
+          S[q][2 * i] = __ffma2_rn(make_float2(b4[i].x, b4[i].y), uu, __fmul2_rn(dk, S[q][2 * i]));
+          S[q][2 * i + 1] = __ffma2_rn(make_float2(b4[i].z, b4[i].w), uu, __fmul2_rn(dk, S[q][2 * i + 1]));
+          a0 = __ffma2_rn(S[q][2 * i], make_float2(c4[i].x, c4[i].y), a0);
+          a1 = __ffma2_rn(S[q][2 * i + 1], make_float2(c4[i].z, c4[i].w), a1);
+        }
+        const float2 s2 = __fadd2_rn(a0, a1);
+        y[q] = s2.x + s2.y;
+      }
+      *reinterpret_cast<float4*>(&sm.part[tok][grp][4 * part]) = make_float4(y[0], y[1], y[2], y[3]);
+    };
+    if (n_here == SW_CHUNK) {                        // a whole chunk: the tokens' loads and sums interleave
+#pragma unroll
+      for (int tok = 0; tok < SW_CHUNK; tok++) token(tok);
+    } else {
+      for (int tok = 0; tok < n_here; tok++) token(tok);
+    }
+    __syncwarp();                                    // the chunk's partial read-outs are all there
+#pragma unroll
+    for (int o = lane; o < SW_CHUNK * 8; o += 32) {  // (token, column): the 16 lanes' parts, four chains of four
+      const int tok = o >> 3, c = o & 7;
+      if (tok >= n_here) break;
+      const float* p = &sm.part[tok][c >> 2][c & 3];
+      float y[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) y[u] = ((p[16 * u] + p[16 * u + 4]) + p[16 * u + 8]) + p[16 * u + 12];
+      P.y_raw[(size_t)(c0 + tok) * inner + (size_t)h * V + tile * 8 + c] =
+          fmaf(d_skip, sm.in[buf][tok][2 * NP + c], (y[0] + y[1]) + (y[2] + y[3]));
+    }
+  }
+  if (P.write_state)
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+      for (int i = 0; i < G; i++)
+        if (64 * i + 4 * part < N)
+          *reinterpret_cast<float4*>(Sg + (size_t)q * N + 64 * i) =
+              make_float4(S[q][2 * i].x, S[q][2 * i].y, S[q][2 * i + 1].x, S[q][2 * i + 1].y);
+}
+
+template <int R, int WARPS>
+static int ssm_recur_warp_launch(const SsmScan& P, cudaStream_t stream) {
+  const int smem = WARPS * (int)sizeof(float) * (2 * SW_CHUNK * (2 * 64 * (R / 4) + 8) + 2 * SW_CHUNK * 2 + SW_CHUNK * 2 * 68);
+  static int once = (int)cudaFuncSetAttribute(ssm_recur_warp_kernel<R, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (once) return once;
+  const dim3 grid((P.vdim / 8 + WARPS - 1) / WARPS, P.n_heads, P.n_seqs);
+  ssm_recur_warp_kernel<R, WARPS><<<grid, WARPS * 32, smem, stream>>>(P);
+  return launch_status();
+}
+
 // ---------------------------------------------------------------- finish: a block per (token, part of the row)
 // The sum of squares is added in an order that the part's size alone fixes: a thread over its strided entries, a
 // warp by shuffles, the warps one after another.
@@ -338,6 +555,57 @@ __global__ void __launch_bounds__(SS_FIN_THREADS) ssm_finish_kernel(const SsmSca
     out[d] = from_float<T>(ld_fresh(y + d) * ss_silu(ld_fresh(z + d)) * mul * gain[d]);
 }
 
+// Parts of up to 1,024 entries in 16-byte aligned rows: a thread keeps two float4 between the two passes, so nothing is
+// read, and no exponential evaluated, twice.  2,000 tokens of 8,192 entries (164 MB): 36 us against 79.
+template <typename T>
+__global__ void __launch_bounds__(SS_FIN_THREADS) ssm_finish4_kernel(const SsmScan P) {
+  __shared__ float warp_ss[SS_FIN_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_trigger();
+  pdl_wait();                // y_raw and the projection are the work of kernels before this one: ld_fresh
+  const long long item = blockIdx.x;
+  const int t = (int)(item / P.norm_groups), part = (int)(item - (long long)t * P.norm_groups);
+  const int inner = P.n_heads * P.vdim, size = inner / P.norm_groups;
+  const float4* y = reinterpret_cast<const float4*>(P.y_raw + (size_t)t * inner + (size_t)part * size);
+  const float4* z = reinterpret_cast<const float4*>(P.proj + (size_t)t * P.ld + (size_t)part * size);
+  const float4* gain = reinterpret_cast<const float4*>(P.gain + (size_t)part * size);
+  T* out = (T*)P.out + (size_t)t * P.ldo + (size_t)part * size;
+  float4 v[2], zz[2];
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const int d = threadIdx.x + i * SS_FIN_THREADS;
+    const bool in = 4 * d < size;
+    v[i] = in ? ld_fresh(y + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+    zz[i] = in ? ld_fresh(z + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    v[i].x *= ss_silu(zz[i].x); v[i].y *= ss_silu(zz[i].y); v[i].z *= ss_silu(zz[i].z); v[i].w *= ss_silu(zz[i].w);
+    ss = fmaf(v[i].x, v[i].x, ss); ss = fmaf(v[i].y, v[i].y, ss); ss = fmaf(v[i].z, v[i].z, ss); ss = fmaf(v[i].w, v[i].w, ss);
+  }
+  ss = warp_sum(ss);
+  if (lane == 0) warp_ss[warp] = ss;
+  __syncthreads();
+  float total = 0.f;
+#pragma unroll
+  for (int i = 0; i < SS_FIN_THREADS / 32; i++) total += warp_ss[i];
+  const float mul = 1.0f / sqrtf(total / (float)size + P.eps);
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const int d = threadIdx.x + i * SS_FIN_THREADS;
+    if (4 * d >= size) break;
+    const float4 gn = gain[d];
+    const float4 o = make_float4(v[i].x * mul * gn.x, v[i].y * mul * gn.y, v[i].z * mul * gn.z, v[i].w * mul * gn.w);
+    if constexpr (sizeof(T) == 4) {
+      *reinterpret_cast<float4*>(out + 4 * d) = o;
+    } else {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(o.x, o.y), hi = __floats2bfloat162_rn(o.z, o.w);
+      *reinterpret_cast<uint2*>(out + 4 * d) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+  }
+}
+
 static int ssm_check(const SsmScan& P) {
   if (P.n_heads < 1 || P.n_groups < 1 || P.n_heads % P.n_groups != 0 || P.vdim < 1 || P.n_state < 1 || P.taps < 1)
     return STRATUM_ERR_SHAPE;
@@ -363,15 +631,26 @@ STRATUM_EXPORT int stratum_ssm_scan(const SsmScan* params, int out_dtype, cudaSt
   if (P.n_tokens <= 0 || P.n_seqs <= 0) return 0;
   const int bad = ssm_check(P);
   if (bad) return bad;
-  {
-    const int inner = P.n_heads * P.vdim, items = inner + 2 * P.n_groups * P.n_state + P.n_heads;
+  const int inner = P.n_heads * P.vdim, C = inner + 2 * P.n_groups * P.n_state;
+  const uintptr_t all = (uintptr_t)P.proj | (uintptr_t)P.act | (uintptr_t)P.state | (uintptr_t)P.y_raw | (uintptr_t)P.out |
+                        (uintptr_t)P.gain | (uintptr_t)P.conv_w | (uintptr_t)P.conv_b;
+  const bool rows16 = all % 16 == 0 && P.ld % 4 == 0 && P.lda % 4 == 0 && P.ldo % 4 == 0 && P.state_stride % 4 == 0 &&
+                      inner % 4 == 0 && P.n_state % 4 == 0;
+  if (rows16 && P.taps == 4) {
+    launch_pdl(ssm_prep4_kernel, dim3((P.n_tokens + SS_PREP_TOKENS - 1) / SS_PREP_TOKENS,
+                                      (C / 4 + P.n_heads + SS_PREP_THREADS - 1) / SS_PREP_THREADS), SS_PREP_THREADS, 0, stream, P);
+  } else {
+    const int items = C + P.n_heads;
     launch_pdl(ssm_prep_kernel, dim3(P.n_tokens, (items + SS_PREP_THREADS - 1) / SS_PREP_THREADS), SS_PREP_THREADS, 0,
                stream, P);
   }
   int st = launch_status();
   if (st) return st;
+  if (rows16 && P.n_state > 32 && P.n_state <= 128 && P.vdim % 8 == 0) {
+    st = P.n_state > 64 ? ssm_recur_warp_launch<8, SW_WARPS>(P, stream) : ssm_recur_warp_launch<4, SW_WARPS>(P, stream);
+    if (st) return st;
   // few rows per lane while a warp still covers the rows: 4 up to 128 rows, 8 up to 256, 16 beyond
-  if (P.n_state > 256) ssm_recur_launch<32, 16>(P, stream);
+  } else if (P.n_state > 256) ssm_recur_launch<32, 16>(P, stream);
   else if (P.n_state > 128) ssm_recur_launch<32, 8>(P, stream);
   else {
     int L = 1;
@@ -389,8 +668,12 @@ STRATUM_EXPORT int stratum_ssm_scan(const SsmScan* params, int out_dtype, cudaSt
   if (st) return st;
   const long long blocks = (long long)P.n_tokens * P.norm_groups;
   if (blocks > 0x7fffffffLL) return STRATUM_ERR_LIMIT;
-  if (out_dtype == STRATUM_DT_F32) launch_pdl(ssm_finish_kernel<float>, (unsigned)blocks, SS_FIN_THREADS, 0, stream, P);
-  else if (out_dtype == STRATUM_DT_BF16) launch_pdl(ssm_finish_kernel<bf16>, (unsigned)blocks, SS_FIN_THREADS, 0, stream, P);
-  else return STRATUM_ERR_DTYPE;
+  if (out_dtype != STRATUM_DT_F32 && out_dtype != STRATUM_DT_BF16) return STRATUM_ERR_DTYPE;
+  const int size = inner / P.norm_groups;
+  if (rows16 && size % 4 == 0 && size <= 8 * SS_FIN_THREADS) {
+    if (out_dtype == STRATUM_DT_F32) launch_pdl(ssm_finish4_kernel<float>, (unsigned)blocks, SS_FIN_THREADS, 0, stream, P);
+    else launch_pdl(ssm_finish4_kernel<bf16>, (unsigned)blocks, SS_FIN_THREADS, 0, stream, P);
+  } else if (out_dtype == STRATUM_DT_F32) launch_pdl(ssm_finish_kernel<float>, (unsigned)blocks, SS_FIN_THREADS, 0, stream, P);
+  else launch_pdl(ssm_finish_kernel<bf16>, (unsigned)blocks, SS_FIN_THREADS, 0, stream, P);
   return launch_status();
 }

@@ -117,6 +117,53 @@ def test_state_space_kernels(heads, vdim, state, groups, taps, parts, long):
     assert float(st[0].abs().max()) == 0.0 and float(st[5].abs().max()) == 0.0            # rows of nobody stay clean
 
 
+@pytest.mark.parametrize("heads,vdim,state,groups,taps,parts", [
+    (8, 16, 128, 1, 4, 4), (4, 32, 64, 2, 4, 1), (2, 24, 36, 1, 4, 3), (3, 8, 100, 3, 4, 1), (16, 64, 48, 2, 4, 1),
+    (4, 24, 68, 2, 3, 2), (32, 64, 128, 8, 4, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_state_space_kernels_on_aligned_rows(heads, vdim, state, groups, taps, parts, dtype):
+    """Rows of 16-byte pitch: the vector forms of the three kernels and the recurrence by warps, at the edges of their
+    eight tokens, tails that reach into the step before, rows of no sequence between two sequences."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(state + vdim + taps)
+    inner, C = heads * vdim, heads * vdim + 2 * groups * state
+    width = inner + C + heads
+    f = lambda lo, hi, *shape: rng.uniform(lo, hi, shape)
+    conv, conv_b, a_log, dt_bias = f(-0.8, 0.8, C, taps), f(-0.3, 0.3, C), f(-2, 0.5, heads), f(-1, 1, heads)
+    d_skip, gain = f(-1, 1.5, heads), f(0.5, 1.5, inner)
+    m = {"heads": heads, "vdim": vdim, "state": state, "groups": groups, "conv": taps, "norm_groups": parts}
+    w = {"in": np.eye(width), "conv": conv, "conv.b": conv_b, "A_log": a_log, "dt_bias": dt_bias, "D": d_skip,
+         "norm": gain, "o": np.eye(inner)}
+    cuts = ((17, 7), (1, 8), (2, 9), (8, 1))
+    proj = [rng.standard_normal((sum(c[i] for c in cuts), width)) for i in range(2)]
+    want = [V.state_space_mixer(p, w, m, 1e-5) for p in proj]
+    up = lambda n: -(-n // 4) * 4
+    st = torch.zeros(4, up(inner * state + (taps - 1) * C), device="cuda")
+    done, got = [0, 0], [[], []]
+    for cut in cuts:
+        T = sum(cut) + 3                                               # three rows of nobody between the two
+        rows = np.zeros((T, up(width) + 4))
+        at = (0, cut[0] + 3)
+        for i in range(2):
+            rows[at[i]:at[i] + cut[i], :width] = proj[i][done[i]:done[i] + cut[i]]
+        pos = np.concatenate([np.arange(done[0], done[0] + cut[0]), [0] * 3, np.arange(done[1], done[1] + cut[1])])
+        seq = np.concatenate([np.zeros(cut[0]), [-1] * 3, np.full(cut[1], 2)])
+        out = torch.full((T, up(inner) + 8), 7.0, dtype=dtype, device="cuda")
+        K.ssm_scan(_dev(rows), _dev(conv), _dev(conv_b), _dev(a_log), _dev(dt_bias), _dev(d_skip), _dev(gain),
+                   torch.empty(T, up(C + 2 * heads), device="cuda"), torch.empty(T, inner, device="cuda"), out, st,
+                   _dev(pos, torch.int32), _dev(seq, torch.int32), _dev(np.array([0, cut[0], cut[0] + 3, T]), torch.int32),
+                   _dev(np.array([3, 0, 1]), torch.int32), heads, vdim, state, groups, parts, 1e-5, True)
+        assert float((out[:, inner:].float() - 7.0).abs().max()) == 0.0
+        for i in range(2):
+            got[i].append(out[at[i]:at[i] + cut[i], :inner].float().cpu().numpy())
+        done = [done[i] + cut[i] for i in range(2)]
+    for i in range(2):
+        g = np.concatenate(got[i])
+        tol = 3e-5 if dtype == torch.float32 else 2.0 ** -8            # (bfloat16: half a unit of the last place)
+        assert np.max(np.abs(g - want[i])) <= tol * np.max(np.abs(want[i])), (i, np.max(np.abs(g - want[i])))
+    assert float(st[0].abs().max()) == 0.0 and float(st[2].abs().max()) == 0.0
+
+
 def test_state_space_kernel_leaves_the_state_alone_when_told_to():
     from stratum_b200 import kernels as K
     rng = np.random.default_rng(3)
