@@ -175,10 +175,13 @@ STRATUM_EXPORT int stratum_argmax(const float* logits, int ld, int n_rows, int v
 //   temperature[r] <= 0 -> greedy;  top_k[r] <= 0 -> off;  top_p[r] >= 1 -> off;  uniform[r] in [0,1).
 // Every sum is taken in an order that depends on the sizes only, so a row's pick is the same in every batch and run.
 
-// order-preserving map float -> uint32 (larger float, larger key)
+// order-preserving map float -> uint32 (larger float, larger key; the two zeros are equals), and back
 __device__ __forceinline__ uint32_t float_key(float f) {
-  const uint32_t u = __float_as_uint(f);
+  const uint32_t u = __float_as_uint(__fadd_rn(f, 0.f));
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float key_float(uint32_t key) {
+  return __uint_as_float((key & 0x80000000u) ? (key ^ 0x80000000u) : ~key);
 }
 
 // Inclusive prefix sum over the lanes of a warp (lane 0 first).
@@ -226,13 +229,13 @@ __device__ __forceinline__ T block_excl_scan(T v, T* scratch, T* total) {
   return scratch[warp] + incl - v;
 }
 
-// One warp: lane l holds the SAMPLE_CAND_MAX / 32 consecutive candidates from its first on (sorted: descending
+// One warp: lane l holds the PER consecutive candidates from its first on (n_cand <= 32 PER, sorted: descending
 // logit, ascending id among equals; cand_e their weights, zero beyond n_cand); sums in float64: their total, the
 // top-p cut over the normalised weights, and the draw among what is kept.
-__device__ __forceinline__ void draw_from_candidates(const float* cand_v, const int* cand_i, const float* cand_e,
+template <int PER>
+__device__ __forceinline__ void draw_from(const float* cand_v, const int* cand_i, const float* cand_e,
                                                      int n_cand, float tp, float u, int r, int* ids, float* values) {
   const int lane = threadIdx.x & 31;
-  constexpr int PER = SAMPLE_CAND_MAX / 32;
   const int c0 = lane * PER;
   double own = 0.0;
 #pragma unroll
@@ -273,6 +276,17 @@ __device__ __forceinline__ void draw_from_candidates(const float* cand_v, const 
     ids[r] = cand_i[pick];
     if (values) values[r] = cand_v[pick];
   }
+}
+
+// (a lane's share follows from the number of candidates: 50 of them in shares of 16 kept four lanes busy; shares of 2
+// take a row's draw with a top-p cut from 32 to 21 us in all)
+__device__ __forceinline__ void draw_from_candidates(const float* cand_v, const int* cand_i, const float* cand_e,
+                                                     int n_cand, float tp, float u, int r, int* ids, float* values) {
+  static_assert(SAMPLE_CAND_MAX == 16 * 32, "the largest share");
+  if (n_cand <= 64) draw_from<2>(cand_v, cand_i, cand_e, n_cand, tp, u, r, ids, values);
+  else if (n_cand <= 128) draw_from<4>(cand_v, cand_i, cand_e, n_cand, tp, u, r, ids, values);
+  else if (n_cand <= 256) draw_from<8>(cand_v, cand_i, cand_e, n_cand, tp, u, r, ids, values);
+  else draw_from<16>(cand_v, cand_i, cand_e, n_cand, tp, u, r, ids, values);
 }
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
@@ -474,17 +488,20 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab, const float* 
 // temperature alone, 100 to 130 us with filters, whatever the batch.  Here a row is cut into SS_SPLITS stretches
 // of consecutive ids.  A block takes one stretch into shared memory and leaves: its largest logit (greedy rows,
 // and the row's maximum); without filters, the sums of its weights exp((l - its maximum) / T) over eight
-// sub-stretches; with filters, its own min(k, SS_KEEP) largest logits in ascending id order, and the key of the
-// last of them.  The block that finishes last (a counter per row tells; no block waits) does the rest from those
-// leavings: the row's maximum, then either the sub-stretch that holds the draw and a walk through it, or the k
-// largest of the 32 lists (in shared memory), sorted, cut by top-p and drawn from, as above.
+// sub-stretches; with filters, at least its own min(k, SS_KEEP) largest logits (gather_largest), the key that all it left
+// out lie below and how many it kept.  The block that finishes last (a counter per row tells; no block waits) does the
+// rest from those leavings: the row's maximum, then either the sub-stretch that holds the draw and a walk through it, or
+// the k largest of the 32 lists (in shared memory), sorted, cut by top-p and drawn from, as above.
 //
-// A stretch leaves at most SS_KEEP candidates, although any number of the row's k largest could lie in one
-// stretch.  So the last block checks: a stretch that kept fewer than k has nothing hidden among the row's k largest
-// if the key of its last kept candidate is below the key of the k-th largest of all lists.  With 128,256 logits
-// and k = 512 the k-th largest is the 99.6th percentile of the row, a stretch's 64th largest the 98.4th of its
-// own, so the check holds unless the large logits crowd in one stretch; when it does not hold the row is marked
-// and the one-block kernel, launched behind this one for marked rows only, does the row by itself.
+// For k above SS_KEEP any number of the row's k largest could lie in one stretch.  So the last block checks: a stretch has
+// nothing hidden among the row's k largest if the key its leavings out lie below is at most the key of the k-th largest of
+// all lists.  With 128,256 logits and k = 512 the k-th largest is the 99.6th percentile of the row, a stretch's 64th
+// largest the 98.4th of its own, so the check holds unless the large logits crowd in one stretch; when it does not hold
+// (or logits equal to one another straddle a cut that the lists, which are in no order, cannot make) the row is marked and
+// the one-block kernel, launched behind this one for marked rows only, does the row by itself.
+//
+// 128,256 logits, top-k 50, top-p 0.95 (us, 1 / 24 / 64 rows): 21 / 31 / 48; with two radix selections and lists in id
+// order it took 36 / 61 / 113, and one block a row takes 87.  k = 512: 43 / 54 / 72 against 47 / 72 / 125.
 // Sums are taken in an order that depends on the sizes only.
 #define SS_SPLITS 32
 #define SS_THREADS 256
@@ -492,31 +509,26 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab, const float* 
 static_assert(SS_THREADS == 256, "one thread per bucket of the radix passes");
 #define SS_CHUNK_MAX 8192
 #define SS_KEEP 64
-#define SS_LIST_MAX (SS_SPLITS * SS_KEEP)
+#define SS_LIST 128              // room of a stretch's list
+#define SS_LIST_MAX (SS_SPLITS * SS_LIST)
+#define SS_FEW 128               // up to this k the last block places the candidates by counting
 
 struct SsScratch {               // in global memory, per row (counters zeroed once; every launch leaves them at zero)
   float* part_v; int* part_i;    // [rows][SS_SPLITS] largest logit of the stretch and its id
   float* part_e;                 // [rows][SS_SPLITS][SS_WARPS] sums of the sub-stretches' weights (stretch's own maximum)
-  unsigned* part_key;            // [rows][SS_SPLITS] key of the stretch's last kept candidate
-  float* cand_v; int* cand_i;    // [rows][SS_LIST_MAX]: the stretches' lists one after another
+  unsigned* part_key;            // [rows][SS_SPLITS] what the stretch did not keep lies below this key (0: it kept all)
+  float* cand_v; int* cand_i;    // [rows][SS_SPLITS][SS_LIST]: the stretches' lists, keys (as bits) and ids; the number
+                                 // of entries lies in part_e, as bits, at the stretch's first place
   unsigned* counters;            // [rows]
   int* redo;                     // [rows] 1: the one-block kernel does this row
 };
 
-// Among n values in ascending id order (val(j), id(j)), the k largest, the lowest ids first among equals at the
-// cut, written in ascending id order to out_v / out_i.  Returns how many (min(k, n)); *kth_key gets the key of the
-// smallest of them (0 if all n were taken).  Every thread of the block calls it.  hist: 256 words, sh: 2,
-// w_scratch: 2 * SS_WARPS.
-template <typename Val, typename Id>
-__device__ int select_in_order(Val val, Id id, int n, int k, float* out_v, int* out_i, unsigned* hist, unsigned* sh,
-                               unsigned* w_scratch, unsigned* w_scratch33, uint32_t* kth_key) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (k >= n) {
-    for (int j = tid; j < n; j += SS_THREADS) { out_v[j] = val(j); out_i[j] = id(j); }
-    __syncthreads();
-    *kth_key = 0u;
-    return n;
-  }
+// The key of the k-th largest of n keys, 1 <= k <= n, by a radix select; *equals: how many have that key.  Returns how many
+// of those belong to the k largest.  Every thread of the block calls it.  hist: 256 words, sh: 2.
+template <typename Key>
+__device__ unsigned radix_kth(Key key_of, int n, int k, unsigned* hist, unsigned* sh, unsigned* w_scratch33, uint32_t* kth,
+                              uint32_t* equals) {
+  const int tid = threadIdx.x;
   if (tid == 0) { sh[0] = 0; sh[1] = (unsigned)k; }
   __syncthreads();
   for (int pass = 0; pass < 4; pass++) {          // radix select, 8 bits a pass from the top
@@ -526,7 +538,7 @@ __device__ int select_in_order(Val val, Id id, int n, int k, float* out_v, int* 
     const unsigned prefix = sh[0];
     const unsigned mask = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
     for (int j = tid; j < n; j += SS_THREADS) {
-      const uint32_t key = float_key(val(j));
+      const uint32_t key = key_of(j);
       if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
     }
     __syncthreads();
@@ -545,8 +557,27 @@ __device__ int select_in_order(Val val, Id id, int n, int k, float* out_v, int* 
     }
     __syncthreads();
   }
-  const uint32_t kth = sh[0];
-  const unsigned want_eq = sh[1];                  // how many of those equal to the k-th largest are taken
+  *kth = sh[0];
+  *equals = hist[sh[0] & 255u];                    // the last pass's bucket
+  return sh[1];
+}
+
+// Among n values in ascending id order (val(j), id(j)), the k largest, the lowest ids first among equals at the
+// cut, written in ascending id order to out_v / out_i.  Returns how many (min(k, n)); *kth_key gets the key of the
+// smallest of them (0 if all n were taken).  Every thread of the block calls it.  hist: 256 words, sh: 2,
+// w_scratch: 2 * SS_WARPS.
+template <typename Val, typename Id>
+__device__ int select_in_order(Val val, Id id, int n, int k, float* out_v, int* out_i, unsigned* hist, unsigned* sh,
+                               unsigned* w_scratch, unsigned* w_scratch33, uint32_t* kth_key) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (k >= n) {
+    for (int j = tid; j < n; j += SS_THREADS) { out_v[j] = val(j); out_i[j] = id(j); }
+    __syncthreads();
+    *kth_key = 0u;
+    return n;
+  }
+  uint32_t kth, equals;
+  const unsigned want_eq = radix_kth([&](int j) { return float_key(val(j)); }, n, k, hist, sh, w_scratch33, &kth, &equals);
   // in id order, 256 ids a round: an element's rank among the equal ones and its place in the output are counts of
   // the elements before it (votes inside a warp, the warps' counts through shared memory)
   unsigned eq_before = 0, out_before = 0;
@@ -576,6 +607,68 @@ __device__ int select_in_order(Val val, Id id, int n, int k, float* out_v, int* 
   return k;
 }
 
+// At least the k largest of n, k <= SS_THREADS, by their keys: thread t's largest element is one of SS_THREADS maxima, and
+// the k-th largest of those is at most the k-th largest of all.  put(slot, key, j) is called for every element that
+// reaches it (a little more than k of them as a rule, in any order; all of those with that key) whose slot is below
+// `room`.  Returns how many there are; *least_of gets the key.  Three barriers in place of the radix passes' sixteen and
+// two per 256 elements.  maxima: SS_THREADS words; sh: 2.
+template <typename Key, typename Put>
+__device__ __forceinline__ unsigned gather_largest(Key key, Put put, int n, int k, unsigned room, uint32_t* maxima,
+                                                   unsigned* sh, uint32_t* least_of) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t mine = 0u;
+  for (int j = tid; j < n; j += SS_THREADS) mine = max(mine, key(j));
+  if (tid == 0) sh[1] = 0u;
+  // every maximum's rank: its place in its warp's, sorted by shuffles, and searches through the other warps'
+  uint32_t v = mine;
+#pragma unroll
+  for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      const uint32_t other = __shfl_xor_sync(0xffffffffu, v, stride);
+      const bool larger = ((lane & stride) == 0) == ((lane & size) == 0);      // descending in the end
+      v = larger ? max(v, other) : min(v, other);
+    }
+  maxima[tid] = v;
+  __syncthreads();
+  int before = lane;
+#pragma unroll
+  for (int w = 0; w < SS_WARPS; w++) {
+    if (w == warp) continue;
+    const uint32_t* list = maxima + 32 * w;
+    int lo = 0;                                    // how many of warp w's come before v (equal ones of lower warps do)
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1) {
+      const uint32_t o = list[lo + step - 1];
+      if (o > v || (o == v && w < warp)) lo += step;
+    }
+    const uint32_t o = list[lo];                   // lo <= 31 after five steps
+    before += lo + (o > v || (o == v && w < warp));
+  }
+  if (before == k - 1) sh[0] = v;
+  __syncthreads();
+  const uint32_t least = sh[0];
+  if (mine >= least)
+    for (int j = tid; j < n; j += SS_THREADS) {
+      const uint32_t kj = key(j);
+      if (kj < least) continue;
+      const unsigned slot = atomicAdd(&sh[1], 1u);
+      if (slot < room) put(slot, kj, j);
+    }
+  __syncthreads();
+  *least_of = least;
+  return sh[1];
+}
+// How many of the n gathered elements come before element i: larger keys, then lower ids.
+__device__ __forceinline__ int place_of(const uint32_t* f_key, const int* f_id, int n, int i) {
+  const uint32_t mine = f_key[i];
+  const int id = f_id[i];
+  int before = 0;
+#pragma unroll 4
+  for (int j = 0; j < n; j++) before += f_key[j] > mine || (f_key[j] == mine && f_id[j] < id);
+  return before;
+}
+
 __global__ void __launch_bounds__(SS_THREADS)
 sample_split_kernel(const float* __restrict__ logits, int ld, int vocab, const float* __restrict__ temperature,
                     const int* __restrict__ top_k, const float* __restrict__ top_p,
@@ -591,6 +684,9 @@ sample_split_kernel(const float* __restrict__ logits, int ld, int vocab, const f
   __shared__ float cand_e[SAMPLE_CAND_MAX];
   __shared__ float cand_v[SAMPLE_CAND_MAX];
   __shared__ int cand_i[SAMPLE_CAND_MAX];
+  __shared__ uint32_t f_key[SS_THREADS];
+  __shared__ int f_id[SS_THREADS];
+  __shared__ int list_at[SS_SPLITS + 1];
   __shared__ int sh_owner;
   __shared__ bool last;
 
@@ -615,11 +711,11 @@ sample_split_kernel(const float* __restrict__ logits, int ld, int vocab, const f
   const int sub = (chunk + SS_WARPS - 1) / SS_WARPS;
 
   // ---- this block's stretch
-  for (int j = tid; j < n; j += SS_THREADS) lv[j] = ld_fresh(row + b0 + j);
-  __syncthreads();
   MaxIdx mine{-INFINITY, 0x7fffffff};
+#pragma unroll 4
   for (int j = tid; j < n; j += SS_THREADS) {
-    const float v = lv[j];
+    const float v = ld_fresh(row + b0 + j);
+    lv[j] = v;
     if (v > mine.v) { mine.v = v; mine.i = b0 + j; }              // ascending ids per thread: the first of equals stays
   }
   const MaxIdx local = block_argmax(mine, mi_scratch);
@@ -631,13 +727,32 @@ sample_split_kernel(const float* __restrict__ logits, int ld, int vocab, const f
     e = warp_sum(e);
     if (lane == 0) Q.part_e[(size_t)part * SS_WARPS + warp] = e;
   } else if (filtered) {
-    int off = 0;                                    // what the stretches before this one leave
-    for (int s2 = 0; s2 < sp; s2++) off += min(k1, stretch_len(s2));
-    uint32_t kth;
-    select_in_order([&](int j) { return lv[j]; }, [&](int j) { return b0 + j; }, n, k1,
-                    Q.cand_v + (size_t)r * SS_LIST_MAX + off, Q.cand_i + (size_t)r * SS_LIST_MAX + off, hist, sh,
-                    w_scratch, u_scratch, &kth);
-    if (tid == 0) Q.part_key[part] = kth;
+    float* to_v = Q.cand_v + (size_t)part * SS_LIST;
+    int* to_i = Q.cand_i + (size_t)part * SS_LIST;
+    auto put = [&](unsigned slot, uint32_t key, int j) {
+      to_v[slot] = __uint_as_float(key);
+      to_i[slot] = b0 + j;
+    };
+    uint32_t below = 0u;
+    unsigned kept;
+    if (n <= SS_LIST) {                             // (so few that all are kept)
+      for (int j = tid; j < n; j += SS_THREADS) put(j, float_key(lv[j]), j);
+      kept = n;
+    } else {
+      kept = gather_largest([&](int j) { return float_key(lv[j]); }, put, n, k1, SS_LIST, hist, sh, &below);
+      if (kept > SS_LIST) {                         // a crowd of equals: exactly k1, the lowest ids first among equals
+        __syncthreads();                            // (everyone knows how many were gathered)
+        uint32_t kth;
+        kept = select_in_order([&](int j) { return lv[j]; }, [&](int j) { return b0 + j; }, n, k1, cand_v, cand_i, hist, sh,
+                               w_scratch, u_scratch, &kth);
+        for (int j = tid; j < (int)kept; j += SS_THREADS) { to_v[j] = __uint_as_float(float_key(cand_v[j])); to_i[j] = cand_i[j]; }
+        below = kth == 0xffffffffu ? kth : kth + 1;
+      }
+    }
+    if (tid == 0) {
+      Q.part_key[part] = below;
+      Q.part_e[(size_t)part * SS_WARPS] = __uint_as_float(kept);
+    }
   }
   __threadfence();
   __syncthreads();
@@ -724,33 +839,77 @@ sample_split_kernel(const float* __restrict__ logits, int ld, int vocab, const f
     return;
   }
 
-  // ---- filtered: the lists, one after another (ascending ids), into shared memory; the k largest of them
-  int n_list = 0;
-  for (int s2 = 0; s2 < SS_SPLITS; s2++) n_list += min(k1, stretch_len(s2));
-  int* li = reinterpret_cast<int*>(lv + SS_LIST_MAX);
-  for (int j = tid; j < n_list; j += SS_THREADS) {
-    lv[j] = __ldcg(Q.cand_v + (size_t)r * SS_LIST_MAX + j);
-    li[j] = __ldcg(Q.cand_i + (size_t)r * SS_LIST_MAX + j);
+  // ---- filtered: the lists' keys, one list after another, into shared memory; the k largest of them
+  if (warp == 0) {
+    const int mine_n = (int)__float_as_uint(__ldcg(Q.part_e + (size_t)(r * SS_SPLITS + lane) * SS_WARPS));
+    const int upto = warp_incl_scan(mine_n);
+    list_at[lane] = upto - mine_n;
+    if (lane == 31) list_at[SS_SPLITS] = upto;
+    if (lane == 0) { sh_owner = 0; sh[1] = 0u; }
   }
   __syncthreads();
-  uint32_t kth;
-  const int n_cand = select_in_order([&](int j) { return lv[j]; }, [&](int j) { return li[j]; }, n_list, k, cand_v,
-                                     cand_i, hist, sh, w_scratch, u_scratch, &kth);
-  // a stretch that kept fewer than k of its ids: is anything it did not keep among the row's k largest?
-  if (tid == 0) sh_owner = 0;
-  __syncthreads();
-  if (tid < SS_SPLITS && k1 < k && stretch_len(tid) > k1) {
-    const uint32_t t_s = __ldcg(Q.part_key + r * SS_SPLITS + tid);
-    if (n_cand < k || t_s >= kth) sh_owner = 1;        // (fewer candidates than k in all: the lists do not hold k)
+  uint32_t* lk = reinterpret_cast<uint32_t*>(lv);
+#pragma unroll
+  for (int s2 = warp; s2 < SS_SPLITS; s2 += SS_WARPS) {
+    const int at = list_at[s2], len = list_at[s2 + 1] - at;
+#pragma unroll
+    for (int i = 0; i < SS_LIST; i += 32)
+      if (i + lane < len) lk[at + i + lane] = __float_as_uint(__ldcg(Q.cand_v + (size_t)(r * SS_SPLITS + s2) * SS_LIST + i + lane));
   }
+  const int n_all = list_at[SS_SPLITS];
+  auto id_of = [&](int j) {                          // the id that belongs to lk[j]: in the last list that begins at or before j
+    int s2 = 0;                                      // (empty lists begin where the next one does)
+#pragma unroll
+    for (int step = SS_SPLITS / 2; step > 0; step >>= 1)
+      if (list_at[s2 + step] <= j) s2 += step;
+    return __ldcg(Q.cand_i + (size_t)(r * SS_SPLITS + s2) * SS_LIST + j - list_at[s2]);
+  };
   __syncthreads();
-  if (sh_owner) {
+  const int n_cand = k;
+  uint32_t kth = 0u;
+  bool sorted = false, given_up = n_all < k;         // (fewer candidates than k in all: the lists do not hold k)
+  if (k <= SS_FEW && !given_up) {
+    uint32_t least;
+    const unsigned found = gather_largest([&](int j) { return lk[j]; },
+                                          [&](unsigned slot, uint32_t key, int j) { f_key[slot] = key; f_id[slot] = id_of(j); },
+                                          n_all, k, SS_THREADS, hist, sh, &least);
+    if (found <= SS_THREADS) {
+      const int place = tid < (int)found ? place_of(f_key, f_id, found, tid) : k;
+      if (place < k) { cand_v[place] = key_float(f_key[tid]); cand_i[place] = f_id[tid]; }
+      if (place == k - 1) sh[0] = f_key[tid];
+      __syncthreads();
+      kth = sh[0];
+      sorted = true;
+    }
+    __syncthreads();                                 // (everyone knows how many were gathered, and the k-th key)
+  }
+  if (!sorted && !given_up) {
+    uint32_t equals;
+    const unsigned wanted = radix_kth([&](int j) { return lk[j]; }, n_all, k, hist, sh, u_scratch, &kth, &equals);
+    // equals that straddle the cut would have to be taken by their ids, which come in no order here
+    given_up = wanted != equals;
+    __syncthreads();
+    if (tid == 0) sh[0] = 0u;
+    __syncthreads();
+    if (!given_up)
+      for (int j = tid; j < n_all; j += SS_THREADS)
+        if (lk[j] >= kth) {
+          const unsigned slot = atomicAdd(&sh[0], 1u);
+          cand_v[slot] = key_float(lk[j]);
+          cand_i[slot] = id_of(j);
+        }
+    __syncthreads();
+  }
+  // is anything that a stretch did not keep among the row's k largest?
+  if (tid < SS_SPLITS && k1 < k && __ldcg(Q.part_key + r * SS_SPLITS + tid) > kth) sh_owner = 1;
+  __syncthreads();
+  if (given_up || sh_owner) {
     if (tid == 0) Q.redo[r] = 1;
     return;
   }
   // pad to a power of two and sort: descending logit, ascending id among equals (bitonic, in shared memory)
   int n_sort = 1;
-  while (n_sort < n_cand) n_sort <<= 1;
+  while (!sorted && n_sort < n_cand) n_sort <<= 1;
   for (int i = n_cand + tid; i < n_sort; i += blockDim.x) { cand_v[i] = -INFINITY; cand_i[i] = 0x7fffffff; }
   __syncthreads();
   for (int size = 2; size <= n_sort; size <<= 1) {
@@ -787,7 +946,7 @@ STRATUM_EXPORT int stratum_sample(const float* logits, int ld, int n_rows, int v
   if (part_v && part_i && part_e && part_key && cand_v && cand_i && counters && redo && vocab >= 8192 &&
       vocab <= SS_SPLITS * SS_CHUNK_MAX) {
     const size_t chunk_bytes = (size_t)((vocab + SS_SPLITS - 1) / SS_SPLITS) * sizeof(float);
-    const size_t list_bytes = (size_t)SS_LIST_MAX * (sizeof(float) + sizeof(int));
+    const size_t list_bytes = (size_t)SS_LIST_MAX * sizeof(uint32_t);
     const size_t smem = chunk_bytes > list_bytes ? chunk_bytes : list_bytes;
     SsScratch Q{part_v, part_i, part_e, part_key, cand_v, cand_i, counters, redo};
     int st = launch_pdl(sample_split_kernel, dim3(n_rows, SS_SPLITS), SS_THREADS, smem, stream, logits, ld, vocab,

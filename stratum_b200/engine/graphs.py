@@ -38,17 +38,15 @@ from .step import Engine, StepDescription, StepEntry, StepError
 
 
 # How a graph picks its tokens: greedy, by a draw, or (many rows with top-k / top-p) by a draw with the sampling kernel
-# that gives a row one block: with filters and more than SAMPLE_SPLIT_MAX_ROWS rows the kernel that cuts a row over
-# 32 blocks queues thousands of blocks for the SMs and loses (110 against 83 us at 64 rows with top-k 50).
+# that gives a row one block (kernels.sample_split_rows).
 PICK_GREEDY, PICK_DRAW, PICK_FILTERED_MANY_ROWS = 0, 1, 2
-SAMPLE_SPLIT_MAX_ROWS = 32
 
 
-def pick_kind(rows: int, temperature: float, top_k: int, top_p: float) -> int:
+def pick_kind(rows: int, temperature: float, top_k: int, top_p: float, vocab: int = 0) -> int:
     if not (temperature > 0.0):
         return PICK_GREEDY
     filtered = top_k > 0 or top_p < 1.0
-    return PICK_FILTERED_MANY_ROWS if filtered and rows > SAMPLE_SPLIT_MAX_ROWS else PICK_DRAW
+    return PICK_FILTERED_MANY_ROWS if filtered and rows > K.sample_split_rows(vocab) else PICK_DRAW
 
 
 def padded_rows(n: int) -> int:
@@ -189,7 +187,7 @@ class DecodeGraphs:
         cache.reserve(slots, ones)
         before = [cache.length(s) for s in slots]
         c = self._get(padded_rows(B), width_bucket(pages_for(max(before) + 1)),
-                      pick_kind(padded_rows(B), temperature, top_k, top_p))
+                      pick_kind(padded_rows(B), temperature, top_k, top_p, eng.vocab))
         if c.graph is None:
             self._capture(c)
         if c.upload_pending:                          # the pinned description is about to be rewritten

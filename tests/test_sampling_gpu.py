@@ -146,3 +146,35 @@ def test_rows_cut_over_blocks_ties_and_odd_rows(vocab):
         for u, g in zip(us, got):
             _lands_in(cum, ids, g, u)
         assert _pick(logits, 0.0, 0, 1.0, us[:3]) == [P.argmax_lowest(logits)] * 3
+
+
+@pytest.mark.parametrize("vocab", [8192, 20011, 128256])
+@pytest.mark.parametrize("k", [1, 2, 63, 64, 65, 127, 128, 129, 300, 512])
+def test_rows_cut_over_blocks_pick_what_one_block_picks(vocab, k):
+    """Filtered draws: the lists of the stretches and the one-block kernel agree bit for bit, whatever lies at the cuts:
+    logits of few distinct values, all equal, zeros of both signs, crowds in one stretch, mostly -inf."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(vocab + k)
+    rows = rng.standard_normal((12, vocab)).astype(np.float32)
+    rows[1] = np.round(rows[1] * 4) / 4                               # dozens of equals at every cut
+    rows[2] = np.round(rows[2] * 64) / 64
+    rows[3] = 1.5
+    rows[4] = np.where(rng.random(vocab) < 0.5, np.float32(0.0), np.float32(-0.0))
+    rows[5, 300:300 + 700] += 20.0                                    # more than any list holds, in three stretches
+    rows[6, vocab - 90:] += 20.0                                      # ... or just what one holds, at the end
+    rows[7] = -np.inf
+    rows[7, rng.permutation(vocab)[:k + 3]] = rng.standard_normal(k + 3)
+    rows[8] = np.sort(rows[8])
+    rows[9] = np.sort(rows[9])[::-1]
+    rows[10] = -np.abs(rows[10]) - 1e-3
+    L = _dev(rows, torch.float32)
+    u = _dev(rng.random(12), torch.float32)
+    got = []
+    for one_block in (False, True):
+        ids = torch.empty(12, dtype=torch.int32, device="cuda")
+        vals = torch.empty(12, dtype=torch.float32, device="cuda")
+        K.sample(L, _dev([1.7] * 12, torch.float32), _dev([k] * 12, torch.int32), _dev([0.97] * 12, torch.float32), u, ids,
+                 vals, one_block_per_row=one_block)
+        got.append((ids.tolist(), vals.tolist()))
+    assert got[0] == got[1]
+    assert all(rows[r, i] == v for r, (i, v) in enumerate(zip(*got[0])))
