@@ -394,49 +394,365 @@ attention_general_mma_kernel(const GeneralAttention P) {
   }
 }
 
+// ---------------------------------------------------------------- decode steps
+// One new token per sequence: a CTA owns (token, key/value head, up to RG groups of 16 of its heads, map, key range) and
+// takes its tiles through a ring of shared memory by cp.async, the next tile's copies under way while one is worked on;
+// values that are a stretch of the key rows are read from the keys' tile.  The kernel above loads its fragments where it
+// needs them, which for a few rows is a chain of round trips to L2: some ten a tile, 5 us.  The arithmetic is the same:
+// four warps per group of rows take 16 keys each for the scores, all warps a share of the value dimensions.
+// Six sequences of 900 to 3,000 tokens, 32 heads of 128: latent rows of 576 20 us against 34 (now bound by mma.sync, whose
+// probabilities go through twice), differential heads of 64 with values of 128 30 against 75.
+template <int RG, int CPW>
+__global__ void __launch_bounds__(RG * GM_WARPS * 32)
+attention_general_decode_kernel(const GeneralAttention P, const int stages) {
+  extern __shared__ __align__(16) unsigned char gm_smem[];
+  constexpr int WARPS = RG * GM_WARPS, THREADS = WARPS * 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int D = P.qk_dim, Dv = P.v_dim, DP = (D + 31) / 32 * 32, kp = DP + 8, vp = P.v_in_k ? kp : (Dv + 31) / 32 * 32 + 8;
+  const int k_tile = GM_TILE * kp, v_tile = P.v_in_k ? 0 : GM_TILE * vp;         // bf16 of a stage
+  bf16* q_s = reinterpret_cast<bf16*>(gm_smem);                                  // [RG * 16][kp]
+  bf16* p_hi = q_s + RG * 16 * kp;                                               // [RG * 16][GM_PSTRIDE]
+  bf16* p_lo = p_hi + RG * 16 * GM_PSTRIDE;
+  float* max_s = reinterpret_cast<float*>(p_lo + RG * 16 * GM_PSTRIDE);          // [RG][GM_WARPS][16]
+  float* sum_s = max_s + RG * GM_WARPS * 16;
+  bf16* ring = reinterpret_cast<bf16*>(sum_s + RG * GM_WARPS * 16);              // [stages][k_tile + v_tile]
+
+  const int head_groups = (P.group + 16 * RG - 1) / (16 * RG), n_kv = P.n_heads / P.group;
+  int item = blockIdx.x;
+  const int split = item % P.n_splits; item /= P.n_splits;
+  const int map = item % P.maps; item /= P.maps;
+  const int hg = item % head_groups; item /= head_groups;
+  const int kv = item % n_kv; item /= n_kv;
+  const int tok = item;
+  const int seq = P.token_seq[tok];
+  if (seq < 0) return;                                                           // padding
+  const int pos = P.token_pos[tok];
+  const int first_head = kv * P.group + hg * 16 * RG, heads_here = min(16 * RG, P.group - hg * 16 * RG);
+  const int lo = general_first_key(P, pos), lo_tile = lo / GM_TILE * GM_TILE;
+  const int k_begin = split * P.chunk, k_end = min(k_begin + P.chunk, pos + 1);
+  const int keep = P.window > 0 ? P.keep_first : 0;
+  const int* bt = P.block_table + (size_t)seq * P.bt_stride;
+  const bf16* k_head = (const bf16*)P.k_cache + (size_t)(kv * P.maps + map) * GM_TILE * D;
+  const bf16* v_head = (const bf16*)P.v_cache + (size_t)kv * GM_TILE * Dv;
+  const size_t k_page = (size_t)P.n_k_heads * GM_TILE * D, v_page = (size_t)P.n_v_heads * GM_TILE * Dv;
+  // tiles wholly in front of the window hold nothing that is seen, unless they hold kept first keys
+  auto from = [&](int key0) { return key0 < lo_tile && key0 >= keep ? lo_tile : key0; };
+  auto copy = [&](bf16* to, const void* src, bool there) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(src),
+                 "r"(there ? 16 : 0)
+                 : "memory");
+  };
+  const int k_pieces = D / 8, v_pieces = P.v_in_k ? 0 : Dv / 8, v_div = v_pieces ? v_pieces : 1;
+  const int k_r0 = threadIdx.x / k_pieces, k_c0 = threadIdx.x % k_pieces, k_dr = THREADS / k_pieces, k_dc = THREADS % k_pieces;
+  const int v_r0 = threadIdx.x / v_div, v_c0 = threadIdx.x % v_div, v_dr = THREADS / v_div, v_dc = THREADS % v_div;
+  auto fetch = [&](int key0, int stage) {            // rows behind the last key become zeros
+    if (key0 < k_end) {
+      const size_t page = bt[key0 / GM_TILE];
+      bf16* kt = ring + (size_t)stage * (k_tile + v_tile);
+      auto rows = [&](bf16* to, int pitch, const bf16* src, int pieces, int r, int c, int dr, int dc) {
+#pragma unroll 4
+        while (r < GM_TILE) {                        // piece after piece, THREADS on
+          copy(to + r * pitch + 8 * c, src + 8 * (r * pieces + c), key0 + r < k_end);
+          r += dr;
+          c += dc;
+          if (c >= pieces) { c -= pieces; r++; }
+        }
+      };
+      rows(kt, kp, k_head + page * k_page, k_pieces, k_r0, k_c0, k_dr, k_dc);
+      if (v_pieces) rows(kt + k_tile, vp, v_head + page * v_page, v_pieces, v_r0, v_c0, v_dr, v_dc);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  int ahead = from(k_begin);                         // the next tile to ask for
+  for (int i = 0; i < stages - 1; i++, ahead = from(ahead + GM_TILE)) fetch(ahead, i);
+
+  const uint4 zero4 = make_uint4(0, 0, 0, 0);
+  for (int i = threadIdx.x; i < RG * 16 * (DP / 8); i += THREADS) {              // queries; rows that do not exist are zero
+    const int r = i / (DP / 8), c = i - r * (DP / 8);
+    *reinterpret_cast<uint4*>(q_s + r * kp + 8 * c) =
+        r < heads_here && 8 * c < D
+            ? ld_fresh((const uint4*)((const bf16*)P.q + (size_t)tok * P.ldq + ((size_t)(first_head + r) * P.maps + map) * D + 8 * c))
+            : zero4;
+  }
+  for (int i = threadIdx.x; i < RG * 16 * GM_PSTRIDE; i += THREADS) p_hi[i] = p_lo[i] = __float2bfloat16_rn(0.f);
+  if (DP != D)                                       // the keys' columns beyond D: no copy touches them
+    for (int i = threadIdx.x; i < stages * GM_TILE * ((DP - D) / 8); i += THREADS) {
+      const int r = i / ((DP - D) / 8), c = i % ((DP - D) / 8);
+      *reinterpret_cast<uint4*>(ring + (size_t)(r / GM_TILE) * (k_tile + v_tile) + (r % GM_TILE) * kp + D + 8 * c) = zero4;
+    }
+
+  const int my_rg = warp / GM_WARPS, my_kb = warp % GM_WARPS;                    // whose scores this warp takes
+  float factor[2], slope[2];
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    const int r = my_rg * 16 + g + 8 * e, head = first_head + (r < heads_here ? r : 0);
+    float temp = 1.f;
+    if (P.temp_coef != 0.f) temp = 1.f + P.temp_coef * logf((float)((pos + 1) / P.temp_every) + 1.f);
+    factor[e] = P.scale * temp * (P.head_scale ? P.head_scale[head] : 1.f);
+    slope[e] = P.slope ? P.slope[head] : 0.f;
+  }
+  float o[RG][CPW * 4][4], m_run[RG][2], l_run[2] = {0.f, 0.f};
+#pragma unroll
+  for (int rg = 0; rg < RG; rg++) {
+#pragma unroll
+    for (int i = 0; i < CPW * 4; i++) { o[rg][i][0] = o[rg][i][1] = o[rg][i][2] = o[rg][i][3] = 0.f; }
+    m_run[rg][0] = m_run[rg][1] = -INFINITY;
+  }
+  const int n_vc = (Dv + 31) / 32;
+  const bool upper = heads_here - my_rg * 16 > 8;    // whether rows 8 .. 15 of this warp's group are anyone's
+  const float inv_cap = P.softcap > 0.f ? 1.0f / P.softcap : 0.f;
+  int stage = 0;
+  for (int key0 = from(k_begin); key0 < k_end; key0 = from(key0 + GM_TILE)) {
+    if (stages == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    else asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();                                 // the tile has landed; the one before is no longer read
+    fetch(ahead, stage == 0 ? stages - 1 : stage - 1);
+    ahead = from(ahead + GM_TILE);
+    const bf16* kt = ring + (size_t)stage * (k_tile + v_tile);
+    const bf16* vt = P.v_in_k ? kt : kt + k_tile;
+    // ---- scores
+    float s[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; i++) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
+    const bf16* qa = q_s + (my_rg * 16 + (lane & 15)) * kp + 8 * (lane >> 4);
+    const bf16* kb = kt + (16 * my_kb + (lane & 7)) * kp + 8 * (lane >> 3);
+#pragma unroll 4
+    for (int d = 0; d < DP; d += 32) {
+      uint32_t a0[4], a1[4], b0[4], b1[4];
+      gm_ldmatrix4(a0, qa + d);
+      gm_ldmatrix4(a1, qa + d + 16);
+      gm_ldmatrix4(b0, kb + d);                      // keys 0 .. 7 of the sixteen, 32 columns
+      gm_ldmatrix4(b1, kb + 8 * kp + d);
+      gm_mma(s[0], a0[0], a0[1], a0[2], a0[3], b0[0], b0[1]);
+      gm_mma(s[1], a0[0], a0[1], a0[2], a0[3], b1[0], b1[1]);
+      gm_mma(s[0], a1[0], a1[1], a1[2], a1[3], b0[2], b0[3]);
+      gm_mma(s[1], a1[0], a1[1], a1[2], a1[3], b1[2], b1[3]);
+    }
+    const bool whole_tile = key0 >= lo && key0 >= k_begin && key0 + GM_TILE <= k_end;
+    float bm[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int e = j >> 1, key = key0 + 16 * my_kb + 8 * i + 2 * t + (j & 1);
+        if (e && !upper) { s[i][j] = 0.f; continue; }
+        float v = s[i][j] * factor[e];
+        if (P.softcap > 0.f) v = P.softcap * tanhf(v * inv_cap);
+        if (P.slope) v -= slope[e] * (float)(pos - key);
+        if (!whole_tile && !(key < k_end && key >= k_begin && (key >= lo || key < keep))) v = -INFINITY;
+        s[i][j] = v;
+        bm[e] = fmaxf(bm[e], v);
+      }
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      bm[e] = fmaxf(bm[e], __shfl_xor_sync(0xffffffffu, bm[e], 1));
+      bm[e] = fmaxf(bm[e], __shfl_xor_sync(0xffffffffu, bm[e], 2));
+      if (t == 0) max_s[warp * 16 + g + 8 * e] = bm[e];
+    }
+    __syncthreads();
+    float corr[RG][2], m_use[RG][2];
+#pragma unroll
+    for (int rg = 0; rg < RG; rg++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const float* mx = max_s + rg * GM_WARPS * 16 + g + 8 * e;
+        const float m_new = fmaxf(m_run[rg][e], fmaxf(fmaxf(mx[0], mx[16]), fmaxf(mx[32], mx[48])));
+        m_use[rg][e] = (m_new == -INFINITY) ? 0.f : m_new;
+        corr[rg][e] = __expf(m_run[rg][e] - m_use[rg][e]);
+        m_run[rg][e] = m_new;
+      }
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const float mu = RG == 2 && my_rg ? m_use[RG - 1][e] : m_use[0][e], co = RG == 2 && my_rg ? corr[RG - 1][e] : corr[0][e];
+      if (e && !upper) continue;                     // (their probabilities stay the zeros they were set to)
+      float psum = 0.f;
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const float p0 = __expf(s[i][2 * e] - mu), p1 = __expf(s[i][2 * e + 1] - mu);
+        psum += p0 + p1;
+        const __nv_bfloat162 hi = __floats2bfloat162_rn(p0, p1);
+        const __nv_bfloat162 low = __floats2bfloat162_rn(p0 - __bfloat162float(hi.x), p1 - __bfloat162float(hi.y));
+        const int at = (my_rg * 16 + g + 8 * e) * GM_PSTRIDE + 16 * my_kb + 8 * i + 2 * t;
+        *reinterpret_cast<__nv_bfloat162*>(p_hi + at) = hi;
+        *reinterpret_cast<__nv_bfloat162*>(p_lo + at) = low;
+      }
+      l_run[e] = l_run[e] * co + psum;
+    }
+    __syncthreads();
+    // ---- values
+#pragma unroll
+    for (int rg = 0; rg < RG; rg++)
+#pragma unroll
+      for (int i = 0; i < CPW * 4; i++) {
+        o[rg][i][0] *= corr[rg][0]; o[rg][i][1] *= corr[rg][0]; o[rg][i][2] *= corr[rg][1]; o[rg][i][3] *= corr[rg][1];
+      }
+    const int blocks = (min(GM_TILE, k_end - key0) + 15) / 16;
+    for (int b16 = 0; b16 < blocks; b16++) {
+      uint32_t hi[RG][4], low[RG][4];
+#pragma unroll
+      for (int rg = 0; rg < RG; rg++) {
+        const int at = (rg * 16 + (lane & 15)) * GM_PSTRIDE + 16 * b16 + 8 * (lane >> 4);
+        gm_ldmatrix4(hi[rg], p_hi + at);
+        gm_ldmatrix4(low[rg], p_lo + at);
+      }
+#pragma unroll
+      for (int cc = 0; cc < CPW; cc++) {
+        const int c = warp + WARPS * cc;
+        if (c >= n_vc) break;
+        const bf16* vb = vt + (16 * b16 + (lane & 15)) * vp + 32 * c + 8 * (lane >> 4);
+        uint32_t b[2][4];
+#pragma unroll
+        for (int h = 0; h < 2; h++)                  // 16 keys by 16 dimensions, transposed
+          asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(b[h][0]), "=r"(b[h][1]), "=r"(b[h][2]), "=r"(b[h][3])
+                       : "r"((uint32_t)__cvta_generic_to_shared(vb + 16 * h)) : "memory");
+#pragma unroll
+        for (int rg = 0; rg < RG; rg++) {
+#pragma unroll
+          for (int i = 0; i < 4; i++)
+            gm_mma(o[rg][4 * cc + i], hi[rg][0], hi[rg][1], hi[rg][2], hi[rg][3], b[i >> 1][2 * (i & 1)], b[i >> 1][2 * (i & 1) + 1]);
+#pragma unroll
+          for (int i = 0; i < 4; i++)
+            gm_mma(o[rg][4 * cc + i], low[rg][0], low[rg][1], low[rg][2], low[rg][3], b[i >> 1][2 * (i & 1)], b[i >> 1][2 * (i & 1) + 1]);
+        }
+      }
+    }
+    stage = stage + 1 == stages ? 0 : stage + 1;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    float l = l_run[e];
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    if (t == 0) sum_s[warp * 16 + g + 8 * e] = l;
+  }
+  __syncthreads();
+  const bool direct = P.n_splits == 1 && P.combine == 0;
+#pragma unroll
+  for (int rg = 0; rg < RG; rg++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int r = rg * 16 + g + 8 * e;
+      if (r >= heads_here) continue;
+      const int head = first_head + r;
+      const float* ls = sum_s + rg * GM_WARPS * 16 + g + 8 * e;
+      float l_all = (ls[0] + ls[16]) + (ls[32] + ls[48]);
+      if (direct && P.sink) l_all += expf(P.sink[head] - m_run[rg][e]);
+      const float inv = 1.0f / l_all;
+      const size_t slot = (((size_t)tok * P.n_heads + head) * P.maps + map) * P.n_splits + split;
+#pragma unroll
+      for (int i = 0; i < CPW * 4; i++) {
+        const int d = 32 * (warp + WARPS * (i >> 2)) + 8 * (i & 3) + 2 * t;
+        if (d >= Dv) continue;                       // v_dim % 8 == 0: a pair of columns is inside or outside together
+        float x = o[rg][i][2 * e], y = o[rg][i][2 * e + 1];
+        if (!direct) {
+          *reinterpret_cast<float2*>(P.part_o + slot * Dv + d) = make_float2(x, y);
+          continue;
+        }
+        x *= inv;
+        y *= inv;
+        if (P.gate) {
+          const float2 z = *reinterpret_cast<const float2*>(P.gate + (size_t)tok * P.ld_gate + (size_t)head * Dv + d);
+          x /= 1.0f + expf(-z.x);
+          y /= 1.0f + expf(-z.y);
+        }
+        *reinterpret_cast<uint32_t*>((bf16*)P.out + (size_t)tok * P.ldo + (size_t)head * Dv + d) = pack_bf16(x, y);
+      }
+      if (!direct && warp == 0 && t == 0) {
+        P.part_ml[slot * 2] = m_run[rg][e];
+        P.part_ml[slot * 2 + 1] = l_all;
+      }
+    }
+}
+
+// Bytes of shared memory of the decode kernel for a shape, with `stages` tiles under way.
+static size_t gm_decode_smem(int qk_dim, int v_dim, int v_in_k, int rg, int stages) {
+  const size_t kp = (qk_dim + 31) / 32 * 32 + 8, vp = v_in_k ? 0 : (v_dim + 31) / 32 * 32 + 8;
+  return 2 * (rg * 16 * kp + 2 * rg * 16 * GM_PSTRIDE + stages * GM_TILE * (kp + vp)) + 2 * rg * GM_WARPS * 16 * sizeof(float);
+}
+
+// Heads of a group that one CTA of the decode kernel takes (16 or 32), or 0 where it does not take the shape: what the
+// host plans key ranges by.  Two groups of 16 where there are as many heads: they share the tile.
+STRATUM_EXPORT int stratum_attention_general_decode_rows(int group, int qk_dim, int v_dim, int v_in_k) {
+  const int rg = group > 16 ? 2 : 1;
+  const int cpw = ((v_dim + 31) / 32 + rg * GM_WARPS - 1) / (rg * GM_WARPS);
+  if (cpw > (rg == 2 ? 2 : 4) || gm_decode_smem(qk_dim, v_dim, v_in_k, rg, 2) > 220 * 1024) return 0;
+  return 16 * rg;
+}
+
+static int gm_decode_stages(int qk_dim, int v_dim, int v_in_k, int rg) {       // three where three CTAs then fit an SM
+  return gm_decode_smem(qk_dim, v_dim, v_in_k, rg, 3) <= 74 * 1024 ? 3 : 2;
+}
+
+// CTAs of a decode step worth planning for (0: the shape is not the decode kernel's).  One to an SM where a CTA takes an SM's
+// shared memory: its two tiles overlap, two waves of single tiles do not (latent rows of 576, six sequences: 26 us with the
+// finishing kernel against 33 with 296 CTAs wanted).  Else several to a place, since sequences are of unequal length
+// (differential heads of 64: 30 us with 592, 35 with 444, 39 with 296, 64 with 148).
+STRATUM_EXPORT int stratum_attention_general_decode_ctas(int group, int qk_dim, int v_dim, int v_in_k) {
+  const int rows = stratum_attention_general_decode_rows(group, qk_dim, v_dim, v_in_k);
+  if (rows == 0) return 0;
+  const size_t smem = gm_decode_smem(qk_dim, v_dim, v_in_k, rows / 16, gm_decode_stages(qk_dim, v_dim, v_in_k, rows / 16));
+  return smem > 113 * 1024 ? 148 : 148 * 4;
+}
+
 // Merge the key ranges of every (token, head, map) in range order, then combine the maps; one block per
-// (token, head), one thread per value dimension.  A range that held no key of a row left maximum -inf and sum 0
+// (token, head).  A range that held no key of a row left maximum -inf and sum 0
 // and drops out.
-#define GM_MAX_SPLITS 64
+#define GM_MAX_SPLITS 64          // two to a lane of the finishing kernel
+#define GM_FIN_THREADS 256
 template <int MAPS>
-__global__ void __launch_bounds__(128) attention_general_finish_kernel(const GeneralAttention P) {
+__global__ void __launch_bounds__(GM_FIN_THREADS) attention_general_finish_kernel(const GeneralAttention P) {
   __shared__ float weight[MAPS][GM_MAX_SPLITS];
+  __shared__ __align__(16) float sums[MAPS][4 * GM_FIN_THREADS];
   __shared__ float scratch[33];
-  const int item = blockIdx.x;
+  const int item = blockIdx.x, tid = threadIdx.x;
   const int tok = item / P.n_heads, h = item - tok * P.n_heads;
   if (P.token_seq[tok] < 0) return;
   const int Dv = P.v_dim, S = P.n_splits;
-  if (threadIdx.x < MAPS) {
-    const int m = threadIdx.x;
-    const float* ml = P.part_ml + ((size_t)item * MAPS + m) * S * 2;
-    float mx = -INFINITY;
-    for (int s = 0; s < S; s++) mx = fmaxf(mx, ml[2 * s]);
-    float l = 0.f;
-    for (int s = 0; s < S; s++) {
-      const float w = ml[2 * s] == -INFINITY ? 0.f : expf(ml[2 * s] - mx);
-      weight[m][s] = w;
-      l += ml[2 * s + 1] * w;
-    }
+  if (tid < 32 * MAPS) {                             // a warp a map, a lane two ranges (one thread through all of them was a
+    const int m = tid >> 5, lane = tid & 31;         // chain of loads: 12 of the 15 us that 24 ranges took)
+    const float2* ml = reinterpret_cast<const float2*>(P.part_ml) + ((size_t)item * MAPS + m) * S;
+    const float2 none = make_float2(-INFINITY, 0.f);
+    const float2 a = lane < S ? ml[lane] : none, b = lane + 32 < S ? ml[lane + 32] : none;
+    const float mx = warp_max(fmaxf(a.x, b.x));
+    const float wa = a.x == -INFINITY ? 0.f : expf(a.x - mx), wb = b.x == -INFINITY ? 0.f : expf(b.x - mx);
+    float l = warp_sum(a.y * wa + b.y * wb);
     if (P.sink) l += expf(P.sink[h] - mx);
     const float inv = 1.0f / l;
-    for (int s = 0; s < S; s++) weight[m][s] *= inv;
+    weight[m][lane] = wa * inv;
+    weight[m][lane + 32] = wb * inv;
+  }
+  __syncthreads();
+  // thread (q, part): four neighbouring dimensions, every n_parts-th range; the parts are added in order
+  const int quads = Dv / 4, width = quads > 64 ? 128 : quads > 32 ? 64 : 32;           // v_dim % 8 == 0, v_dim <= 512
+  const int q = tid % width, part = tid / width, n_parts = GM_FIN_THREADS / width;
+#pragma unroll
+  for (int m = 0; m < MAPS; m++) {
+    if (q >= quads) break;
+    const float4* po = reinterpret_cast<const float4*>(P.part_o + ((size_t)item * MAPS + m) * S * Dv) + q;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int s = part; s < S; s += n_parts) {
+      const float w = weight[m][s];
+      const float4 v = po[(size_t)s * quads];
+      acc.x = fmaf(v.x, w, acc.x); acc.y = fmaf(v.y, w, acc.y); acc.z = fmaf(v.z, w, acc.z); acc.w = fmaf(v.w, w, acc.w);
+    }
+    *reinterpret_cast<float4*>(&sums[m][part * Dv + 4 * q]) = acc;
   }
   __syncthreads();
   bf16* op = (bf16*)P.out + (size_t)tok * P.ldo + (size_t)h * Dv;
-  float o[4], ss = 0.f;                              // v_dim <= 512: at most four dimensions per thread
+  float o[2], ss = 0.f;                              // at most two dimensions a thread
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int d = threadIdx.x + 128 * i;
+  for (int i = 0; i < 2; i++) {
+    const int d = tid + GM_FIN_THREADS * i;
     o[i] = 0.f;
     if (d >= Dv) continue;
     float a[MAPS];
 #pragma unroll
     for (int m = 0; m < MAPS; m++) {
-      const float* po = P.part_o + ((size_t)item * MAPS + m) * S * Dv + d;
-      float acc = 0.f;
-#pragma unroll 4
-      for (int s = 0; s < S; s++) acc = fmaf(po[(size_t)s * Dv], weight[m][s], acc);
-      a[m] = acc;
+      a[m] = sums[m][d];
+      for (int g = 1; g < n_parts; g++) a[m] += sums[m][g * Dv + d];
     }
     if (MAPS == 1) {
       float r = a[0];
@@ -455,8 +771,8 @@ __global__ void __launch_bounds__(128) attention_general_finish_kernel(const Gen
     mul *= 1.0f / (1.0f + expf(-z));
   }
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int d = threadIdx.x + 128 * i;
+  for (int i = 0; i < 2; i++) {
+    const int d = tid + GM_FIN_THREADS * i;
     if (d < Dv) op[d] = __float2bfloat16_rn(o[i] * mul);
   }
 }
@@ -505,29 +821,44 @@ STRATUM_EXPORT int stratum_attention_general_mma(const GeneralAttention* params,
   if (!direct && (!P.part_o || !P.part_ml)) return STRATUM_ERR_SHAPE;
   const int n_vc = (P.v_dim + 31) / 32;
   const int cpw = (n_vc + GM_WARPS - 1) / GM_WARPS;
-  // groups of 16 rows per CTA: as many as the accumulators leave registers for (prompts; decode steps have one)
-  const int rg = P.reserved <= 1 ? 1 : P.reserved;
-  if (rg > 2) return STRATUM_ERR_SHAPE;
-  const size_t smem = (size_t)stratum_attention_general_mma_smem(P.qk_dim, rg);
-  if (smem > 200 * 1024) return STRATUM_ERR_LIMIT;
-  const int head_groups = (P.group + 15) / 16;
-  const long long items = (long long)P.n_qblocks * (P.n_heads / P.group) * head_groups * P.maps * P.n_splits;
-  if (items > 0x7fffffffLL) return STRATUM_ERR_LIMIT;
   void (*kern)(const GeneralAttention) = nullptr;
-  if (cpw <= 1) kern = rg == 1 ? attention_general_mma_kernel<1, 1> : attention_general_mma_kernel<1, 2>;
-  else if (cpw <= 2) kern = rg == 1 ? attention_general_mma_kernel<2, 1> : attention_general_mma_kernel<2, 2>;
-  else if (cpw <= 4) kern = rg == 1 ? attention_general_mma_kernel<4, 1> : attention_general_mma_kernel<4, 2>;
-  else return STRATUM_ERR_LIMIT;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const int decode_rows = P.dense || P.qb_seq || (P.v_in_k && P.maps > 1) ? 0 : stratum_attention_general_decode_rows(P.group, P.qk_dim, P.v_dim, P.v_in_k);
+  if (decode_rows) {
+    const int rg = decode_rows / 16;
+    const int stages = gm_decode_stages(P.qk_dim, P.v_dim, P.v_in_k, rg);
+    const size_t smem = gm_decode_smem(P.qk_dim, P.v_dim, P.v_in_k, rg, stages);
+    const long long items = (long long)P.n_qblocks * (P.n_heads / P.group) * ((P.group + decode_rows - 1) / decode_rows) * P.maps * P.n_splits;
+    if (items > 0x7fffffffLL) return STRATUM_ERR_LIMIT;
+    void (*dec)(const GeneralAttention, int) = nullptr;
+    if (rg == 2) dec = n_vc <= 8 ? attention_general_decode_kernel<2, 1> : attention_general_decode_kernel<2, 2>;
+    else dec = cpw <= 1 ? attention_general_decode_kernel<1, 1> : cpw <= 2 ? attention_general_decode_kernel<1, 2> : attention_general_decode_kernel<1, 4>;
+    cudaError_t e = cudaFuncSetAttribute(dec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
+    dec<<<(unsigned)items, rg * GM_WARPS * 32, smem, stream>>>(P, stages);
+  } else {
+    // groups of 16 rows per CTA: as many as the accumulators leave registers for (prompts; decode steps have one)
+    const int rg = P.reserved <= 1 ? 1 : P.reserved;
+    if (rg > 2) return STRATUM_ERR_SHAPE;
+    const size_t smem = (size_t)stratum_attention_general_mma_smem(P.qk_dim, rg);
+    if (smem > 200 * 1024) return STRATUM_ERR_LIMIT;
+    const int head_groups = (P.group + 15) / 16;
+    const long long items = (long long)P.n_qblocks * (P.n_heads / P.group) * head_groups * P.maps * P.n_splits;
+    if (items > 0x7fffffffLL) return STRATUM_ERR_LIMIT;
+    if (cpw <= 1) kern = rg == 1 ? attention_general_mma_kernel<1, 1> : attention_general_mma_kernel<1, 2>;
+    else if (cpw <= 2) kern = rg == 1 ? attention_general_mma_kernel<2, 1> : attention_general_mma_kernel<2, 2>;
+    else if (cpw <= 4) kern = rg == 1 ? attention_general_mma_kernel<4, 1> : attention_general_mma_kernel<4, 2>;
+    else return STRATUM_ERR_LIMIT;
+    if (smem > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return (int)e;
+    }
+    kern<<<(unsigned)items, GM_WARPS * 32, smem, stream>>>(P);
   }
-  kern<<<(unsigned)items, GM_WARPS * 32, smem, stream>>>(P);
   int st = launch_status();
   if (st || direct) return st;
   const long long rows = (long long)P.n_tokens * P.n_heads;
   if (rows > 0x7fffffffLL) return STRATUM_ERR_LIMIT;
-  if (P.maps == 1) attention_general_finish_kernel<1><<<(unsigned)rows, 128, 0, stream>>>(P);
-  else attention_general_finish_kernel<2><<<(unsigned)rows, 128, 0, stream>>>(P);
+  if (P.maps == 1) attention_general_finish_kernel<1><<<(unsigned)rows, GM_FIN_THREADS, 0, stream>>>(P);
+  else attention_general_finish_kernel<2><<<(unsigned)rows, GM_FIN_THREADS, 0, stream>>>(P);
   return launch_status();
 }

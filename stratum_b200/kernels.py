@@ -827,6 +827,23 @@ def attention_general_mma_ok(shape: AttentionShape, q: torch.Tensor, out: torch.
             and (gate is None or (gate.stride(0) % 4 == 0 and gate.data_ptr() % 16 == 0)))
 
 
+def attention_general_decode_rows(shape: AttentionShape) -> int:
+    """Heads of a group that one CTA of a decode step of attention_general_mma takes: what key ranges are planned by."""
+    return _general_decode(shape)[0] or 16
+
+
+def attention_general_decode_ctas(shape: AttentionShape) -> int:
+    """CTAs such a step is planned for (0: no opinion)."""
+    return _general_decode(shape)[1]
+
+
+def _general_decode(shape: AttentionShape) -> Tuple[int, int]:
+    if shape.v_in_k and shape.maps > 1:
+        return 0, 0
+    lib, sizes = build.load("attention_general_mma"), (shape.group, shape.qk_dim, shape.v_dim, int(shape.v_in_k))
+    return lib.stratum_attention_general_decode_rows(*sizes), lib.stratum_attention_general_decode_ctas(*sizes)
+
+
 def attention_general_mma_row_groups(v_dim: int) -> int:
     """Groups of 16 query rows a CTA of the tensor-core general attention takes in prompt steps."""
     return int(build.load("attention_general_mma").stratum_attention_general_mma_row_groups(int(v_dim)))

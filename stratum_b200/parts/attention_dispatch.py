@@ -82,21 +82,20 @@ def run(att, qkv: torch.Tensor, cache, step, out: torch.Tensor) -> None:
                          PAGE_TOKENS, att.window, att.scale)
 
 
-# CTAs wanted on decode steps of the general attention: two to an SM of 148.  Measured at batch 8 and 4,090 cached
-# tokens, four layers (three latent, one differential): 0.166 ms with 296 against 0.209 / 0.197 / 0.191 with 148 /
-# 592 / 1,184 on a 2,048-wide model, 0.288 against 0.388 / 0.344 / 0.417 on a 4,096-wide one: more ranges are more
-# partial results for the finishing kernel to merge, fewer leave SMs idle.
-GENERAL_TARGET_CTAS = int(os.environ.get("STRATUM_GENERAL_ATTENTION_CTAS", 148 * 2))
+# CTAs wanted on decode steps of the general attention where its decode kernel names no number of its own: two to an SM
+# of 148 (STRATUM_GENERAL_ATTENTION_CTAS: that many for every shape; measurements)
+GENERAL_TARGET_CTAS = int(os.environ.get("STRATUM_GENERAL_ATTENTION_CTAS", 0))
 GENERAL_MAX_SPLITS = 64
 
 
-def plan_general_splits(n_items: int, max_len: int, window: int = 0):
+def plan_general_splits(n_items: int, max_len: int, window: int = 0, ctas: int = 0):
     """(n_splits, keys per split) for decode steps of the general attention: whole pages per split.  Ranges are
     counted from position 0 for every sequence; with a window only the last ones hold keys a row can see (the others
     leave at once), so the ranges are sized to cut the window's stretch, not the whole sequence, into enough pieces."""
+    ctas = GENERAL_TARGET_CTAS or ctas or 148 * 2
     pages = max(1, (max_len + PAGE_TOKENS - 1) // PAGE_TOKENS)
     seen = pages if window <= 0 else min(pages, (window + PAGE_TOKENS - 1) // PAGE_TOKENS + 1)
-    want = max(1, min(seen, GENERAL_MAX_SPLITS, (GENERAL_TARGET_CTAS + n_items - 1) // n_items))
+    want = max(1, min(seen, GENERAL_MAX_SPLITS, (ctas + n_items - 1) // n_items))
     per = max((seen + want - 1) // want, (pages + GENERAL_MAX_SPLITS - 1) // GENERAL_MAX_SPLITS)
     chunk = per * PAGE_TOKENS
     return (max_len + chunk - 1) // chunk, chunk
@@ -147,11 +146,13 @@ def run_general(att, shape, q: torch.Tensor, cache, step, out: torch.Tensor, gat
         return
     rows_per_token = min(shape.group, 16)
     per_block = 16 // rows_per_token
-    streams = (shape.n_heads // shape.group) * ((shape.group + 15) // 16) * shape.maps
     row_groups = 1
     if step.all_single:
         qblocks = None
-        n_splits, chunk = plan_general_splits(step.n_tokens * streams, step.max_len, shape.span)
+        rows = K.attention_general_decode_rows(shape)
+        streams = (shape.n_heads // shape.group) * ((shape.group + rows - 1) // rows) * shape.maps
+        n_splits, chunk = plan_general_splits(step.n_tokens * streams, step.max_len, shape.span,
+                                              K.attention_general_decode_ctas(shape))
     else:
         # prompts: a CTA takes several groups of 16 rows through every tile of keys, which then comes from L2 once
         row_groups = K.attention_general_mma_row_groups(shape.v_dim)

@@ -525,3 +525,50 @@ def test_long_prompts_take_the_per_head_form(setup, monkeypatch):
     engine.release(s)
     assert not any(dense_calls)
     assert_close(second, refs[0][[299]], dtype, f"{name} continued portion")
+
+
+@pytest.mark.parametrize("heads,group,maps,D,Dv,v_in_k,extra", [
+    (32, 32, 1, 576, 512, True, {}), (20, 20, 1, 48, 40, True, {"window": 70}), (40, 40, 1, 104, 96, True, {"keep_first": 3, "window": 90}),
+    (8, 4, 2, 64, 128, False, {"softcap": 30.0, "temp_coef": 0.1, "temp_every": 50}), (6, 3, 2, 72, 24, False, {"softcap": 5.0}),
+    (16, 16, 1, 256, 512, False, {}), (9, 9, 1, 8, 8, False, {"chunk": 100}), (4, 1, 1, 128, 128, False, {"sink": True})])
+@pytest.mark.parametrize("plan", [(1, 384), (6, 64), (3, 128)])
+def test_general_attention_of_decode_steps(heads, group, maps, D, Dv, v_in_k, extra, plan):
+    """Single tokens against the CUDA-core kernel: whole and half groups of 16 heads, sizes that fill no block of 32, tiles
+    cut at a token's position, a padding row; keys and values behind a token's position are NaN and reach nobody."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(D + Dv + group)
+    kv = heads // group
+    lens = [1, 64, 65, 380, 200]
+    pages = 32
+    kc = torch.full((pages, kv * maps, 64, D), float("nan"), dtype=torch.bfloat16, device="cuda")
+    vc = None if v_in_k else torch.full((pages, kv, 64, Dv), float("nan"), dtype=torch.bfloat16, device="cuda")
+    order = rng.permutation(pages).tolist()
+    table = np.full((len(lens), 6), -1)
+    put = lambda *shape: torch.tensor(rng.standard_normal(shape), dtype=torch.bfloat16, device="cuda")
+    for s, n in enumerate(lens):
+        for p in range((n + 63) // 64):
+            table[s, p] = order.pop()
+            m = min(64, n - 64 * p)
+            kc[table[s, p], :, :m] = put(kv * maps, m, D)
+            if vc is not None:
+                vc[table[s, p], :, :m] = put(kv, m, Dv)
+    extra = dict(extra)
+    if extra.pop("sink", False):
+        extra["sink"] = torch.tensor(rng.standard_normal(heads), dtype=torch.float32, device="cuda")
+    shape = K.AttentionShape(heads, group, maps, D, Dv, v_in_k, D ** -0.5, lam=0.3, out_scale=0.8, eps=1e-6, **extra)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    T = len(lens) + 1
+    q = put(T, heads * maps * D) if (heads * maps * D) % 8 == 0 else None
+    pos, seq = i32([n - 1 for n in lens] + [0]), i32(list(range(len(lens))) + [-1])
+    out = torch.zeros(T, heads * Dv, dtype=torch.bfloat16, device="cuda")
+    ref = torch.zeros(T, heads * Dv, dtype=torch.bfloat16, device="cuda")
+    K.attention_general(shape, q, kc, vc, pos, seq, i32(table), ref, 64)
+    assert K.attention_general_mma_ok(shape, q, out, 64) and K.attention_general_decode_rows(shape) == (32 if group > 16 else 16)
+    splits, chunk = plan
+    n = T * heads * maps * splits
+    K.attention_general_mma(shape, q, kc, vc, pos, seq, i32(table), out, 64, None, 1, splits, chunk,
+                            torch.empty(n * Dv, device="cuda"), torch.empty(2 * n, device="cuda"))
+    assert bool(torch.isfinite(ref).all()) and bool(torch.isfinite(out).all())
+    assert not out[-1].any()
+    # both round once to bfloat16; between them the probabilities' 16 bits
+    assert float((out.float() - ref.float()).abs().max()) <= 2.0 ** -7 * float(ref.float().abs().max())
