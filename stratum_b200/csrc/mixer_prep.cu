@@ -15,8 +15,8 @@
 //
 // gate_heads: a[t][j * block + i] *= sigmoid(g[t][j]): every head's stretch of a row times the head's gate, whose
 // pre-activation is a column of a projection.
-// Everything is evaluated in float32 and rounded once to the storage type.  One block per token; the order of
-// every sum depends on the row alone.
+// Everything is evaluated in float32 and rounded once to the storage type.  A block per token, or several (MP_BLOCKS) where
+// a step has few tokens; the order of every sum depends on the row alone.
 #include <math.h>
 
 #include "common.cuh"
@@ -42,6 +42,11 @@ struct MixerPrep {
   int k_out_ld, interleaved;
 };
 
+// Steps of up to 64 tokens give a token eight blocks: with one, six tokens of 32 heads were a chain of 16 to 48 turns of a
+// block on six SMs, 8.6 us; now 4.3.  (More tokens fill the SMs by themselves, and every block evaluates the angles.)
+#define MP_FEW_TOKENS 64
+#define MP_BLOCKS 8
+
 template <typename T>
 __global__ void __launch_bounds__(128) mixer_prep_kernel(const MixerPrep P) {
   extern __shared__ float2 mp_cs[];                 // [rot_pairs] (cos, sin)
@@ -51,7 +56,7 @@ __global__ void __launch_bounds__(128) mixer_prep_kernel(const MixerPrep P) {
   const int seq = P.token_seq[t];
   if (seq < 0) {                                    // a padding token
     pdl_wait();
-    if (P.k_out) {
+    if (P.k_out && blockIdx.y == 0) {
       T* ko = (T*)P.k_out + (size_t)t * P.k_out_ld;
       for (int d = threadIdx.x; d < P.n_k * P.k_dim; d += blockDim.x) ko[d] = from_float<T>(0.f);
     }
@@ -73,7 +78,8 @@ __global__ void __launch_bounds__(128) mixer_prep_kernel(const MixerPrep P) {
   // queries: rotate in place, or into q_out together with what follows the rotated dimensions
   const int tail = P.q_out ? P.q_dim - P.q_rot_off - 2 * R : 0;
   T* qo = P.q_out ? (T*)P.q_out + (size_t)t * P.q_out_ld + P.q_out_off : nullptr;
-  for (int it = threadIdx.x; it < P.n_q * (R + tail); it += blockDim.x) {
+  const int first = blockIdx.y * blockDim.x + threadIdx.x, stride = gridDim.y * blockDim.x;    // a token's blocks share its work
+  for (int it = first; it < P.n_q * (R + tail); it += stride) {
     const int j = it / (R + tail), i = it - j * (R + tail);
     T* u = x + P.q_col + (size_t)j * P.q_dim + P.q_rot_off;
     T* w = qo ? qo + (size_t)j * P.q_out_step : u;
@@ -88,7 +94,7 @@ __global__ void __launch_bounds__(128) mixer_prep_kernel(const MixerPrep P) {
     }
   }
   if (!P.write_cache) return;
-  for (int j = 0; j < P.n_k; j++) {
+  for (int j = gridDim.y - 1 - blockIdx.y; j < P.n_k; j += gridDim.y) {
     const T* k = x + P.k_col + (size_t)j * P.k_dim;
     T* dst = (T*)P.k_cache + ((row * P.n_k + j) * P.page_tokens + in_page) * (size_t)P.k_dim;
     float mul = 1.f;
@@ -123,7 +129,7 @@ __global__ void __launch_bounds__(128) mixer_prep_kernel(const MixerPrep P) {
       if (P.k_out) ((T*)P.k_out)[(size_t)t * P.k_out_ld + (size_t)j * P.k_dim + d] = from_float<T>(v);
     }
   }
-  for (int it = threadIdx.x; it < P.n_v * P.v_dim; it += blockDim.x) {
+  for (int it = first; it < P.n_v * P.v_dim; it += stride) {
     const int j = it / P.v_dim, d = it - j * P.v_dim;
     T* dst = (T*)P.v_cache + ((row * P.n_v + j) * P.page_tokens + in_page) * (size_t)P.v_dim;
     dst[d] = from_float<T>(ld_fresh(x + P.v_col + it));
@@ -173,7 +179,8 @@ STRATUM_EXPORT int stratum_mixer_prep(const MixerPrep* params, int dtype, cudaSt
     return STRATUM_ERR_SHAPE;
   const size_t smem = (size_t)P.rot_pairs * sizeof(float2);
   if (smem > 40 * 1024) return STRATUM_ERR_LIMIT;
-  if (dtype == STRATUM_DT_F32) return launch_pdl(mixer_prep_kernel<float>, P.n_tokens, 128, smem, stream, P);
-  if (dtype == STRATUM_DT_BF16) return launch_pdl(mixer_prep_kernel<bf16>, P.n_tokens, 128, smem, stream, P);
+  const dim3 grid(P.n_tokens, P.n_tokens <= MP_FEW_TOKENS ? MP_BLOCKS : 1);
+  if (dtype == STRATUM_DT_F32) return launch_pdl(mixer_prep_kernel<float>, grid, 128, smem, stream, P);
+  if (dtype == STRATUM_DT_BF16) return launch_pdl(mixer_prep_kernel<bf16>, grid, 128, smem, stream, P);
   return STRATUM_ERR_DTYPE;
 }
