@@ -363,11 +363,13 @@ attention_f32_cluster_kernel(const PagedF32 p) {
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int t = blockIdx.y, kvh = blockIdx.z, group = p.n_q / p.n_kv;
+  pdl_trigger();
   const int seq = p.token_seq[t], pos = p.token_pos[t];
+  pdl_wait();                                    // queries and the newest keys and values come from kernels before this one
   if (seq < 0) return;                           // padding token (of the whole cluster)
   const int lo = p.window > 0 && pos - p.window + 1 > 0 ? pos - p.window + 1 : 0;
   const int* bt = p.block_table + (size_t)seq * p.bt_stride;
-  for (int c = tid; c < group * HD; c += 128) qs[c] = p.q[(size_t)t * p.ldq + (size_t)kvh * group * HD + c];
+  for (int c = tid; c < group * HD; c += 128) qs[c] = ld_fresh(p.q + (size_t)t * p.ldq + (size_t)kvh * group * HD + c);
 
   const int first_page = lo / AF_PAGE, last_page = pos / AF_PAGE;
   const int e = rank * (group * HD / AF_CLUSTER) + tid;                   // the output element this thread merges
@@ -441,8 +443,7 @@ static int launch_attention_f32(const PagedF32& p, cudaStream_t stream) {
     const int smem = (AF_MAX_GROUP * HD + 2 * 64 * (HD + 4) + AF_MAX_GROUP * (AF_PAGE + 4)) * 4;
     static int once = (int)cudaFuncSetAttribute(attention_f32_cluster_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (once) return once;
-    attention_f32_cluster_kernel<HD><<<dim3(AF_CLUSTER, p.n_tokens, p.n_kv), 128, smem, stream>>>(p);
-    return launch_status();
+    return launch_pdl(attention_f32_cluster_kernel<HD>, dim3(AF_CLUSTER, p.n_tokens, p.n_kv), 128, smem, stream, p);
   }
   const int smem = (3 * 64 * (HD + 4) + 64 * (AF_PAGE + 4)) * 4, per = 64 / group;
   static int once = (int)cudaFuncSetAttribute(attention_f32_tile_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

@@ -111,10 +111,10 @@ static int launch_linear_simple(const void* x, const void* w, const float* bias,
 // tiles of 64 or 32 rows by 128 columns in registers.  Measured by themselves with a cold L2 (us; the one kernel of scalar
 // FMA on 64 x 64 tiles that served every shape before in brackets):
 //   rows of x               1            8            64           611
-//   N 3072   K 2048      14 (176)     19 (176)     38 (181)    192 (488)
-//   N 16384  K 2048      47 (254)     54 (257)    128 (278)    949 (2079)
-//   N 2048   K 8192      35 (706)     41 (707)     67 (721)    462 (1427)
-//   N 128256 K 2048     244 (1431)   311 (1455)
+//   N 3072   K 2048      14 (176)     18 (176)     38 (181)    192 (488)
+//   N 16384  K 2048      45 (254)     51 (257)    128 (278)    949 (2079)
+//   N 2048   K 8192      25 (706)     31 (707)     67 (721)    462 (1427)
+//   N 128256 K 2048     219 (1431)   285 (1455)
 // and the error against 64 bits is 2.1e-7 (8.1e-7) at K 2048, 4.1e-7 (1.6e-6) at 8192: shorter chains.  The line between
 // the two lies at eight rows: 13 rows as two groups of eight took 90, 50 and 605 us on the last three shapes, 17 rows on
 // a tile of 32 rows 77, 48 and 432.
@@ -171,60 +171,98 @@ struct F32Product {
 __device__ __forceinline__ void f32_finish(const F32Product& p, int head, int m, int n, float v) {
   if (p.bias) v += p.bias[n];
   float* o = p.out + (size_t)m * p.ldo + n + (size_t)head * p.o_step;
-  if (p.epilogue == 1) *o += v;
+  if (p.epilogue == 1) *o = ld_fresh(o) + v;
   else *o = p.epilogue == 0 ? activate(v, p.act) : v;
 }
 
 // Few rows of x: bound by the bytes of W.  A thread owns one (row of W, segment) and all MR rows of x; a warp streams
-// its 32 stretches of W through a ring of its own (cp.async, four stages of 4 KB: 147 KB in flight on an SM with two
-// blocks), so nothing but the sum over the segments at the end needs the block.  The rows of x come with W's stages.
-template <int MR, bool VEC>
+// its 32 stretches of W through a ring of its own (cp.async, 4 KB a stage), so nothing but the sum over the segments needs
+// the block.  The rows of x come with W's stages.  A block goes from tile to tile (of 128 / segments rows of W) with
+// its ring full, and fills it before it waits for the kernel in front of it.  STAGES: 4, two blocks to an SM; where the
+// tiles are fewer than the SMs 8, so that the one block of an SM still has 130 KB in flight.
+// In a chain of launches, 1 / 3 / 8 rows of x: 16,384 x 2,048 28 / 32 / 41 us (4.8 / 4.2 / 3.3 TB/s of W), 128,256 x 2,048
+// 198 / 213 / 276, 2,048 x 8,192 16 / 20 / 23.  (Two rows of W a thread, for half as many loads of x, and half as many warps:
+// 26 / 33 / 38, 188 / 209 / 261 and 18 / 23 / 31.)
+template <int MR, bool VEC, int STAGES>
 __global__ void __launch_bounds__(128)
 linear_f32_few_kernel(const F32Product p, const int rows_per_block /* 128 / segments rounded up to a power of two */) {
-  constexpr int STAGES = 4, W_FLOATS = 32 * F32_PITCH, X_FLOATS = 2 * MR * F32_PITCH;
+  constexpr int W_FLOATS = 32 * F32_PITCH, X_FLOATS = 2 * MR * F32_PITCH;
   extern __shared__ __align__(16) float smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, head = blockIdx.z;
-  float* ring = smem + warp * STAGES * (W_FLOATS + X_FLOATS);
+  float* sums = smem;                            // [MR][128]
+  float* ring = smem + MR * 128 + warp * STAGES * (W_FLOATS + X_FLOATS);
   const float* w = p.w + (size_t)head * p.w_step;
   const float* x = p.x + (size_t)head * p.x_step;
-  const int n0 = blockIdx.x * rows_per_block;
-  // what this lane copies in each of eight rounds: 16 bytes of row (round * 4 + lane / 8) of the warp's 32
-  const int ck = (lane & 7) * 4;
+  const int tiles = (p.N + rows_per_block - 1) / rows_per_block, iters = p.segment / F32_BK;
+  const int my_tiles = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x, total = my_tiles * iters;
   const int warp_segments = rows_per_block < 32 ? 32 / rows_per_block : 1;      // 1 or 2
   const int first_segment = warp * 32 / rows_per_block;
-  const int iters = (p.segment + F32_BK - 1) / F32_BK;
+  // what this lane copies of W in each of eight rounds: 16 bytes of row (round * 4 + lane / 8) of the warp's 32.  The rows'
+  // places are worked out once: in every stage they were half of the kernel's instructions, and its bound (51 against 42 us
+  // for 16,384 + 3,072 rows of 2,048).
+  const int ck = (lane & 7) * 4, row0 = lane >> 3;
+  long long place[8];
+#pragma unroll
+  for (int r = 0; r < 8; r++) {
+    const int id = warp * 32 + r * 4 + row0;
+    place[r] = (long long)(id % rows_per_block) * p.K + (id / rows_per_block) * p.segment;
+  }
+  const bool whole = VEC && p.K == p.segments * p.segment && rows_per_block * p.segments == 128 && p.N % rows_per_block == 0;
 
-  auto fetch = [&](int it) {
-    float* st = ring + (it % STAGES) * (W_FLOATS + X_FLOATS);
+  auto fetch_w = [&](int tile, int it, int stage) {
+    float* st = ring + stage * (W_FLOATS + X_FLOATS) + row0 * F32_PITCH + ck;
+    if (whole) {                                 // every copy is there
+      const float* from = w + (size_t)tile * rows_per_block * p.K + it * F32_BK + ck;
+      const unsigned to = (unsigned)__cvta_generic_to_shared(st);
+#pragma unroll
+      for (int r = 0; r < 8; r++)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + r * 16 * F32_PITCH), "l"(from + place[r]) : "memory");
+      return;
+    }
 #pragma unroll
     for (int r = 0; r < 8; r++) {
-      const int row = r * 4 + (lane >> 3), id = warp * 32 + row;
-      const int n = n0 + id % rows_per_block, s = id / rows_per_block;
-      copy4<VEC>(st + row * F32_PITCH + ck, w + (size_t)(n < p.N ? n : 0) * p.K, s * p.segment + it * F32_BK + ck, p.K,
+      const int id = warp * 32 + r * 4 + row0;
+      const int n = tile * rows_per_block + id % rows_per_block, s = id / rows_per_block;
+      copy4<VEC>(st + r * 4 * F32_PITCH, w + (size_t)(n < p.N ? n : 0) * p.K, s * p.segment + it * F32_BK + ck, p.K,
                  n < p.N && s < p.segments);
     }
+  };
+  auto fetch_x = [&](int it, int stage) {
+    float* st = ring + stage * (W_FLOATS + X_FLOATS) + W_FLOATS;
     for (int c = lane; c < warp_segments * MR * 8; c += 32) {
       const int row = c >> 3, m = row % MR, s = first_segment + row / MR;
-      copy4<VEC>(st + W_FLOATS + row * F32_PITCH + (c & 7) * 4, x + (size_t)(m < p.M ? m : 0) * p.ldx,
+      copy4<VEC>(st + row * F32_PITCH + (c & 7) * 4, x + (size_t)(m < p.M ? m : 0) * p.ldx,
                  s * p.segment + it * F32_BK + (c & 7) * 4, p.K, m < p.M && s < p.segments);
     }
   };
-
+  pdl_trigger();
+  // the next stage to ask for: tile, stage of it, place in the ring
+  int f_tile = blockIdx.x, f_it = 0, f_stage = 0;
+  auto next = [&]() {
+    if (++f_it == iters) { f_it = 0; f_tile += gridDim.x; }
+    f_stage = f_stage + 1 == STAGES ? 0 : f_stage + 1;
+  };
+  for (int j = 0; j < STAGES - 1 && j < total; j++, next()) fetch_w(f_tile, f_it, f_stage);
+  pdl_wait();                                    // x, and what is added into, are the work of kernels before this one
+  for (int j = 0, it = 0; j < STAGES - 1; j++, it = it + 1 == iters ? 0 : it + 1) {
+    if (j < total) fetch_x(it, j);
+    copies_commit();
+  }
   f32x2 acc[MR];
 #pragma unroll
   for (int m = 0; m < MR; m++) acc[m] = 0;
-#pragma unroll
-  for (int it = 0; it < STAGES - 1; it++) {
-    if (it < iters) fetch(it);
-    copies_commit();
-  }
   const int x_off = W_FLOATS + (tid / rows_per_block - first_segment) * MR * F32_PITCH;
-  for (int it = 0; it < iters; it++) {
+  int tile = blockIdx.x, it = 0, stage = 0;
+  for (int j = 0; j < total; j++) {
     copies_wait<STAGES - 2>();
     __syncwarp();
-    if (it + STAGES - 1 < iters) fetch(it + STAGES - 1);
+    if (j + STAGES - 1 < total) {
+      fetch_w(f_tile, f_it, f_stage);
+      fetch_x(f_it, f_stage);
+      next();
+    }
     copies_commit();
-    const float* st = ring + (it % STAGES) * (W_FLOATS + X_FLOATS);
+    const float* st = ring + stage * (W_FLOATS + X_FLOATS);
 #pragma unroll
     for (int c = 0; c < F32_BK / 4; c++) {
       const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(st + lane * F32_PITCH + c * 4);
@@ -235,18 +273,21 @@ linear_f32_few_kernel(const F32Product p, const int rows_per_block /* 128 / segm
         fma2(acc[m], a.y, b.y);
       }
     }
-  }
-  copies_wait<0>();
-  __syncthreads();                               // the rings are idle: the segments' sums take their place
+    stage = stage + 1 == STAGES ? 0 : stage + 1;
+    if (++it < iters) continue;
+    __syncthreads();                             // the tile before this one has been added up
 #pragma unroll
-  for (int m = 0; m < MR; m++) smem[m * 128 + tid] = even_plus_odd(acc[m]);
-  __syncthreads();
-  for (int i = tid; i < MR * rows_per_block; i += 128) {
-    const int m = i / rows_per_block, r = i % rows_per_block, n = n0 + r;
-    if (m >= p.M || n >= p.N) continue;
-    float v = smem[m * 128 + r];
-    for (int s = 1; s < p.segments; s++) v = __fadd_rn(v, smem[m * 128 + s * rows_per_block + r]);
-    f32_finish(p, head, m, n, v);
+    for (int m = 0; m < MR; m++) { sums[m * 128 + tid] = even_plus_odd(acc[m]); acc[m] = 0; }
+    __syncthreads();
+    for (int i = tid; i < MR * rows_per_block; i += 128) {
+      const int m = i / rows_per_block, r = i % rows_per_block, n = tile * rows_per_block + r;
+      if (m >= p.M || n >= p.N) continue;
+      float v = sums[m * 128 + r];
+      for (int s = 1; s < p.segments; s++) v = __fadd_rn(v, sums[m * 128 + s * rows_per_block + r]);
+      f32_finish(p, head, m, n, v);
+    }
+    it = 0;
+    tile += gridDim.x;
   }
 }
 
@@ -405,16 +446,23 @@ static int f32_tile_cuts(int M, int N, int K, int heads) {
   return tiles > (1 << 20) ? 1 : f32_cuts((int)tiles, segments, segment, (long long)M * N * heads, F32_SCRATCH_FLOATS);
 }
 
+template <int MR, bool VEC, int STAGES>
+static int launch_f32_few_stages(const F32Product& p, int heads, int rows_per_block, int tiles, cudaStream_t stream) {
+  const int smem = (MR * 128 + 4 * STAGES * (32 + 2 * MR) * F32_PITCH) * 4;
+  static int once = (int)cudaFuncSetAttribute(linear_f32_few_kernel<MR, VEC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (once) return once;
+  const int places = 148 * (STAGES == 4 ? 2 : 1);
+  return launch_pdl(linear_f32_few_kernel<MR, VEC, STAGES>, dim3(tiles < places ? tiles : places, 1, heads), 128, smem, stream, p,
+                    rows_per_block);
+}
+
 template <int MR, bool VEC>
 static int launch_f32_few(const F32Product& p, int heads, cudaStream_t stream) {
   int lanes = 1;
   while (lanes < p.segments) lanes *= 2;
-  const int smem = 4 * 4 * (32 + 2 * MR) * F32_PITCH * 4;
-  static int once = (int)cudaFuncSetAttribute(linear_f32_few_kernel<MR, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (once) return once;
-  const dim3 grid((p.N + 128 / lanes - 1) / (128 / lanes), 1, heads);
-  linear_f32_few_kernel<MR, VEC><<<grid, 128, smem, stream>>>(p, 128 / lanes);
-  return launch_status();
+  const int rows_per_block = 128 / lanes, tiles = (p.N + rows_per_block - 1) / rows_per_block;
+  return (long long)tiles * heads <= 148 ? launch_f32_few_stages<MR, VEC, 8>(p, heads, rows_per_block, tiles, stream)
+                                         : launch_f32_few_stages<MR, VEC, 4>(p, heads, rows_per_block, tiles, stream);
 }
 
 template <int BM, int TM, bool VEC>
@@ -438,7 +486,9 @@ static int launch_f32(F32Product p, int heads, cudaStream_t stream) {
   if (p.M <= F32_FEW_ROWS) {
     if (p.M == 1) return launch_f32_few<1, VEC>(p, heads, stream);
     if (p.M == 2) return launch_f32_few<2, VEC>(p, heads, stream);
-    if (p.M <= 4) return launch_f32_few<4, VEC>(p, heads, stream);
+    if (p.M == 3) return launch_f32_few<3, VEC>(p, heads, stream);
+    if (p.M == 4) return launch_f32_few<4, VEC>(p, heads, stream);
+    if (p.M <= 6) return launch_f32_few<6, VEC>(p, heads, stream);
     return launch_f32_few<8, VEC>(p, heads, stream);
   }
   const int cuts = p.parts ? f32_tile_cuts(p.M, p.N, p.K, heads) : 1;
