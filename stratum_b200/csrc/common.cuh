@@ -64,23 +64,54 @@ __device__ __forceinline__ float block_sum(float v, float* scratch /* >= 33 floa
 #define STRATUM_ACT_GELU_TANH 2
 #define STRATUM_ACT_RELU_SQ 3
 #define STRATUM_ACT_CLAMPED_GATE 4
+// FAST: the quick exponential and division (a few units of float32's last place), for kernels whose result is rounded to
+// bfloat16 and whose epilogue is in the way of the next tile.  The tanh form is then z sigmoid(2 ...), the same function.
+template <int ACT, bool FAST = false>
+__device__ __forceinline__ float activate_as(float z) {
+  if (ACT == STRATUM_ACT_GELU_ERF) return 0.5f * z * (1.0f + erff(z * 0.70710678118654752440f));
+  if (ACT == STRATUM_ACT_GELU_TANH) {
+    const float u = 0.79788456080286535588f * (z + 0.044715f * z * z * z);
+    return FAST ? __fdividef(z, 1.0f + __expf(-2.0f * u)) : 0.5f * z * (1.0f + tanhf(u));
+  }
+  if (ACT == STRATUM_ACT_RELU_SQ) { const float r = fmaxf(z, 0.f); return r * r; }
+  return z;
+}
 __device__ __forceinline__ float activate(float z, int act) {
-  if (act == STRATUM_ACT_GELU_ERF) return 0.5f * z * (1.0f + erff(z * 0.70710678118654752440f));
-  if (act == STRATUM_ACT_GELU_TANH) return 0.5f * z * (1.0f + tanhf(0.79788456080286535588f * (z + 0.044715f * z * z * z)));
-  if (act == STRATUM_ACT_RELU_SQ) { const float r = fmaxf(z, 0.f); return r * r; }
+  if (act == STRATUM_ACT_GELU_ERF) return activate_as<STRATUM_ACT_GELU_ERF>(z);
+  if (act == STRATUM_ACT_GELU_TANH) return activate_as<STRATUM_ACT_GELU_TANH>(z);
+  if (act == STRATUM_ACT_RELU_SQ) return activate_as<STRATUM_ACT_RELU_SQ>(z);
   return z;
 }
 
-// The gated epilogue's value for one pair (FAST: the quick exponential, for kernels whose result is rounded to
-// bfloat16 and whose epilogue is in the way of the next tile).
+// The gated epilogue's value for one pair.
+template <int ACT, bool FAST>
+__device__ __forceinline__ float gated_as(float gate, float up, float limit) {
+  if (ACT == STRATUM_ACT_CLAMPED_GATE) {
+    const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
+    return (FAST ? __fdividef(g, 1.0f + __expf(-1.702f * g)) : g / (1.0f + expf(-1.702f * g))) * (u + 1.0f);
+  }
+  if (ACT) return activate_as<ACT, FAST>(gate) * up;
+  return (FAST ? __fdividef(gate, 1.0f + __expf(-gate)) : gate / (1.0f + expf(-gate))) * up;
+}
 template <bool FAST>
 __device__ __forceinline__ float gated(float gate, float up, int act, float limit) {
-  if (act == STRATUM_ACT_CLAMPED_GATE) {
-    const float g = fminf(gate, limit), u = fminf(fmaxf(up, -limit), limit);
-    return g / (1.0f + (FAST ? __expf(-1.702f * g) : expf(-1.702f * g))) * (u + 1.0f);
-  }
-  if (act) return activate(gate, act) * up;
-  return gate / (1.0f + (FAST ? __expf(-gate) : expf(-gate))) * up;
+  if (act == STRATUM_ACT_CLAMPED_GATE) return gated_as<STRATUM_ACT_CLAMPED_GATE, FAST>(gate, up, limit);
+  if (act == STRATUM_ACT_GELU_ERF) return gated_as<STRATUM_ACT_GELU_ERF, FAST>(gate, up, limit);
+  if (act == STRATUM_ACT_GELU_TANH) return gated_as<STRATUM_ACT_GELU_TANH, FAST>(gate, up, limit);
+  if (act == STRATUM_ACT_RELU_SQ) return gated_as<STRATUM_ACT_RELU_SQ, FAST>(gate, up, limit);
+  return gated_as<STRATUM_ACT_NONE, FAST>(gate, up, limit);
+}
+
+// f(std::integral_constant-like tag) for the activation `act`: an epilogue that goes through many values chooses once, not
+// for every value (each choice among five, unrolled over a chunk, was more code than the instruction cache holds).
+template <int ACT> struct ActTag { static constexpr int value = ACT; };
+template <typename F>
+__device__ __forceinline__ void with_activation(int act, F f) {
+  if (act == STRATUM_ACT_NONE) f(ActTag<STRATUM_ACT_NONE>());
+  else if (act == STRATUM_ACT_GELU_ERF) f(ActTag<STRATUM_ACT_GELU_ERF>());
+  else if (act == STRATUM_ACT_GELU_TANH) f(ActTag<STRATUM_ACT_GELU_TANH>());
+  else if (act == STRATUM_ACT_RELU_SQ) f(ActTag<STRATUM_ACT_RELU_SQ>());
+  else f(ActTag<STRATUM_ACT_CLAMPED_GATE>());
 }
 
 struct GateLimit {

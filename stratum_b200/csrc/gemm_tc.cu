@@ -131,12 +131,18 @@ __device__ __forceinline__ void tc_store_chunk(const TcParams& P, int m, int col
 #pragma unroll
     for (int j = 0; j < CW; j++) v[j] *= R.scale;
   }
-  if (P.bias) {
+  const bool whole = col0 + CW <= P.N;
+  if (P.bias && whole && (reinterpret_cast<uintptr_t>(P.bias) & 15) == 0) {       // (col0 is a multiple of 16)
+#pragma unroll
+    for (int j = 0; j < CW; j += 4) {
+      const float4 b = __ldg(reinterpret_cast<const float4*>(P.bias + col0 + j));
+      v[j] += b.x; v[j + 1] += b.y; v[j + 2] += b.z; v[j + 3] += b.w;
+    }
+  } else if (P.bias) {
 #pragma unroll
     for (int j = 0; j < CW; j++)
       if (col0 + j < P.N) v[j] += P.bias[col0 + j];
   }
-  const bool whole = col0 + CW <= P.N;
   if (EPI == 5) {
     // (the host checked: head_dim % CW == 0, so a chunk lies inside one head; N % CW == 0; 16-byte aligned rows)
     if (!whole) return;
@@ -176,18 +182,23 @@ __device__ __forceinline__ void tc_store_chunk(const TcParams& P, int m, int col
   } else if (EPI == 3) {
     bf16* o = (bf16*)P.out + (size_t)m * P.ldo + (col0 >> 1);
     uint32_t packed[CW / 4];
+    // With the activation chosen for every pair anew this epilogue took 30 us for a tile of 256 x 224, against 11 (K = 2,048)
+    // or 23 (4,096) of products: it was what bounded the gated products of every prompt.
+    with_activation(P.X.act, [&](auto tag) {
 #pragma unroll
-    for (int j = 0; j < CW; j += 4) {
-      float a[2];
+      for (int j = 0; j < CW; j += 4) {
+        float a[2];
 #pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const float gate = __bfloat162float(__float2bfloat16_rn(v[j + 2 * e]));
-        const float up = __bfloat162float(__float2bfloat16_rn(v[j + 2 * e + 1]));
-        a[e] = gated<true>(gate, up, P.X.act, P.X.act_limit.at((col0 + j + 2 * e) >> 1));
+        for (int e = 0; e < 2; e++) {
+          const float gate = __bfloat162float(__float2bfloat16_rn(v[j + 2 * e]));
+          const float up = __bfloat162float(__float2bfloat16_rn(v[j + 2 * e + 1]));
+          const float limit = tag.value == STRATUM_ACT_CLAMPED_GATE ? P.X.act_limit.at((col0 + j + 2 * e) >> 1) : 0.f;
+          a[e] = gated_as<tag.value, true>(gate, up, limit);
+        }
+        __nv_bfloat162 pr = __floats2bfloat162_rn(a[0], a[1]);
+        packed[j / 4] = *reinterpret_cast<uint32_t*>(&pr);
       }
-      __nv_bfloat162 pr = __floats2bfloat162_rn(a[0], a[1]);
-      packed[j / 4] = *reinterpret_cast<uint32_t*>(&pr);
-    }
+    });
     if (whole && ((reinterpret_cast<uintptr_t>(o) & 15) == 0)) {
 #pragma unroll
       for (int q = 0; q < CW / 16; q++)
@@ -202,10 +213,11 @@ __device__ __forceinline__ void tc_store_chunk(const TcParams& P, int m, int col
     }
   } else if (EPI == 0) {
     bf16* o = (bf16*)P.out + (size_t)m * P.ldo + col0;
-    if (P.X.act) {
+    if (P.X.act)
+      with_activation(P.X.act, [&](auto tag) {
 #pragma unroll
-      for (int j = 0; j < CW; j++) v[j] = activate(v[j], P.X.act);
-    }
+        for (int j = 0; j < CW; j++) v[j] = activate_as<tag.value, true>(v[j]);
+      });
     if (whole && ((reinterpret_cast<uintptr_t>(o) & 15) == 0)) {
 #pragma unroll
       for (int q = 0; q < CW / 8; q++) {
@@ -819,22 +831,41 @@ __device__ __forceinline__ void sk_store(const SkParams& P, const SkTables& T, i
       if (is_q) ((bf16*)P.out)[(size_t)m * P.ldo + n] = __float2bfloat16_rn(val);
       else if (T.cache[m] >= 0) cache[T.cache[m]] = __float2bfloat16_rn(val);
     }
-  } else {
+  } else if constexpr (EPI == 3) {
+    // gate (even n) and up (odd n) lie in neighbouring lanes: of every two rows the even lane takes one, the odd lane the other
+    const bool odd = n & 1;
+    float gate[CW / 2], up[CW / 2];
 #pragma unroll
-  for (int j = 0; j < CW; j++) {
-    const int m = m0 + j;
-    float val = v[j];
-    if (EPI == 3) {
-      val = __bfloat162float(__float2bfloat16_rn(val));
-      const float other = __shfl_xor_sync(0xffffffffu, val, 1);     // gate (even n) <-> up (odd n)
-      if (m < P.M && n + 1 < P.N && (n & 1) == 0)
-        ((bf16*)P.out)[(size_t)m * P.ldo + (n >> 1)] = __float2bfloat16_rn(gated<true>(val, other, P.X.act, P.X.act_limit.at(n >> 1)));
-    } else if (m < P.M && n < P.N) {
-      const size_t idx = (size_t)m * P.ldo + n;
-      if (EPI == 0) ((bf16*)P.out)[idx] = __float2bfloat16_rn(activate(val, P.X.act));
-      else ((float*)P.out)[idx] = val;
+    for (int i = 0; i < CW / 2; i++) {
+      const float v0 = __bfloat162float(__float2bfloat16_rn(v[2 * i])), v1 = __bfloat162float(__float2bfloat16_rn(v[2 * i + 1]));
+      const float other = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
+      gate[i] = odd ? other : v0;
+      up[i] = odd ? v1 : other;
     }
-  }
+    const int c = n >> 1;
+    const float limit = P.X.act_limit.at(c);
+    with_activation(P.X.act, [&](auto tag) {
+#pragma unroll
+      for (int i = 0; i < CW / 2; i++) {
+        const int m = m0 + 2 * i + (odd ? 1 : 0);
+        if (m < P.M && 2 * c + 1 < P.N)
+          ((bf16*)P.out)[(size_t)m * P.ldo + c] = __float2bfloat16_rn(gated_as<tag.value, true>(gate[i], up[i], limit));
+      }
+    });
+  } else {
+    if (EPI == 0 && P.X.act)
+      with_activation(P.X.act, [&](auto tag) {
+#pragma unroll
+        for (int j = 0; j < CW; j++) v[j] = activate_as<tag.value, true>(v[j]);
+      });
+#pragma unroll
+    for (int j = 0; j < CW; j++) {
+      const int m = m0 + j;
+      if (m >= P.M || n >= P.N) continue;
+      const size_t idx = (size_t)m * P.ldo + n;
+      if (EPI == 0) ((bf16*)P.out)[idx] = __float2bfloat16_rn(v[j]);
+      else ((float*)P.out)[idx] = v[j];
+    }
   }
 }
 
