@@ -477,36 +477,47 @@ attention_stream_merge_kernel(const SaParams P, int G) {
   for (int i = 0; i < (int)(blockDim.x >> 5); i++) { before += red[0][i]; total += red[1][i]; }
   const long long T = (long long)total * P.n_kv;
   const long long ub = (long long)before * P.n_kv + (long long)kvh * sq.n, ue = ub + sq.n;
-  pdl_wait();              // every block: the kernel after this one must not start on unfinished output
-  if (sq.n == 0) return;
-  const int first_c = sa_owner(ub, G, T), last_c = sa_owner(ue - 1, G, T);
-  if (first_c == last_c) return;                 // one CTA saw all keys and wrote the output itself
-  const int n_c = min(last_c - first_c + 1, SA_MAX_PIECES);      // (the launcher keeps G <= SA_MAX_PIECES)
+  // where the pieces lie follows from the step's description, so it is worked out in front of the wait (a handful of
+  // 64-bit divisions), and behind it the first pieces' values are asked for together with their maxima and sums: one
+  // round trip to L2 instead of two (a decode step of eight sequences at 3,700 tokens on the 8B shape 3.83 against 3.92 ms,
+  // of 64 on the 1B shape 1.53 against 1.57; with one sequence level)
+  int first_c = 0, n_c = 0;
+  if (sq.n > 0) {
+    first_c = sa_owner(ub, G, T);
+    const int last_c = sa_owner(ue - 1, G, T);
+    if (first_c != last_c) n_c = min(last_c - first_c + 1, SA_MAX_PIECES);      // (the launcher keeps G <= SA_MAX_PIECES)
+  }                                              // (one CTA saw all keys: it wrote the output itself)
   const size_t slot_floats = (size_t)(gs * (HD + 2));
   for (int i = threadIdx.x; i < n_c; i += blockDim.x) {
     const int cc = first_c + i;
     const long long s0 = sa_begin(cc, G, T);
-    int off = -1;
-    float m = -INFINITY, l = 0.f;
-    if (sa_begin(cc + 1, G, T) != s0) {          // with fewer pages than CTAs some stretches are empty
-      off = (int)(((size_t)cc * 2 + ((s0 >= ub && s0 < ue) ? 0 : 1)) * slot_floats);
-      m = __ldcg(P.scratch + off + gs * HD + 2 * h);
-      l = __ldcg(P.scratch + off + gs * HD + 2 * h + 1);
-    }
-    off_s[i] = off; m_s[i] = m; l_s[i] = l;
+    // (with fewer pages than CTAs some stretches are empty)
+    off_s[i] = sa_begin(cc + 1, G, T) == s0 ? -1 : (int)(((size_t)cc * 2 + ((s0 >= ub && s0 < ue) ? 0 : 1)) * slot_floats);
   }
   __syncthreads();
-  float M = -INFINITY;
-  for (int i = 0; i < n_c; i++) M = fmaxf(M, m_s[i]);
+  pdl_wait();              // every block: the kernel after this one must not start on unfinished output
+  if (n_c == 0) return;
   const int d = threadIdx.x;
-  float acc = 0.f, L = 0.f;
-  for (int i0 = 0; i0 < n_c; i0 += 8) {
-    float v[8];
+  float v[8];
+  auto values = [&](int i0) {
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       const int i = i0 + j;
       v[j] = (i < n_c && off_s[i] >= 0) ? __ldcg(P.scratch + off_s[i] + h * HD + d) : 0.f;
     }
+  };
+  values(0);
+  for (int i = threadIdx.x; i < n_c; i += blockDim.x) {
+    const int off = off_s[i];
+    m_s[i] = off >= 0 ? __ldcg(P.scratch + off + gs * HD + 2 * h) : -INFINITY;
+    l_s[i] = off >= 0 ? __ldcg(P.scratch + off + gs * HD + 2 * h + 1) : 0.f;
+  }
+  __syncthreads();
+  float M = -INFINITY;
+  for (int i = 0; i < n_c; i++) M = fmaxf(M, m_s[i]);
+  float acc = 0.f, L = 0.f;
+  for (int i0 = 0; i0 < n_c; i0 += 8) {
+    if (i0 > 0) values(i0);
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       const int i = i0 + j;
