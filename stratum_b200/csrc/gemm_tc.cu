@@ -184,19 +184,21 @@ __device__ __forceinline__ void tc_store_chunk(const TcParams& P, int m, int col
     uint32_t packed[CW / 4];
     // With the activation chosen for every pair anew this epilogue took 30 us for a tile of 256 x 224, against 11 (K = 2,048)
     // or 23 (4,096) of products: it was what bounded the gated products of every prompt.
+    float gate[CW / 2], up[CW / 2];
+#pragma unroll
+    for (int j = 0; j < CW / 2; j++) {
+      gate[j] = __bfloat162float(__float2bfloat16_rn(v[2 * j]));
+      up[j] = __bfloat162float(__float2bfloat16_rn(v[2 * j + 1]));
+    }
     with_activation(P.X.act, [&](auto tag) {
+      float a[CW / 2];
+      gated_chunk<tag.value>(gate, up, [&](int j) {
+        return tag.value == STRATUM_ACT_CLAMPED_GATE ? P.X.act_limit.at((col0 >> 1) + j) : 0.f;
+      }, a);
 #pragma unroll
-      for (int j = 0; j < CW; j += 4) {
-        float a[2];
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const float gate = __bfloat162float(__float2bfloat16_rn(v[j + 2 * e]));
-          const float up = __bfloat162float(__float2bfloat16_rn(v[j + 2 * e + 1]));
-          const float limit = tag.value == STRATUM_ACT_CLAMPED_GATE ? P.X.act_limit.at((col0 + j + 2 * e) >> 1) : 0.f;
-          a[e] = gated_as<tag.value, true>(gate, up, limit);
-        }
-        __nv_bfloat162 pr = __floats2bfloat162_rn(a[0], a[1]);
-        packed[j / 4] = *reinterpret_cast<uint32_t*>(&pr);
+      for (int j = 0; j < CW / 2; j += 2) {
+        __nv_bfloat162 pr = __floats2bfloat162_rn(a[j], a[j + 1]);
+        packed[j / 2] = *reinterpret_cast<uint32_t*>(&pr);
       }
     });
     if (whole && ((reinterpret_cast<uintptr_t>(o) & 15) == 0)) {
@@ -216,7 +218,7 @@ __device__ __forceinline__ void tc_store_chunk(const TcParams& P, int m, int col
     if (P.X.act)
       with_activation(P.X.act, [&](auto tag) {
 #pragma unroll
-        for (int j = 0; j < CW; j++) v[j] = activate_as<tag.value, true>(v[j]);
+        for (int j = 0; j < CW; j++) v[j] = activate_as<tag.value>(v[j]);
       });
     if (whole && ((reinterpret_cast<uintptr_t>(o) & 15) == 0)) {
 #pragma unroll
@@ -845,18 +847,19 @@ __device__ __forceinline__ void sk_store(const SkParams& P, const SkTables& T, i
     const int c = n >> 1;
     const float limit = P.X.act_limit.at(c);
     with_activation(P.X.act, [&](auto tag) {
+      float a[CW / 2];
+      gated_chunk<tag.value>(gate, up, [&](int) { return limit; }, a);
 #pragma unroll
       for (int i = 0; i < CW / 2; i++) {
         const int m = m0 + 2 * i + (odd ? 1 : 0);
-        if (m < P.M && 2 * c + 1 < P.N)
-          ((bf16*)P.out)[(size_t)m * P.ldo + c] = __float2bfloat16_rn(gated_as<tag.value, true>(gate[i], up[i], limit));
+        if (m < P.M && 2 * c + 1 < P.N) ((bf16*)P.out)[(size_t)m * P.ldo + c] = __float2bfloat16_rn(a[i]);
       }
     });
   } else {
     if (EPI == 0 && P.X.act)
       with_activation(P.X.act, [&](auto tag) {
 #pragma unroll
-        for (int j = 0; j < CW; j++) v[j] = activate_as<tag.value, true>(v[j]);
+        for (int j = 0; j < CW; j++) v[j] = activate_as<tag.value>(v[j]);
       });
 #pragma unroll
     for (int j = 0; j < CW; j++) {

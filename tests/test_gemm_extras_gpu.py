@@ -141,6 +141,76 @@ def test_query_key_value_epilogue_rotates_and_writes_the_cache(M, n_q, n_kv, hd,
     assert torch.equal(out2[:, :n_q * hd], out[:, :n_q * hd]) and bool((kc == 7.0).all())
 
 
+def _chosen_columns(M, K, w64):
+    """x picks one of the first 64 columns of w per row, so that a product's sums are w's values in every form."""
+    x = np.zeros((M, K))
+    x[np.arange(M), np.arange(M) % 64] = 1.0
+    w = torch.zeros(w64.shape[0], K, dtype=torch.bfloat16, device="cuda")
+    w[:, :64] = w64
+    return _bf(x), w
+
+
+@pytest.mark.parametrize("M", ROWS)
+@pytest.mark.parametrize("act", [0, 1, 2, 3, 4])
+def test_gates_of_every_size_in_every_form(M, act):
+    """Every finite bfloat16 gate above 2^-100 (with the rows there are): denominators that a quick division takes for
+    infinite, tails of the tanh form, whole tiles and tiles cut along k alike."""
+    from stratum_b200 import kernels as Kn
+    N, K = 2048, 2048
+    gates = torch.arange(1 << 16, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).reshape(1024, 64)
+    gates = torch.where(torch.isfinite(gates) & (gates.abs().float() > 2.0 ** -100), gates, torch.zeros_like(gates))
+    ups = _bf(np.random.default_rng(act).uniform(0.5, 2.0, (1024, 64))).cpu()
+    w64 = torch.stack([gates, ups], dim=1).reshape(N, 64).cuda()
+    x, w = _chosen_columns(M, K, w64)
+    out = torch.empty(M, N // 2, dtype=torch.bfloat16, device="cuda")
+    Kn.gemm_tc(x, w, None, out, Kn.EPI_SWIGLU, Kn.GemmExtra().activation(act, 7.0))
+    torch.cuda.synchronize()
+    Kn.check_status()
+    if act in (1, 2, 3):                     # the same functions as the kernel for few rows: the same bits
+        want = torch.empty(64, N // 2, dtype=torch.bfloat16, device="cuda")
+        xs, _ = _chosen_columns(64, K, w64)
+        for half in (0, 32):
+            Kn.gemm_skinny(xs[half:half + 32].contiguous(), w, None, want[half:half + 32], Kn.EPI_SWIGLU, act)
+        assert torch.equal(out, want[torch.arange(M) % 64])
+        return
+    g, u = as64(gates).T, as64(ups).T        # [column of w, pair]
+    with np.errstate(over="ignore"):
+        if act == 4:
+            g = np.minimum(g, 7.0)
+            want = g / (1.0 + np.exp(-1.702 * g)) * (np.clip(u, -7.0, 7.0) + 1.0)
+        else:
+            want = g / (1.0 + np.exp(-g)) * u
+    want = want[np.arange(M) % 64]
+    got, sure = as64(out), np.abs(want) < 3e38
+    # (where float32's exponential overflows, above 88.72, the result is zero)
+    want = np.where(((1.702 if act == 4 else 1.0) * g < -88.7)[np.arange(M) % 64], 0.0, want)
+    # half a unit of bfloat16's last place, and of float32: the quick exponential of up to 1.2 |g| + 2 units at |g| <= 89,
+    # four more roundings
+    bound = np.abs(want) * (2.0 ** -8 + 112 * 2.0 ** -23) + 2.0 ** -126
+    assert np.all(np.abs(got - want)[sure] <= bound[sure])
+
+
+@pytest.mark.parametrize("act", [1, 2, 3])
+def test_activations_are_the_same_in_every_form(act):
+    from stratum_b200 import kernels as Kn
+    N, K = 2048, 2048
+    w64 = _bf(np.random.default_rng(act).standard_normal((N, 64)) * 3.0)
+    xs, w = _chosen_columns(64, K, w64)
+    want = torch.empty(64, N, dtype=torch.bfloat16, device="cuda")
+    for half in (0, 32):
+        Kn.gemm_skinny(xs[half:half + 32].contiguous(), w, None, want[half:half + 32], Kn.EPI_STORE, act)
+    forms = set()
+    for M in ROWS:
+        x, _ = _chosen_columns(M, K, w64)
+        out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+        Kn.gemm_tc(x, w, None, out, Kn.EPI_STORE, Kn.GemmExtra().activation(act))
+        torch.cuda.synchronize()
+        Kn.check_status()
+        forms.add(Kn.gemm_tc_last_form()[0])
+        assert torch.equal(out, want[torch.arange(M) % 64]), (M, Kn.gemm_tc_last_form())
+    assert len(forms) >= 2
+
+
 def test_extras_are_refused_where_they_cannot_hold():
     from stratum_b200 import kernels as Kn
     x, w = _bf(np.zeros((4, 64))), _bf(np.zeros((200, 64)))
