@@ -61,6 +61,15 @@ def width_bucket(n_pages: int) -> int:
     return w
 
 
+def _pool_for(owner) -> tuple:
+    """The memory pool that `owner`'s next graph is captured into: the one its other graphs share.  When none of them is
+    left the pool has no user, but it lives on while a caller holds a result that lies in it, and torch takes no new
+    capture into it: a new one then."""
+    if owner.pool is None or not any(c.graph is not None for c in owner.graphs.values()):
+        owner.pool = torch.cuda.graph_pool_handle()
+    return owner.pool
+
+
 class _Captured:
     def __init__(self, engine: Engine, rows: int, width: int, pick: int):
         self.rows, self.width, self.pick = rows, width, pick
@@ -125,11 +134,9 @@ class DecodeGraphs:
         self._forward_and_pick(c)
         torch.cuda.synchronize()
         K.check_status()
-        if self.pool is None:
-            self.pool = torch.cuda.graph_pool_handle()
         g = torch.cuda.CUDAGraph()
         before = K.launch_count()
-        with torch.cuda.graph(g, pool=self.pool):
+        with torch.cuda.graph(g, pool=_pool_for(self)):
             self._forward_and_pick(c)
         c.kernels = K.launch_count() - before
         K.count_launches(-c.kernels)                  # captured, not run
@@ -357,11 +364,9 @@ class PromptGraphs:
         torch.cuda.synchronize()
         K.check_status()
         # 3. the capture
-        if self.pool is None:
-            self.pool = torch.cuda.graph_pool_handle()
         g = torch.cuda.CUDAGraph()
         before = K.launch_count()
-        with torch.cuda.graph(g, pool=self.pool):
+        with torch.cuda.graph(g, pool=_pool_for(self)):
             c.logits = eng.model.forward(c.desc.batch(max_len), eng.cache)
         c.kernels = K.launch_count() - before
         K.count_launches(-c.kernels)                  # captured, not run

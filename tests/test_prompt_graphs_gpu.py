@@ -82,3 +82,25 @@ def test_what_is_replayed_and_what_is_not(tmp_path):
     assert llm.engine.length(a) == 0 and pg.replays == 0
     out = llm.step([StepEntry(a, toks, [38]), StepEntry(b, toks[:3], [2])])
     assert out.shape == (2, TINY["A"]["vocab_size"]) and pg.replays == 1 and llm.engine.length(a) == 39
+
+
+def test_a_result_outlives_the_graph_it_came_from(tmp_path):
+    """Scratch that is regrown drops every captured graph; a result that is still held keeps their memory pool from being
+    taken again, and the next capture goes into a pool of its own."""
+    from stratum_b200 import StepEntry, Stratum
+    from stratum_b200 import kernels as K
+    path = make_model_dir(str(tmp_path / "m"), TINY["A"], seed=3, dtype="float32")
+    llm = Stratum(path, dtype="float32", max_tokens=4096)
+    llm.prompt_graphs.capture_after = 0
+    slot = llm.acquire()
+    held = [llm.step([StepEntry(slot, [5, 6, 7], [2])])]
+    held.append(llm.decode_step([slot], [8], with_logits=True)[2])
+    copies = [h.clone() for h in held]
+    for turn in range(2):                                              # dropped and captured again, twice over
+        K.scratch_regrown()
+        other = llm.acquire()
+        again = [llm.step([StepEntry(other, [5, 6, 7], [2])])]
+        again.append(llm.decode_step([other], [8], with_logits=True)[2])
+        assert all(torch.equal(a, b) for a, b in zip(again, copies))
+        assert all(torch.equal(a, b) for a, b in zip(held, copies))
+    assert llm.prompt_graphs.captures == 3 and llm.graphs.captures == 3
