@@ -139,7 +139,8 @@ __device__ __forceinline__ float even_plus_odd(f32x2 v) {
   return __fadd_rn(__uint_as_float((unsigned)v), __uint_as_float((unsigned)(v >> 32)));
 }
 
-// four floats of a row from column k on into shared memory, zeros where the row ends (`row` false: none of it is there)
+// four floats of a row from column k on into shared memory, zeros where the row ends (`row` false: none of it is there).
+// VEC = false goes through L1: for a kernel launched ahead of the end of the one before, weights only.
 template <bool VEC>
 __device__ __forceinline__ void copy4(float* dst, const float* src, int k, int K, bool row) {
   const unsigned to = (unsigned)__cvta_generic_to_shared(dst);
@@ -231,8 +232,15 @@ linear_f32_few_kernel(const F32Product p, const int rows_per_block /* 128 / segm
     float* st = ring + stage * (W_FLOATS + X_FLOATS) + W_FLOATS;
     for (int c = lane; c < warp_segments * MR * 8; c += 32) {
       const int row = c >> 3, m = row % MR, s = first_segment + row / MR;
-      copy4<VEC>(st + row * F32_PITCH + (c & 7) * 4, x + (size_t)(m < p.M ? m : 0) * p.ldx,
-                 s * p.segment + it * F32_BK + (c & 7) * 4, p.K, m < p.M && s < p.segments);
+      const int k = s * p.segment + it * F32_BK + (c & 7) * 4;
+      const float* from = x + (size_t)(m < p.M ? m : 0) * p.ldx;
+      float* to = st + row * F32_PITCH + (c & 7) * 4;
+      if (VEC) {
+        copy4<true>(to, from, k, p.K, m < p.M && s < p.segments);
+      } else {                                   // not by 4-byte copies: they go through L1, where a line of x may be an
+#pragma unroll                                   // earlier kernel's
+        for (int i = 0; i < 4; i++) to[i] = m < p.M && s < p.segments && k + i < p.K ? ld_fresh(from + k + i) : 0.f;
+      }
     }
   };
   pdl_trigger();

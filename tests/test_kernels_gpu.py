@@ -160,6 +160,45 @@ def test_linear_simple_float32_sums_have_one_order(N, K_):
             assert torch.equal(base[:, :N], 1.0 + plain) and torch.equal(base[:, N:], torch.ones(rows, 2, device="cuda"))
 
 
+@pytest.mark.parametrize("N,K_", [(4800, 2048), (4803, 2048), (9001, 2051), (10000, 300), (20003, 102)])
+def test_linear_simple_float32_blocks_that_go_from_tile_to_tile(N, K_):
+    """More tiles than blocks for the kernel for few rows: every count of rows it has a form for, whole tiles, a ragged last
+    one, K that no 16-byte copy can take, one segment and eight; the bits of the tile kernel."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(N)
+    x, w, b = dev(rng.standard_normal((65, K_))), dev(rng.standard_normal((N, K_)) * 0.1), dev(rng.standard_normal(N))
+    want = torch.empty(65, N, device="cuda")
+    K.linear_simple(x, w, b, want, K.EPI_STORE)
+    assert rel_err(as64(want), P.linear(as64(x), as64(w), as64(b))) < 2e-6
+    for rows in (1, 2, 3, 4, 5, 6, 7, 8):
+        out = torch.empty(rows, N, device="cuda")
+        K.linear_simple(x[:rows], w, b, out, K.EPI_STORE)
+        assert torch.equal(out, want[:rows]), rows
+
+
+@pytest.mark.parametrize("rows", [1, 3, 8])
+def test_linear_simple_float32_reads_what_the_kernel_before_wrote(rows):
+    """Products of ragged K one behind the other on two buffers in turn, launched ahead of one another, against the same
+    products with a pause between them: the same bits."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(rows)
+    n = 102
+    ws = [dev(rng.standard_normal((n, n)) * n ** -0.5) for _ in range(4)]
+    first = dev(rng.standard_normal((rows, n)))
+    ends = []
+    for pause in (True, False):
+        a, b = first.clone(), torch.empty(rows, n, device="cuda")
+        for i in range(200):
+            K.linear_simple(a, ws[i % 4], None, b, K.EPI_STORE)
+            if pause:
+                torch.cuda.synchronize()
+            if i % 8 == 7:
+                K.rmsnorm(b, torch.ones(n, device="cuda"), 1e-6, b)
+            a, b = b, a
+        ends.append(a)
+    assert torch.isfinite(ends[0]).all() and torch.equal(*ends)
+
+
 @pytest.mark.parametrize("rows", [1, 5, 20, 70])
 def test_linear_heads_float32(rows):
     from stratum_b200 import kernels as K
