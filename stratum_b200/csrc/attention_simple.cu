@@ -441,13 +441,13 @@ static int launch_attention_f32(const PagedF32& p, cudaStream_t stream) {
   const int group = p.n_q / p.n_kv;
   if (p.n_tokens <= AF_FEW_TOKENS && group <= AF_MAX_GROUP && p.n_kv <= 65535) {
     const int smem = (AF_MAX_GROUP * HD + 2 * 64 * (HD + 4) + AF_MAX_GROUP * (AF_PAGE + 4)) * 4;
-    static int once = (int)cudaFuncSetAttribute(attention_f32_cluster_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (once) return once;
+    const cudaError_t e = cudaFuncSetAttribute(attention_f32_cluster_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
     return launch_pdl(attention_f32_cluster_kernel<HD>, dim3(AF_CLUSTER, p.n_tokens, p.n_kv), 128, smem, stream, p);
   }
   const int smem = (3 * 64 * (HD + 4) + 64 * (AF_PAGE + 4)) * 4, per = 64 / group;
-  static int once = (int)cudaFuncSetAttribute(attention_f32_tile_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (once) return once;
+  const cudaError_t e = cudaFuncSetAttribute(attention_f32_tile_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
   attention_f32_tile_kernel<HD><<<dim3((p.n_tokens + per - 1) / per, p.n_kv), 128, smem, stream>>>(p, per);
   return launch_status();
 }

@@ -457,8 +457,8 @@ static int f32_tile_cuts(int M, int N, int K, int heads) {
 template <int MR, bool VEC, int STAGES>
 static int launch_f32_few_stages(const F32Product& p, int heads, int rows_per_block, int tiles, cudaStream_t stream) {
   const int smem = (MR * 128 + 4 * STAGES * (32 + 2 * MR) * F32_PITCH) * 4;
-  static int once = (int)cudaFuncSetAttribute(linear_f32_few_kernel<MR, VEC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (once) return once;
+  const cudaError_t e = cudaFuncSetAttribute(linear_f32_few_kernel<MR, VEC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
   const int places = 148 * (STAGES == 4 ? 2 : 1);
   return launch_pdl(linear_f32_few_kernel<MR, VEC, STAGES>, dim3(tiles < places ? tiles : places, 1, heads), 128, smem, stream, p,
                     rows_per_block);
@@ -476,8 +476,8 @@ static int launch_f32_few(const F32Product& p, int heads, cudaStream_t stream) {
 template <int BM, int TM, bool VEC>
 static int launch_f32_tile(const F32Product& p, int heads, int cuts, cudaStream_t stream) {
   const int smem = (F32_TILE_STAGES * (BM + 128) * F32_PITCH + BM * 128) * 4;
-  static int once = (int)cudaFuncSetAttribute(linear_f32_tile_kernel<BM, TM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (once) return once;
+  const cudaError_t e = cudaFuncSetAttribute(linear_f32_tile_kernel<BM, TM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
   const int m_tiles = (p.M + BM - 1) / BM;
   const long long blocks = (long long)m_tiles * ((p.N + 127) / 128);
   if (blocks > 0x7fffffffLL) return STRATUM_ERR_LIMIT;

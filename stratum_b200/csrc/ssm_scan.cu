@@ -502,8 +502,8 @@ __global__ void __launch_bounds__(WARPS * 32) ssm_recur_warp_kernel(const SsmSca
 template <int R, int WARPS>
 static int ssm_recur_warp_launch(const SsmScan& P, cudaStream_t stream) {
   const int smem = WARPS * (int)sizeof(float) * (2 * SW_CHUNK * (2 * 64 * (R / 4) + 8) + 2 * SW_CHUNK * 2 + SW_CHUNK * 2 * 68);
-  static int once = (int)cudaFuncSetAttribute(ssm_recur_warp_kernel<R, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (once) return once;
+  const cudaError_t e = cudaFuncSetAttribute(ssm_recur_warp_kernel<R, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
   const dim3 grid((P.vdim / 8 + WARPS - 1) / WARPS, P.n_heads, P.n_seqs);
   ssm_recur_warp_kernel<R, WARPS><<<grid, WARPS * 32, smem, stream>>>(P);
   return launch_status();

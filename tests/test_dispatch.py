@@ -134,3 +134,17 @@ def test_extra_epilogue_rules(recorded, monkeypatch):
         recorded.clear()
         A.run(att, torch.zeros(300, 48 * 128, dtype=torch.bfloat16), cache, step, torch.zeros(300, 4096, dtype=torch.bfloat16))
         assert recorded[0][0] == "attention_tc" and sizes[-1] == tokens
+
+
+def test_shared_memory_is_opted_into_at_every_launch():
+    """The opt-in belongs to the device that is current when it is made, and may fail once: no launcher keeps its result for
+    the life of the process."""
+    import glob
+    import os
+    import re
+    import stratum_b200
+    sources = glob.glob(os.path.join(os.path.dirname(stratum_b200.__file__), "csrc", "*.cu*"))
+    assert len(sources) > 20
+    for path in sources:
+        with open(path) as f:
+            assert not re.search(r"static\b[^;{}]*=[^;{}]*cudaFuncSetAttribute", f.read()), path
