@@ -108,16 +108,27 @@ attention_simple_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ 
 //
 //   attention_f32_tile_kernel     64 rows (tokens x heads of a kv head's group) a block, keys and values of a page in shared
 //                                 memory once for all of them, both products on register tiles: bound by the FMA units
-//   attention_f32_cluster_kernel  one (token, kv head) a cluster of eight blocks, which take eight pages at a time and
-//                                 merge them through distributed shared memory: a few tokens fill the GPU, whatever
-//                                 their length, in one launch and without scratch
+//   attention_f32_cluster_kernel  one (token, kv head) a cluster of up to eight blocks, which take a page each at a time
+//                                 and merge them through distributed shared memory: a few tokens fill the GPU, whatever
+//                                 their length, in one launch and without scratch.  It takes the tokens whose pages no
+//                                 tile could share: steps of one token a sequence, and of steps that mix such sequences
+//                                 with prompts those that bring AF_SHORT_RUN tokens or fewer (AF_SCATTERED)
 //
-// Measured on the 1B shape (32 heads of 64 in groups of four), against one warp per (token, head) with a key a lane:
-// 611 tokens 197 us (1,822), three tokens behind 120 to 450 keys 10.5 us (399).
+// Measured against one warp per (token, head) with a key a lane, which was the only kernel once (us, in brackets):
+//                                              32 heads of 64, 8 of keys    32 heads of 128, each its own keys
+//   a prompt of 611 tokens                        182 (1,835)                  387 (3,234)
+//   1 token behind 2,000                           35 (859)                     57 (1,423)
+//   64 x 1 behind 1,500                           194 (1,743)                1,212 (2,734)   as tiles 5,826 and 36,482
+//   20 x 1 behind 1,500 and a prompt of 600       374 (2,258)                  930 (3,643)   as tiles 5,856 and 11,716
+//   100 x 2 behind 700                            280 (1,775)                2,160 (2,794)
+//   5 x 1 behind 1,500 and a prompt of 600      1,224 (1,829)                2,116 (3,329)
+//   40 prompts of 9 tokens                         44 (35)                     283 (55)
 #define AF_PAGE 64
-#define AF_CLUSTER 8
 #define AF_MAX_GROUP 8          // heads per kv head the cluster kernel takes
 #define AF_FEW_TOKENS 32        // steps of at most this many tokens take it
+#define AF_SHORT_RUN 4          // (100 x 4 behind 300: 1,936 us by token, 2,128 by tiles; 30 x 16 behind 200 1,524 and 559)
+#define AF_SCATTERED 64         // steps of fewer tokens than this a sequence on the average look for short runs (with more of
+                                // them the blocks that find none cost more: 5 prompts of 548 tokens, 9 us of 71)
 
 typedef unsigned long long f32x2;
 __device__ __forceinline__ void fma2(f32x2& acc, f32x2 a, f32x2 b) {
@@ -136,7 +147,16 @@ struct PagedF32 {
   float* out;
   int ldq, ldo, bt_stride, n_tokens, n_q, n_kv, page_tokens, window;
   float scale;
-};
+  int short_run;                // > 0: tokens of runs (neighbours of one sequence) of at most this many are the cluster kernel's,
+};                              // the others the tile kernel's; 0: the kernel that is launched takes all
+
+__device__ __forceinline__ bool in_short_run(const PagedF32& p, int t) {
+  const int seq = p.token_seq[t];
+  int n = 1;
+  for (int i = t - 1; i >= 0 && n <= p.short_run && p.token_seq[i] == seq; i--) n++;
+  for (int i = t + 1; i < p.n_tokens && n <= p.short_run && p.token_seq[i] == seq; i++) n++;
+  return n <= p.short_run;
+}
 
 // A page's keys (or values) of one kv head into shared memory, rows of HD + 4 floats.  Halves of 32 keys without a key of
 // [first, last] are zeros: their pages may be nobody's.
@@ -215,8 +235,9 @@ attention_f32_tile_kernel(const PagedF32 p, const int tokens_per_block) {
 #pragma unroll
     for (int n = 0; n < NV; n++) o[i][n][0] = o[i][n][1] = 0;
 
-  // one sequence of the block's tokens after the other (a step's tokens are packed: runs of equal sequences)
-  for (int a0 = 0; a0 < n_tok;) {
+  // one sequence of the block's tokens after the other (a step's tokens are packed: runs of equal sequences); where there
+  // are many, gridDim.z blocks share them, every gridDim.z-th to each
+  for (int a0 = 0, run = 0; a0 < n_tok; run++) {
     const int seq = rseq[a0 * group];
     int a1 = a0, last = 0, first = 0x7fffffff;
     for (; a1 < n_tok && rseq[a1 * group] == seq; a1++) {
@@ -226,18 +247,19 @@ attention_f32_tile_kernel(const PagedF32 p, const int tokens_per_block) {
     }
     const int r0 = a0 * group, r1 = a1 * group;
     a0 = a1;
-    if (seq < 0) continue;                       // padding tokens
+    if (p.short_run > 0 && seq >= 0 && in_short_run(p, t0 + r0 / group)) continue;
+    if (seq < 0 || run % (int)gridDim.z != (int)blockIdx.z) continue;     // padding tokens, or another block's
     const int* bt = p.block_table + (size_t)seq * p.bt_stride;
     for (int base = first / AF_PAGE * AF_PAGE; base <= last; base += AF_PAGE) {
       fetch_page<HD>(ks, p.k, p, bt, kvh, base, first, last);
       fetch_page<HD>(vs, p.v, p, bt, kvh, base, first, last);
-      bool whole = true;                         // every row sees every key of the page
+      bool whole = true;                         // every row of this sequence sees every key of the page
       if (tid < 64) {
         const int pos = rpos[tid], lo = p.window > 0 && pos - p.window + 1 > 0 ? pos - p.window + 1 : 0;
         const bool mine = tid >= r0 && tid < r1;
         rj0[tid] = mine ? max(lo - base, 0) : 64;
         rj1[tid] = mine ? min(pos - base, 63) : -1;
-        whole = tid >= rows || (mine && lo <= base && pos >= base + 63);
+        whole = !mine || (lo <= base && pos >= base + 63);
       }
       asm volatile("cp.async.wait_group 1;" ::: "memory");
       const bool all_whole = __syncthreads_and(whole);
@@ -288,9 +310,9 @@ attention_f32_tile_kernel(const PagedF32 p, const int tokens_per_block) {
       for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int n = 0; n < NV; n++) u[i][n][0] = u[i][n][1] = 0;
-      if (all_whole) {
+      auto values = [&](int j_begin, int j_end, auto seen) {
 #pragma unroll 2
-        for (int j = 0; j < AF_PAGE; j += 4) {
+        for (int j = j_begin; j < j_end; j += 4) {
           float4 w[4];
 #pragma unroll
           for (int i = 0; i < 4; i++) w[i] = *reinterpret_cast<const float4*>(ss + (tr + 16 * i) * SP + j);
@@ -301,27 +323,22 @@ attention_f32_tile_kernel(const PagedF32 p, const int tokens_per_block) {
             for (int n = 0; n < NV; n++) b[n] = *reinterpret_cast<const ulonglong2*>(vs + (j + jj) * PITCH + 4 * tc + 32 * n);
 #pragma unroll
             for (int i = 0; i < 4; i++) {
+              if (!seen(i, j + jj)) continue;
               const f32x2 pp = twice(jj == 0 ? w[i].x : jj == 1 ? w[i].y : jj == 2 ? w[i].z : w[i].w);
 #pragma unroll
               for (int n = 0; n < NV; n++) { fma2(u[i][n][0], pp, b[n].x); fma2(u[i][n][1], pp, b[n].y); }
             }
           }
         }
+      };
+      if (all_whole) {
+        values(0, AF_PAGE, [](int, int) { return true; });
       } else {                                   // a key that a row does not see is not multiplied by 0 but left out: its
-        for (int j = 0; j < AF_PAGE; j++) {      // value may be another token's NaN, or nothing that was ever written
+        int j0[4], j1[4];                        // value may be another token's NaN, or nothing that was ever written
 #pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const int r = tr + 16 * i;
-            if (j < rj0[r] || j > rj1[r]) continue;
-            const f32x2 pp = twice(ss[r * SP + j]);
-#pragma unroll
-            for (int n = 0; n < NV; n++) {
-              const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(vs + j * PITCH + 4 * tc + 32 * n);
-              fma2(u[i][n][0], pp, b.x);
-              fma2(u[i][n][1], pp, b.y);
-            }
-          }
-        }
+        for (int i = 0; i < 4; i++) { j0[i] = rj0[tr + 16 * i]; j1[i] = rj1[tr + 16 * i]; }
+        values(max(first - base, 0) & ~3, min(last - base, AF_PAGE - 1) + 1,
+               [&](int i, int j) { return j >= j0[i] && j <= j1[i]; });
       }
 #pragma unroll
       for (int i = 0; i < 4; i++) {
@@ -343,7 +360,7 @@ attention_f32_tile_kernel(const PagedF32 p, const int tokens_per_block) {
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const int r = tr + 16 * i;
-    if (r >= rows || rseq[r] < 0) continue;
+    if (rl[r] == 0.f) continue;                  // not a row of this block (a token sees itself at least: its sum is not zero)
     const float inv = 1.0f / rl[r];
     float* to = p.out + (size_t)(t0 + r / group) * p.ldo + (size_t)(kvh * group + r % group) * HD;
 #pragma unroll
@@ -353,31 +370,32 @@ attention_f32_tile_kernel(const PagedF32 p, const int tokens_per_block) {
   }
 }
 
-template <int HD>
-__global__ void __cluster_dims__(AF_CLUSTER, 1, 1) __launch_bounds__(128)
+template <int HD, int C>
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(128)
 attention_f32_cluster_kernel(const PagedF32 p) {
   constexpr int PITCH = HD + 4, SP = AF_PAGE + 4, LANES = HD;             // threads side by side over the output's columns
+  constexpr int MINE = (AF_MAX_GROUP * HD + 128 * C - 1) / (128 * C);     // output elements a thread merges at most
   extern __shared__ __align__(16) float smem[];
-  float *qs = smem, *ks = qs + AF_MAX_GROUP * HD, *vs = ks + 64 * PITCH, *ss = vs + 64 * PITCH;
-  __shared__ float part_o[2][AF_MAX_GROUP * HD], part_m[2][AF_MAX_GROUP], part_l[2][AF_MAX_GROUP];
+  __shared__ float part_m[2][AF_MAX_GROUP], part_l[2][AF_MAX_GROUP];
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int t = blockIdx.y, kvh = blockIdx.z, group = p.n_q / p.n_kv;
+  float *qs = smem, *ks = qs + group * HD, *vs = ks + 64 * PITCH, *ss = vs + 64 * PITCH, *part_o = ss + group * SP;   // [2][group][HD]
   pdl_trigger();
   const int seq = p.token_seq[t], pos = p.token_pos[t];
   pdl_wait();                                    // queries and the newest keys and values come from kernels before this one
-  if (seq < 0) return;                           // padding token (of the whole cluster)
+  if (seq < 0 || (p.short_run > 0 && !in_short_run(p, t))) return;        // (of the whole cluster)
   const int lo = p.window > 0 && pos - p.window + 1 > 0 ? pos - p.window + 1 : 0;
   const int* bt = p.block_table + (size_t)seq * p.bt_stride;
   for (int c = tid; c < group * HD; c += 128) qs[c] = ld_fresh(p.q + (size_t)t * p.ldq + (size_t)kvh * group * HD + c);
 
   const int first_page = lo / AF_PAGE, last_page = pos / AF_PAGE;
-  const int e = rank * (group * HD / AF_CLUSTER) + tid;                   // the output element this thread merges
-  const bool merges = tid < group * HD / AF_CLUSTER;
-  const int row = merges ? e / HD : 0;
-  float m = -INFINITY, l = 0.f, acc = 0.f;
+  const int share = group * HD / C;              // of the output elements, for this block to merge
+  float m[MINE], l[MINE], acc[MINE];
+#pragma unroll
+  for (int i = 0; i < MINE; i++) { m[i] = -INFINITY; l[i] = acc[i] = 0.f; }
   int buf = 0;
-  for (int page0 = first_page; page0 <= last_page; page0 += AF_CLUSTER, buf ^= 1) {
+  for (int page0 = first_page; page0 <= last_page; page0 += C, buf ^= 1) {
     const int page = page0 + rank, base = page * AF_PAGE;
     if (page <= last_page) {
       fetch_page<HD>(ks, p.k, p, bt, kvh, base, lo, pos);
@@ -419,44 +437,77 @@ attention_f32_cluster_kernel(const PagedF32 p) {
         float u = 0.f;
 #pragma unroll 8
         for (int j = j0; j <= j1; j++) u = __fmaf_rn(ss[r * SP + j], vs[j * PITCH + d], u);
-        part_o[buf][r * HD + d] = u;
+        part_o[(buf * group + r) * HD + d] = u;
       }
     }
-    cluster.sync();                              // the round's parts are there (and those of the round before read)
-    if (merges)
+    if constexpr (C > 1) cluster.sync();         // the round's parts are there (and those of the round before read)
+    else __syncthreads();
 #pragma unroll
-      for (int q = 0; q < AF_CLUSTER; q++) {
+    for (int i = 0; i < MINE; i++) {
+      const int e = rank * share + tid + 128 * i, row = e / HD;
+      if (tid + 128 * i >= share) break;
+#pragma unroll
+      for (int q = 0; q < C; q++) {
         if (page0 + q > last_page) break;
         float a, b;
-        merge_page(m, l, *cluster.map_shared_rank(&part_m[buf][row], q), *cluster.map_shared_rank(&part_l[buf][row], q), a, b);
-        acc = __fmaf_rn(acc, a, __fmul_rn(*cluster.map_shared_rank(&part_o[buf][e], q), b));
+        merge_page(m[i], l[i], *cluster.map_shared_rank(&part_m[buf][row], q), *cluster.map_shared_rank(&part_l[buf][row], q), a, b);
+        acc[i] = __fmaf_rn(acc[i], a, __fmul_rn(*cluster.map_shared_rank(&part_o[buf * group * HD + e], q), b));
       }
+    }
   }
-  if (merges) p.out[(size_t)t * p.ldo + (size_t)kvh * group * HD + e] = acc * (1.0f / l);
-  cluster.sync();                                // nobody leaves while another reads its parts
+#pragma unroll
+  for (int i = 0; i < MINE; i++)
+    if (tid + 128 * i < share)
+      p.out[(size_t)t * p.ldo + (size_t)kvh * group * HD + rank * share + tid + 128 * i] = acc[i] * (1.0f / l[i]);
+  if constexpr (C > 1) cluster.sync();           // nobody leaves while another reads its parts
+}
+
+template <int HD, int C>
+static int launch_attention_f32_cluster(const PagedF32& p, cudaStream_t stream) {
+  const int group = p.n_q / p.n_kv, smem = (3 * group * HD + 2 * 64 * (HD + 4) + group * (AF_PAGE + 4)) * 4;
+  const cudaError_t e = cudaFuncSetAttribute(attention_f32_cluster_kernel<HD, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
+  return launch_pdl(attention_f32_cluster_kernel<HD, C>, dim3(C, p.n_tokens, p.n_kv), 128, smem, stream, p);
 }
 
 template <int HD>
-static int launch_attention_f32(const PagedF32& p, cudaStream_t stream) {
-  const int group = p.n_q / p.n_kv;
-  if (p.n_tokens <= AF_FEW_TOKENS && group <= AF_MAX_GROUP && p.n_kv <= 65535) {
-    const int smem = (AF_MAX_GROUP * HD + 2 * 64 * (HD + 4) + AF_MAX_GROUP * (AF_PAGE + 4)) * 4;
-    const cudaError_t e = cudaFuncSetAttribute(attention_f32_cluster_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    return launch_pdl(attention_f32_cluster_kernel<HD>, dim3(AF_CLUSTER, p.n_tokens, p.n_kv), 128, smem, stream, p);
+static int launch_attention_f32(PagedF32 p, int n_seqs, bool all_single, cudaStream_t stream) {
+  const int group = p.n_q / p.n_kv, per = 64 / group;
+  const bool scattered = n_seqs > 1 && p.n_tokens < AF_SCATTERED * (long long)n_seqs;
+  const bool by_token = group <= AF_MAX_GROUP && p.n_tokens <= 65535;
+  const bool all_by_token = by_token && (all_single || p.n_tokens <= AF_FEW_TOKENS);
+  // blocks to a token: eight, four or one, as many as fill the GPU a few times over (blocks with heads of 64 come five to an
+  // SM, with heads of 128 two or three, and idle ones cost as much): 8 x 1 behind 1,500 with eight / four / one, heads of
+  // 64 41 / 56 / 147 us, 32 of 128 with their own keys 299 / 283 / 228; 200 x 1 behind 700 421 / 313 / 267 and 4,745 /
+  // 3,231 / 2,283
+  if (all_by_token || (by_token && scattered)) {
+    p.short_run = all_by_token ? 0 : AF_SHORT_RUN;
+    const long long walks = (long long)p.n_tokens * p.n_kv;
+    const long long most = HD == 64 ? 2048 : 296;
+    const int st = walks * 8 <= most   ? launch_attention_f32_cluster<HD, 8>(p, stream)
+                   : walks * 4 <= most ? launch_attention_f32_cluster<HD, 4>(p, stream)
+                                       : launch_attention_f32_cluster<HD, 1>(p, stream);
+    if (st || all_by_token) return st;
   }
-  const int smem = (3 * 64 * (HD + 4) + 64 * (AF_PAGE + 4)) * 4, per = 64 / group;
+  const int smem = (3 * 64 * (HD + 4) + 64 * (AF_PAGE + 4)) * 4;
   const cudaError_t e = cudaFuncSetAttribute(attention_f32_tile_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
-  attention_f32_tile_kernel<HD><<<dim3((p.n_tokens + per - 1) / per, p.n_kv), 128, smem, stream>>>(p, per);
+  // as many blocks to a tile as it has sequences on the average, and with groups that the cluster kernel does not take as it
+  // may have: every run is a walk through all of its sequence's pages
+  const long long runs = !by_token ? n_seqs : ((long long)n_seqs * per + p.n_tokens - 1) / p.n_tokens;
+  const int most = n_seqs < per ? n_seqs : per, z = runs < most ? (int)runs : most;
+  attention_f32_tile_kernel<HD><<<dim3((p.n_tokens + per - 1) / per, p.n_kv, z < 1 ? 1 : z), 128, smem, stream>>>(p, per);
   return launch_status();
 }
 
+// n_seqs (the rows of the block table) and all_single (every token is the only one of its sequence) say how the step's tokens
+// share pages, for the choice of kernel alone.
 STRATUM_EXPORT int stratum_attention_simple(const void* q, int ldq, const void* k_cache, const void* v_cache,
                                             int dtype, const int* token_pos, const int* token_seq,
                                             const int* block_table, int bt_stride, void* out, int ldo,
                                             int n_tokens, int n_q, int n_kv, int head_dim, int page_tokens,
-                                            int window, float scale, cudaStream_t stream) {
+                                            int window, float scale, int n_seqs, int all_single,
+                                            cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (head_dim < 1 || head_dim > AS_MAX_HD) return STRATUM_ERR_LIMIT;
   if (n_kv < 1 || n_q % n_kv != 0 || page_tokens % 32 != 0) return STRATUM_ERR_SHAPE;
@@ -467,8 +518,9 @@ STRATUM_EXPORT int stratum_attention_simple(const void* q, int ldq, const void* 
   if (dtype == STRATUM_DT_F32 && (head_dim == 64 || head_dim == 128) && n_q / n_kv <= 64 && n_kv <= 65535 && ldq % 4 == 0 &&
       ldo % 4 == 0 && ((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) % 16 == 0) {
     const PagedF32 p = {(const float*)q, (const float*)k_cache, (const float*)v_cache, token_pos, token_seq, block_table,
-                        (float*)out, ldq, ldo, bt_stride, n_tokens, n_q, n_kv, page_tokens, window, scale};
-    return head_dim == 64 ? launch_attention_f32<64>(p, stream) : launch_attention_f32<128>(p, stream);
+                        (float*)out, ldq, ldo, bt_stride, n_tokens, n_q, n_kv, page_tokens, window, scale, 0};
+    return head_dim == 64 ? launch_attention_f32<64>(p, n_seqs, all_single != 0, stream)
+                          : launch_attention_f32<128>(p, n_seqs, all_single != 0, stream);
   }
   if (dtype == STRATUM_DT_F32)
     attention_simple_kernel<float><<<(unsigned)blocks, AS_WARPS * 32, 0, stream>>>(

@@ -615,16 +615,18 @@ def gemm_tc_last_form() -> Tuple[str, int]:
 # ------------------------------------------------------------------ attention (any sizes, CUDA cores)
 def attention_simple(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, token_pos: torch.Tensor,
                      token_seq: torch.Tensor, block_table: torch.Tensor, out: torch.Tensor, n_q: int, n_kv: int,
-                     head_dim: int, page_tokens: int, window: int, scale: float) -> None:
-    """Causal GQA attention of every token of the step over its sequence's cached keys."""
+                     head_dim: int, page_tokens: int, window: int, scale: float, all_single: bool = False) -> None:
+    """Causal GQA attention of every token of the step over its sequence's cached keys.  all_single: every token is the only
+    one of its sequence (which kernel is quicker follows from it; the result does not)."""
     _need(qkv, "qkv"); _need(k_cache, "k_cache", qkv.dtype); _need(v_cache, "v_cache", qkv.dtype)
     _need(out, "out", qkv.dtype); _need(block_table, "block_table", torch.int32)
     f = _fn("attention_simple", "stratum_attention_simple",
             [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int,
-             c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p])
+             c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p])
     _check(f(_ptr(qkv), qkv.stride(0), _ptr(k_cache), _ptr(v_cache), dtype_code(qkv.dtype), _ptr(token_pos),
              _ptr(token_seq), _ptr(block_table), block_table.stride(0), _ptr(out), out.stride(0), qkv.shape[0],
-             n_q, n_kv, head_dim, page_tokens, window, c_float(scale), _stream()), "attention_simple")
+             n_q, n_kv, head_dim, page_tokens, window, c_float(scale), block_table.shape[0], int(all_single),
+             _stream()), "attention_simple")
 
 
 class _MixerPrep(ctypes.Structure):

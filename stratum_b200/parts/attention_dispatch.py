@@ -41,7 +41,7 @@ def run(att, qkv: torch.Tensor, cache, step, out: torch.Tensor) -> None:
     hd = att.head_dim
     if qkv.dtype != torch.bfloat16 or hd % 16 != 0 or hd > 128 or qkv.stride(0) % 8 != 0:
         K.attention_simple(qkv, cache.k, cache.v, step.token_pos, step.token_seq, cache.block_table, out,
-                           att.n_heads, att.n_kv_heads, hd, PAGE_TOKENS, att.window, att.scale)
+                           att.n_heads, att.n_kv_heads, hd, PAGE_TOKENS, att.window, att.scale, step.all_single)
         return
     gs = att.n_heads // att.n_kv_heads
     rows_per_token = min(gs, 16)

@@ -66,7 +66,9 @@ def _attention_call(recorded, dtype, head_dim, n_heads, n_kv, n_tokens, all_sing
 
 def test_attention_rules(recorded):
     bf, f32 = torch.bfloat16, torch.float32
-    assert _attention_call(recorded, f32, 128, 32, 8, 8, True)[0] == "attention_simple"
+    name, args, _ = _attention_call(recorded, f32, 128, 32, 8, 80, True)
+    assert name == "attention_simple" and args[-1] is True           # told that no two tokens share a sequence's pages
+    assert _attention_call(recorded, f32, 128, 32, 8, 80, False)[1][-1] is False
     assert _attention_call(recorded, bf, 256, 4, 2, 8, True)[0] == "attention_simple"        # head size above 128
     name, _, kw = _attention_call(recorded, bf, 128, 32, 8, 8, True)
     assert name == "attention_stream" and kw["late_trigger"] is True

@@ -504,6 +504,33 @@ def test_attention_simple_float32_by_pages(n_q, n_kv, hd, window):
     assert torch.equal(again[:-1], out[:-1]) and bool(torch.isnan(again[-1]).all())
 
 
+@pytest.mark.parametrize("n_q,n_kv,hd,window", [(8, 2, 64, 0), (4, 4, 128, 0), (4, 4, 64, 90), (12, 1, 64, 0)])
+def test_attention_simple_float32_of_many_sequences(n_q, n_kv, hd, window):
+    """Dozens of sequences with a token or a few each beside a prompt: tiles shared by several blocks, a cluster for every
+    token, and one sequence's tokens by themselves give the same bits."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(hd + n_q + window)
+    before = [int(n) for n in rng.integers(0, 300, 45)] + [0]
+    new = [1] * 33 + [int(n) for n in rng.integers(1, 7, 12)] + [70]
+    c = _attention_case(rng, before, new, n_q, n_kv, hd, "float32", window=window)
+    args = (n_q, n_kv, hd, 64, window, 1.0 / math.sqrt(hd))
+
+    def run(rows, all_single, table=c["table"], seq=None):
+        got = torch.zeros(len(rows), n_q * hd, device="cuda")
+        K.attention_simple(c["qkv"][rows].contiguous(), c["kc"], c["vc"], c["pos"][rows].contiguous(),
+                           c["seq"][rows].contiguous() if seq is None else seq, table, got, *args, all_single)
+        return got
+
+    every = torch.arange(c["T"], device="cuda")
+    out = run(every, False)
+    assert rel_err(as64(out), c["ref"]) < 3e-6
+    assert torch.equal(run(every, True), out)                          # whatever it is told of the step
+    assert torch.equal(run(every[:33], True), out[:33]) and torch.equal(run(every[:33], False), out[:33])
+    last = every[-70:]
+    alone = run(last, False, c["table"][-1:].contiguous(), torch.zeros(70, dtype=torch.int32, device="cuda"))
+    assert torch.equal(alone, out[-70:])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_attention_finds_one_far_key_among_hundreds(dtype):
     """Scale one query and one key so that a single far score dominates: the output must be that key's value."""
