@@ -122,20 +122,26 @@ __device__ __forceinline__ void with_activation(int act, F f) {
   else f(ActTag<STRATUM_ACT_CLAMPED_GATE>());
 }
 
-// A chunk of N pairs through gated_as: their gates are looked at together, so that the branch that one division
+// The first `used` of a chunk of N pairs through gated_as, STEP at a time (used: the same in all lanes; what lies behind it in
+// the last step is worked out too).  The gates of a step are looked at together, so that the branch that one division
 // needs is taken once for all of them.
-template <int ACT, int N, typename Limit>
-__device__ __forceinline__ void gated_chunk(const float (&gate)[N], const float (&up)[N], Limit limit, float (&out)[N]) {
-  bool ordinary = ACT == STRATUM_ACT_NONE || ACT == STRATUM_ACT_CLAMPED_GATE;
+template <int ACT, int STEP, int N, typename Limit>
+__device__ __forceinline__ void gated_chunk(const float (&gate)[N], const float (&up)[N], int used, Limit limit, float (&out)[N]) {
+  static_assert(N % STEP == 0, "whole steps");
 #pragma unroll
-  for (int i = 0; i < N; i++)
-    ordinary = ordinary && gate_is_ordinary(ACT == STRATUM_ACT_CLAMPED_GATE ? fminf(gate[i], limit(i)) : gate[i]);
-  if (ordinary) {
+  for (int i0 = 0; i0 < N; i0 += STEP) {
+    if (i0 >= used) break;
+    bool ordinary = ACT == STRATUM_ACT_NONE || ACT == STRATUM_ACT_CLAMPED_GATE;
 #pragma unroll
-    for (int i = 0; i < N; i++) out[i] = gated_as<ACT, true, true>(gate[i], up[i], limit(i));
-  } else {
+    for (int i = i0; i < i0 + STEP; i++)
+      ordinary = ordinary && gate_is_ordinary(ACT == STRATUM_ACT_CLAMPED_GATE ? fminf(gate[i], limit(i)) : gate[i]);
+    if (ordinary) {
 #pragma unroll
-    for (int i = 0; i < N; i++) out[i] = gated_as<ACT, true>(gate[i], up[i], limit(i));
+      for (int i = i0; i < i0 + STEP; i++) out[i] = gated_as<ACT, true, true>(gate[i], up[i], limit(i));
+    } else {
+#pragma unroll
+      for (int i = i0; i < i0 + STEP; i++) out[i] = gated_as<ACT, true>(gate[i], up[i], limit(i));
+    }
   }
 }
 

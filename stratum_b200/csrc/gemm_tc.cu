@@ -192,7 +192,7 @@ __device__ __forceinline__ void tc_store_chunk(const TcParams& P, int m, int col
     }
     with_activation(P.X.act, [&](auto tag) {
       float a[CW / 2];
-      gated_chunk<tag.value>(gate, up, [&](int j) {
+      gated_chunk<tag.value, CW / 2>(gate, up, CW / 2, [&](int j) {
         return tag.value == STRATUM_ACT_CLAMPED_GATE ? P.X.act_limit.at((col0 >> 1) + j) : 0.f;
       }, a);
 #pragma unroll
@@ -295,23 +295,30 @@ __device__ __forceinline__ void fixup_store(const PT& P, int m, int n, float4 v)
   }
   if (EPI == 3) {                                   // (gate, up) pairs: n even
     bf16* o = (bf16*)P.out + (size_t)m * P.ldo + (n >> 1);
+    float gate[2], up[2];
 #pragma unroll
-    for (int j = 0; j < 4; j += 2) {
-      if (n + j + 1 < P.N) {
-        const float g = __bfloat162float(__float2bfloat16_rn(e[j])), u = __bfloat162float(__float2bfloat16_rn(e[j + 1]));
-        o[j >> 1] = __float2bfloat16_rn(gated<true>(g, u, P.X.act, P.X.act_limit.at((n + j) >> 1)));
-      }
+    for (int j = 0; j < 2; j++) {
+      gate[j] = __bfloat162float(__float2bfloat16_rn(e[2 * j]));
+      up[j] = __bfloat162float(__float2bfloat16_rn(e[2 * j + 1]));
     }
+    with_activation(P.X.act, [&](auto tag) {
+      float a[2];
+      gated_chunk<tag.value, 2>(gate, up, 2, [&](int j) { return P.X.act_limit.at((n >> 1) + j); }, a);
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+        if (n + 2 * j + 1 < P.N) o[j] = __float2bfloat16_rn(a[j]);
+    });
     return;
   }
   const size_t idx = (size_t)m * P.ldo + n;
   const bool wide = (n + 3 < P.N) && ((idx & 3) == 0);
   if (EPI == 0) {
     bf16* o = (bf16*)P.out + idx;
-    if (P.X.act) {
+    if (P.X.act)
+      with_activation(P.X.act, [&](auto tag) {
 #pragma unroll
-      for (int j = 0; j < 4; j++) e[j] = activate(e[j], P.X.act);
-    }
+        for (int j = 0; j < 4; j++) e[j] = activate_as<tag.value>(e[j]);
+      });
     if (wide && ((reinterpret_cast<uintptr_t>(o) & 7) == 0)) {
       __nv_bfloat162 lo = __floats2bfloat162_rn(e[0], e[1]), hi = __floats2bfloat162_rn(e[2], e[3]);
       uint2 u; u.x = *reinterpret_cast<uint32_t*>(&lo); u.y = *reinterpret_cast<uint32_t*>(&hi);
@@ -848,7 +855,7 @@ __device__ __forceinline__ void sk_store(const SkParams& P, const SkTables& T, i
     const float limit = P.X.act_limit.at(c);
     with_activation(P.X.act, [&](auto tag) {
       float a[CW / 2];
-      gated_chunk<tag.value>(gate, up, [&](int) { return limit; }, a);
+      gated_chunk<tag.value, (CW < 8 ? CW / 2 : 4)>(gate, up, (P.M - m0 + 1) / 2, [&](int) { return limit; }, a);
 #pragma unroll
       for (int i = 0; i < CW / 2; i++) {
         const int m = m0 + 2 * i + (odd ? 1 : 0);
