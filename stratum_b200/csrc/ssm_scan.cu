@@ -84,17 +84,21 @@ __global__ void __launch_bounds__(SS_PREP_THREADS) ssm_prep_kernel(const SsmScan
 }
 
 // Short convolutions of four taps over 16-byte aligned rows (every configuration so far): a thread takes four channels
-// through SS_PREP_TOKENS tokens with the last three inputs in registers, so an input is read once from L2 by 16-byte
-// loads instead of four times by 4-byte ones.  The sums are those of the kernel above, in its order.  2,000 tokens of
-// 10,240 channels (164 MB in and out) take 59 us; a thread per channel and token, which was bound by its instructions
-// (83 % of the issue slots), took 156.
-#define SS_PREP_TOKENS 8
+// through TOKENS tokens with the last three inputs in registers, so an input is read once from L2 by 16-byte loads instead of
+// four times by 4-byte ones.  The sums are those of the kernel above, in its order.  2,000 tokens of 10,240 channels (164 MB
+// in and out) take 59 us; a thread per channel and token, which was bound by its instructions (83 % of the issue slots),
+// took 156.  TOKENS is eight, but one where a step has few tokens or many sequences (ssm_prep_tokens): a decode step's tokens
+// share no inputs and are each a chain of loads to their sequence's state.  The three kernels of a layer, 64 heads / 128, with
+// one and with eight tokens a thread (us): 8 sequences of one token 17 / 28 and 27 / 42, 64 of them 90 / 174 and 103 / 188, a
+// prompt of 64 tokens 20 / 26 and 24 / 29, of 256 57 / 79 and 58 / 78, of 2,000 403 / 558 and 390 / 534.
+static int ssm_prep_tokens(int n_tokens, int n_seqs) { return n_tokens <= 128 || n_tokens < 4LL * n_seqs ? 1 : 8; }
+template <int TOKENS>
 __global__ void __launch_bounds__(SS_PREP_THREADS) ssm_prep4_kernel(const SsmScan P) {
   pdl_trigger();
   pdl_wait();                // the projection and the state are the work of kernels before this one: ld_fresh
   const int inner = P.n_heads * P.vdim, C = inner + 2 * P.n_groups * P.n_state;
   const int item = blockIdx.y * SS_PREP_THREADS + threadIdx.x;      // four channels, or behind the channels a head
-  const int t0 = blockIdx.x * SS_PREP_TOKENS, t1 = min(P.n_tokens, t0 + SS_PREP_TOKENS);
+  const int t0 = blockIdx.x * TOKENS, t1 = min(P.n_tokens, t0 + TOKENS);
   if (item >= C / 4 + P.n_heads) return;
   if (item >= C / 4) {
     const int h = item - C / 4;
@@ -118,14 +122,14 @@ __global__ void __launch_bounds__(SS_PREP_THREADS) ssm_prep4_kernel(const SsmSca
   }
   const float4 bias = *reinterpret_cast<const float4*>(P.conv_b + c);
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 x[SS_PREP_TOKENS + 3];              // rows t0 - 3 .. t1 - 1, whoever's they are
+  float4 x[TOKENS + 3];                      // rows t0 - 3 .. t1 - 1, whoever's they are
 #pragma unroll
-  for (int i = 0; i < SS_PREP_TOKENS + 3; i++) {
+  for (int i = 0; i < TOKENS + 3; i++) {
     const int t = t0 - 3 + i;
     x[i] = t >= 0 && t < t1 ? ld_fresh(reinterpret_cast<const float4*>(in + (size_t)t * P.ld)) : zero;
   }
 #pragma unroll
-  for (int k = 0; k < SS_PREP_TOKENS; k++) {
+  for (int k = 0; k < TOKENS; k++) {
     const int t = t0 + k;
     if (t >= t1) break;
     const int seq = P.token_seq[t], pos = P.token_pos[t];
@@ -365,15 +369,17 @@ __global__ void __launch_bounds__(SS_THREADS) ssm_recur_kernel(const SsmScan P) 
 // blocks met twice in eight tokens, and whose lanes held half as many entries, for twice the loads); six sequences of 1,000
 // tokens on 64 heads: 786 us a layer with prep and finish, 1,211.  What bounds it is the latency of dependent FMA at seven
 // warps an SM (the FMA pipes are 48 % busy); one, two or four warps a block measure the same.
-#define SW_CHUNK 8
+// CHUNK: tokens staged at a time; eight, or one for steps of a token a sequence, whose warps then fit an SM by their registers
+// and not by ten warps' stages: the layer's three kernels at 64 sequences of one token, 64 heads / 128, 57 / 103 us
+// against 90 / 174.
 #define SW_WARPS 2
-template <int R, int WARPS>
+template <int R, int WARPS, int CHUNK>
 __global__ void __launch_bounds__(WARPS * 32) ssm_recur_warp_kernel(const SsmScan P) {
   constexpr int NP = 64 * (R / 4), G = R / 4, TOKEN = 2 * NP + 8, GROUP_PITCH = 68;
   struct Warp {
-    float in[2][SW_CHUNK][TOKEN];                    // B [NP] | C [NP] | x [8]
-    float dd[2][SW_CHUNK][2];                        // dt, decay
-    float part[SW_CHUNK][2][GROUP_PITCH];
+    float in[2][CHUNK][TOKEN];                    // B [NP] | C [NP] | x [8]
+    float dd[2][CHUNK][2];                        // dt, decay
+    float part[CHUNK][2][GROUP_PITCH];
   };
   extern __shared__ __align__(16) float sw_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane & 15, grp = lane >> 4;
@@ -413,14 +419,14 @@ __global__ void __launch_bounds__(WARPS * 32) ssm_recur_warp_kernel(const SsmSca
       S[q][2 * i + 1] = make_float2(v.z, v.w);
     }
   if (N < NP)                                        // rows beyond n_state stay zero: nothing below writes them
-    for (int i = lane; i < 2 * SW_CHUNK * TOKEN; i += 32) (&sm.in[0][0][0])[i] = 0.f;
+    for (int i = lane; i < 2 * CHUNK * TOKEN; i += 32) (&sm.in[0][0][0])[i] = 0.f;
   __syncwarp();
   const float* act = P.act + inner + (size_t)g * N;
   auto stage = [&](int buf, int c0) {
-    const int n_here = min(SW_CHUNK, r1 - c0);
+    const int n_here = min(CHUNK, r1 - c0);
     const float* a = act + (size_t)c0 * P.lda + 4 * part;
 #pragma unroll
-    for (int tok = 0; tok < SW_CHUNK; tok++)         // half a warp B, half a warp C
+    for (int tok = 0; tok < CHUNK; tok++)         // half a warp B, half a warp C
       if (tok < n_here)
 #pragma unroll
         for (int i = 0; i < G; i++)
@@ -435,11 +441,11 @@ __global__ void __launch_bounds__(WARPS * 32) ssm_recur_warp_kernel(const SsmSca
   };
   stage(0, r0);
   int buf = 0;
-  for (int c0 = r0; c0 < r1; c0 += SW_CHUNK, buf ^= 1) {
+  for (int c0 = r0; c0 < r1; c0 += CHUNK, buf ^= 1) {
     ss_wait_all();
     __syncwarp();                                    // this chunk has landed, and the other buffer is free again
-    if (c0 + SW_CHUNK < r1) stage(buf ^ 1, c0 + SW_CHUNK);
-    const int n_here = min(SW_CHUNK, r1 - c0);
+    if (c0 + CHUNK < r1) stage(buf ^ 1, c0 + CHUNK);
+    const int n_here = min(CHUNK, r1 - c0);
     auto token = [&](int tok) {                      // one token of the chunk: the state moves on, partials out
       const float* in = sm.in[buf][tok];
       float4 b4[G], c4[G];
@@ -470,15 +476,15 @@ __global__ void __launch_bounds__(WARPS * 32) ssm_recur_warp_kernel(const SsmSca
       }
       *reinterpret_cast<float4*>(&sm.part[tok][grp][4 * part]) = make_float4(y[0], y[1], y[2], y[3]);
     };
-    if (n_here == SW_CHUNK) {                        // a whole chunk: the tokens' loads and sums interleave
+    if (n_here == CHUNK) {                        // a whole chunk: the tokens' loads and sums interleave
 #pragma unroll
-      for (int tok = 0; tok < SW_CHUNK; tok++) token(tok);
+      for (int tok = 0; tok < CHUNK; tok++) token(tok);
     } else {
       for (int tok = 0; tok < n_here; tok++) token(tok);
     }
     __syncwarp();                                    // the chunk's partial read-outs are all there
 #pragma unroll
-    for (int o = lane; o < SW_CHUNK * 8; o += 32) {  // (token, column): the 16 lanes' parts, four chains of four
+    for (int o = lane; o < CHUNK * 8; o += 32) {  // (token, column): the 16 lanes' parts, four chains of four
       const int tok = o >> 3, c = o & 7;
       if (tok >= n_here) break;
       const float* p = &sm.part[tok][c >> 2][c & 3];
@@ -499,13 +505,13 @@ __global__ void __launch_bounds__(WARPS * 32) ssm_recur_warp_kernel(const SsmSca
               make_float4(S[q][2 * i].x, S[q][2 * i].y, S[q][2 * i + 1].x, S[q][2 * i + 1].y);
 }
 
-template <int R, int WARPS>
+template <int R, int WARPS, int CHUNK>
 static int ssm_recur_warp_launch(const SsmScan& P, cudaStream_t stream) {
-  const int smem = WARPS * (int)sizeof(float) * (2 * SW_CHUNK * (2 * 64 * (R / 4) + 8) + 2 * SW_CHUNK * 2 + SW_CHUNK * 2 * 68);
-  const cudaError_t e = cudaFuncSetAttribute(ssm_recur_warp_kernel<R, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const int smem = WARPS * (int)sizeof(float) * (2 * CHUNK * (2 * 64 * (R / 4) + 8) + 2 * CHUNK * 2 + CHUNK * 2 * 68);
+  const cudaError_t e = cudaFuncSetAttribute(ssm_recur_warp_kernel<R, WARPS, CHUNK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
   const dim3 grid((P.vdim / 8 + WARPS - 1) / WARPS, P.n_heads, P.n_seqs);
-  ssm_recur_warp_kernel<R, WARPS><<<grid, WARPS * 32, smem, stream>>>(P);
+  ssm_recur_warp_kernel<R, WARPS, CHUNK><<<grid, WARPS * 32, smem, stream>>>(P);
   return launch_status();
 }
 
@@ -637,8 +643,11 @@ STRATUM_EXPORT int stratum_ssm_scan(const SsmScan* params, int out_dtype, cudaSt
   const bool rows16 = all % 16 == 0 && P.ld % 4 == 0 && P.lda % 4 == 0 && P.ldo % 4 == 0 && P.state_stride % 4 == 0 &&
                       inner % 4 == 0 && P.n_state % 4 == 0;
   if (rows16 && P.taps == 4) {
-    launch_pdl(ssm_prep4_kernel, dim3((P.n_tokens + SS_PREP_TOKENS - 1) / SS_PREP_TOKENS,
-                                      (C / 4 + P.n_heads + SS_PREP_THREADS - 1) / SS_PREP_THREADS), SS_PREP_THREADS, 0, stream, P);
+    const int pieces = (C / 4 + P.n_heads + SS_PREP_THREADS - 1) / SS_PREP_THREADS;
+    if (ssm_prep_tokens(P.n_tokens, P.n_seqs) == 1)
+      launch_pdl(ssm_prep4_kernel<1>, dim3(P.n_tokens, pieces), SS_PREP_THREADS, 0, stream, P);
+    else
+      launch_pdl(ssm_prep4_kernel<8>, dim3((P.n_tokens + 7) / 8, pieces), SS_PREP_THREADS, 0, stream, P);
   } else {
     const int items = C + P.n_heads;
     launch_pdl(ssm_prep_kernel, dim3(P.n_tokens, (items + SS_PREP_THREADS - 1) / SS_PREP_THREADS), SS_PREP_THREADS, 0,
@@ -647,7 +656,10 @@ STRATUM_EXPORT int stratum_ssm_scan(const SsmScan* params, int out_dtype, cudaSt
   int st = launch_status();
   if (st) return st;
   if (rows16 && P.n_state > 32 && P.n_state <= 128 && P.vdim % 8 == 0) {
-    st = P.n_state > 64 ? ssm_recur_warp_launch<8, SW_WARPS>(P, stream) : ssm_recur_warp_launch<4, SW_WARPS>(P, stream);
+    if (P.n_tokens <= P.n_seqs)
+      st = P.n_state > 64 ? ssm_recur_warp_launch<8, SW_WARPS, 1>(P, stream) : ssm_recur_warp_launch<4, SW_WARPS, 1>(P, stream);
+    else
+      st = P.n_state > 64 ? ssm_recur_warp_launch<8, SW_WARPS, 8>(P, stream) : ssm_recur_warp_launch<4, SW_WARPS, 8>(P, stream);
     if (st) return st;
   // few rows per lane while a warp still covers the rows: 4 up to 128 rows, 8 up to 256, 16 beyond
   } else if (P.n_state > 256) ssm_recur_launch<32, 16>(P, stream);

@@ -164,6 +164,43 @@ def test_state_space_kernels_on_aligned_rows(heads, vdim, state, groups, taps, p
     assert float(st[0].abs().max()) == 0.0 and float(st[2].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("state,groups", [(128, 1), (64, 2), (36, 1)])
+def test_state_space_steps_of_one_token_give_the_same_bits(state, groups):
+    """Three sequences and a padding row, token by token, against prompts of few and of many tokens: every form of the
+    convolution and of the recurrence's staging does the same arithmetic."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(state)
+    heads, vdim, taps, T = 4, 16, 4, 150
+    inner, C = heads * vdim, heads * vdim + 2 * groups * state
+    width = inner + C + heads
+    up = lambda n: -(-n // 4) * 4
+    f = lambda lo, hi, *shape: _dev(rng.uniform(lo, hi, shape))
+    weights = (f(-0.8, 0.8, C, taps), f(-0.3, 0.3, C), f(-2, 0.5, heads), f(-1, 1, heads), f(-1, 1.5, heads), f(0.5, 1.5, inner))
+    proj = torch.zeros(3, T, up(width), device="cuda")
+    proj[:, :, :width] = _dev(rng.standard_normal((3, T, width)))
+
+    def run(cuts):
+        st, done, got = torch.zeros(4, up(inner * state + 3 * C), device="cuda"), 0, []
+        for n in cuts:
+            rows = torch.cat([proj[:, done:done + n].reshape(3 * n, -1), torch.ones(1, up(width), device="cuda")])
+            pos = np.concatenate([np.arange(done, done + n)] * 3 + [[0]])
+            seq = np.concatenate([np.repeat([0, 1, 2], n), [-1]])
+            out = torch.empty(3 * n + 1, inner, device="cuda")
+            K.ssm_scan(rows, *weights, torch.empty(3 * n + 1, up(C + 2 * heads), device="cuda"),
+                       torch.empty(3 * n + 1, inner, device="cuda"), out, st, _dev(pos, torch.int32), _dev(seq, torch.int32),
+                       _dev(np.array([0, n, 2 * n, 3 * n, 3 * n + 1]), torch.int32), _dev(np.array([2, 0, 1, 3]), torch.int32),
+                       heads, vdim, state, groups, 2, 1e-5, True)
+            got.append(out[:-1].reshape(3, n, inner))
+            assert not out[-1].any()
+            done += n
+        return torch.cat(got, dim=1), st
+
+    want, end = run([T])                                               # 451 rows
+    for cuts in ([1] * T, [40, 1, 9, 1, 1, 8, T - 60]):
+        got, st = run(cuts)
+        assert torch.equal(got, want) and torch.equal(st, end), cuts[:7]
+
+
 def test_state_space_kernel_leaves_the_state_alone_when_told_to():
     from stratum_b200 import kernels as K
     rng = np.random.default_rng(3)
