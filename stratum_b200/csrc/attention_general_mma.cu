@@ -500,7 +500,6 @@ attention_general_decode_kernel(const GeneralAttention P, const int stages) {
   }
   const int n_vc = (Dv + 31) / 32;
   const bool upper = heads_here - my_rg * 16 > 8;    // whether rows 8 .. 15 of this warp's group are anyone's
-  const float inv_cap = P.softcap > 0.f ? 1.0f / P.softcap : 0.f;
   int stage = 0;
   for (int key0 = from(k_begin); key0 < k_end; key0 = from(key0 + GM_TILE)) {
     if (stages == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -537,7 +536,7 @@ attention_general_decode_kernel(const GeneralAttention P, const int stages) {
         const int e = j >> 1, key = key0 + 16 * my_kb + 8 * i + 2 * t + (j & 1);
         if (e && !upper) { s[i][j] = 0.f; continue; }
         float v = s[i][j] * factor[e];
-        if (P.softcap > 0.f) v = P.softcap * tanhf(v * inv_cap);
+        if (P.softcap > 0.f) v = P.softcap * tanhf(v / P.softcap);
         if (P.slope) v -= slope[e] * (float)(pos - key);
         if (!whole_tile && !(key < k_end && key >= k_begin && (key >= lo || key < keep))) v = -INFINITY;
         s[i][j] = v;
@@ -688,7 +687,10 @@ static int gm_decode_stages(int qk_dim, int v_dim, int v_in_k, int rg) {       /
 // CTAs of a decode step worth planning for (0: the shape is not the decode kernel's).  One to an SM where a CTA takes an SM's
 // shared memory: its two tiles overlap, two waves of single tiles do not (latent rows of 576, six sequences: 26 us with the
 // finishing kernel against 33 with 296 CTAs wanted).  Else several to a place, since sequences are of unequal length
-// (differential heads of 64: 30 us with 592, 35 with 444, 39 with 296, 64 with 148).
+// (differential heads of 64: 30 us with 592, 35 with 444, 39 with 296, 64 with 148).  A step of four layers, three latent and one
+// differential, planned so / with 148 / 296 / 592 for either kind (us): 8 sequences of 4,090 tokens 660 / 746 / 719 / 721 on
+// a width of 4,096 and 360 / 424 / 371 / 367 on 2,048, one of 4,090 528 / 543 / 531 / 528, 16 of 2,000 720 / 715 / 707 / 730,
+// 64 of 500 873 / 877 / 876 / 897.
 STRATUM_EXPORT int stratum_attention_general_decode_ctas(int group, int qk_dim, int v_dim, int v_in_k) {
   const int rows = stratum_attention_general_decode_rows(group, qk_dim, v_dim, v_in_k);
   if (rows == 0) return 0;

@@ -43,7 +43,7 @@ struct MixerPrep {
 };
 
 // Steps of up to 64 tokens give a token eight blocks: with one, six tokens of 32 heads were a chain of 16 to 48 turns of a
-// block on six SMs, 8.6 us; now 4.3.  (More tokens fill the SMs by themselves, and every block evaluates the angles.)
+// block on six SMs, 8.6 us; now 4.3, and at 64 tokens half of what one block took, too.  (More tokens fill the SMs by themselves, and every block evaluates the angles.)
 #define MP_FEW_TOKENS 64
 #define MP_BLOCKS 8
 

@@ -572,3 +572,27 @@ def test_general_attention_of_decode_steps(heads, group, maps, D, Dv, v_in_k, ex
     assert not out[-1].any()
     # both round once to bfloat16; between them the probabilities' 16 bits
     assert float((out.float() - ref.float()).abs().max()) <= 2.0 ** -7 * float(ref.float().abs().max())
+
+
+@pytest.mark.parametrize("cap", [3.0, 5.0, 30.0])
+def test_capped_scores_are_the_same_in_decode_steps_and_prompts(cap):
+    """Dot products of whole numbers, exact in either kernel: what the cap makes of a range's largest score is the same
+    float32 from the decode kernel as from the prompt form."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(int(cap))
+    heads, group, D, Dv, splits, lens = 16, 4, 64, 32, 4, [256, 200, 131, 64]
+    whole = lambda *shape: torch.tensor(rng.integers(-2, 3, shape), dtype=torch.bfloat16, device="cuda")
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    T = len(lens)
+    kc, vc, q = whole(4 * T, 2 * heads // group, 64, D), whole(4 * T, heads // group, 64, Dv), whole(T, heads * 2 * D)
+    table = i32(np.arange(4 * T).reshape(T, 4))
+    pos, seq = i32([n - 1 for n in lens]), i32(list(range(T)))
+    shape = K.AttentionShape(heads, group, 2, D, Dv, False, D ** -0.5, softcap=cap, lam=0.3, out_scale=0.8, eps=1e-6)
+    maxima = []
+    for blocks, per in ((None, 1), ((seq, i32(list(range(T))), i32([1] * T)), 4)):
+        n = T * heads * 2 * splits
+        part_ml = torch.zeros(n, 2, device="cuda")
+        K.attention_general_mma(shape, q, kc, vc, pos, seq, table, torch.empty(T, heads * Dv, dtype=torch.bfloat16, device="cuda"),
+                                64, blocks, per, splits, 64, torch.empty(n * Dv, device="cuda"), part_ml)
+        maxima.append(part_ml[:, 0].reshape(T, heads, 2, splits))
+    assert torch.isfinite(maxima[0][0]).all() and torch.equal(*maxima)
