@@ -177,7 +177,7 @@ STRATUM_EXPORT int stratum_argmax(const float* logits, int ld, int n_rows, int v
 
 // order-preserving map float -> uint32 (larger float, larger key; the two zeros are equals), and back
 __device__ __forceinline__ uint32_t float_key(float f) {
-  const uint32_t u = __float_as_uint(__fadd_rn(f, 0.f));
+  const uint32_t u = f == 0.f ? 0u : __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 __device__ __forceinline__ float key_float(uint32_t key) {
@@ -497,8 +497,7 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab, const float* 
 // nothing hidden among the row's k largest if the key its leavings out lie below is at most the key of the k-th largest of
 // all lists.  With 128,256 logits and k = 512 the k-th largest is the 99.6th percentile of the row, a stretch's 64th
 // largest the 98.4th of its own, so the check holds unless the large logits crowd in one stretch; when it does not hold
-// (or logits equal to one another straddle a cut that the lists, which are in no order, cannot make) the row is marked and
-// the one-block kernel, launched behind this one for marked rows only, does the row by itself.
+// the row is marked and the one-block kernel, launched behind this one for marked rows only, does the row by itself.
 //
 // 128,256 logits, top-k 50, top-p 0.95 (us, 1 / 24 / 64 rows): 21 / 31 / 48; with two radix selections and lists in id
 // order it took 36 / 61 / 113, and one block a row takes 87.  k = 512: 43 / 54 / 72 against 47 / 72 / 125.
@@ -562,20 +561,13 @@ __device__ unsigned radix_kth(Key key_of, int n, int k, unsigned* hist, unsigned
   return sh[1];
 }
 
-// Among n values in ascending id order (val(j), id(j)), the k largest, the lowest ids first among equals at the
-// cut, written in ascending id order to out_v / out_i.  Returns how many (min(k, n)); *kth_key gets the key of the
-// smallest of them (0 if all n were taken).  Every thread of the block calls it.  hist: 256 words, sh: 2,
-// w_scratch: 2 * SS_WARPS.
+// Among n values in ascending id order (val(j), id(j)), the k largest, k < n, the lowest ids first among equals at the
+// cut, written in ascending id order to out_v / out_i; *kth_key gets the key of the smallest of them.  Every thread of the
+// block calls it.  hist: 256 words, sh: 2, w_scratch: 2 * SS_WARPS.
 template <typename Val, typename Id>
-__device__ int select_in_order(Val val, Id id, int n, int k, float* out_v, int* out_i, unsigned* hist, unsigned* sh,
+__device__ void select_in_order(Val val, Id id, int n, int k, float* out_v, int* out_i, unsigned* hist, unsigned* sh,
                                unsigned* w_scratch, unsigned* w_scratch33, uint32_t* kth_key) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (k >= n) {
-    for (int j = tid; j < n; j += SS_THREADS) { out_v[j] = val(j); out_i[j] = id(j); }
-    __syncthreads();
-    *kth_key = 0u;
-    return n;
-  }
   uint32_t kth, equals;
   const unsigned want_eq = radix_kth([&](int j) { return float_key(val(j)); }, n, k, hist, sh, w_scratch33, &kth, &equals);
   // in id order, 256 ids a round: an element's rank among the equal ones and its place in the output are counts of
@@ -604,14 +596,13 @@ __device__ int select_in_order(Val val, Id id, int n, int k, float* out_v, int* 
   }
   __syncthreads();
   *kth_key = kth;
-  return k;
 }
 
 // At least the k largest of n, k <= SS_THREADS, by their keys: thread t's largest element is one of SS_THREADS maxima, and
 // the k-th largest of those is at most the k-th largest of all.  put(slot, key, j) is called for every element that
 // reaches it (a little more than k of them as a rule, in any order; all of those with that key) whose slot is below
-// `room`.  Returns how many there are; *least_of gets the key.  Three barriers in place of the radix passes' sixteen and
-// two per 256 elements.  maxima: SS_THREADS words; sh: 2.
+// `room`.  Returns how many there are; *least_of gets the key.  Three barriers in place of the radix passes' 24 and two
+// per 256 elements.  maxima: SS_THREADS words; sh: 2.
 template <typename Key, typename Put>
 __device__ __forceinline__ unsigned gather_largest(Key key, Put put, int n, int k, unsigned room, uint32_t* maxima,
                                                    unsigned* sh, uint32_t* least_of) {
@@ -733,21 +724,16 @@ sample_split_kernel(const float* __restrict__ logits, int ld, int vocab, const f
       to_v[slot] = __uint_as_float(key);
       to_i[slot] = b0 + j;
     };
-    uint32_t below = 0u;
-    unsigned kept;
-    if (n <= SS_LIST) {                             // (so few that all are kept)
-      for (int j = tid; j < n; j += SS_THREADS) put(j, float_key(lv[j]), j);
-      kept = n;
-    } else {
-      kept = gather_largest([&](int j) { return float_key(lv[j]); }, put, n, k1, SS_LIST, hist, sh, &below);
-      if (kept > SS_LIST) {                         // a crowd of equals: exactly k1, the lowest ids first among equals
-        __syncthreads();                            // (everyone knows how many were gathered)
-        uint32_t kth;
-        kept = select_in_order([&](int j) { return lv[j]; }, [&](int j) { return b0 + j; }, n, k1, cand_v, cand_i, hist, sh,
-                               w_scratch, u_scratch, &kth);
-        for (int j = tid; j < (int)kept; j += SS_THREADS) { to_v[j] = __uint_as_float(float_key(cand_v[j])); to_i[j] = cand_i[j]; }
-        below = kth == 0xffffffffu ? kth : kth + 1;
-      }
+    uint32_t below;                                 // (a stretch has more ids than are kept of it: the launcher's least vocabulary)
+    unsigned kept = gather_largest([&](int j) { return float_key(lv[j]); }, put, n, k1, SS_LIST, hist, sh, &below);
+    if (kept > SS_LIST) {                           // a crowd of equals: exactly k1, the lowest ids first among equals
+      __syncthreads();                              // (everyone knows how many were gathered)
+      uint32_t kth;
+      select_in_order([&](int j) { return lv[j]; }, [&](int j) { return b0 + j; }, n, k1, cand_v, cand_i, hist, sh, w_scratch,
+                      u_scratch, &kth);
+      kept = k1;
+      for (int j = tid; j < k1; j += SS_THREADS) { to_v[j] = __uint_as_float(float_key(cand_v[j])); to_i[j] = cand_i[j]; }
+      below = kth == 0xffffffffu ? kth : kth + 1;
     }
     if (tid == 0) {
       Q.part_key[part] = below;
@@ -845,7 +831,6 @@ sample_split_kernel(const float* __restrict__ logits, int ld, int vocab, const f
     const int upto = warp_incl_scan(mine_n);
     list_at[lane] = upto - mine_n;
     if (lane == 31) list_at[SS_SPLITS] = upto;
-    if (lane == 0) { sh_owner = 0; sh[1] = 0u; }
   }
   __syncthreads();
   uint32_t* lk = reinterpret_cast<uint32_t*>(lv);
@@ -867,8 +852,8 @@ sample_split_kernel(const float* __restrict__ logits, int ld, int vocab, const f
   __syncthreads();
   const int n_cand = k;
   uint32_t kth = 0u;
-  bool sorted = false, given_up = n_all < k;         // (fewer candidates than k in all: the lists do not hold k)
-  if (k <= SS_FEW && !given_up) {
+  bool sorted = false;                               // (the lists hold k in all: 32 min(k, SS_KEEP) at least)
+  if (k <= SS_FEW) {
     uint32_t least;
     const unsigned found = gather_largest([&](int j) { return lk[j]; },
                                           [&](unsigned slot, uint32_t key, int j) { f_key[slot] = key; f_id[slot] = id_of(j); },
@@ -883,29 +868,31 @@ sample_split_kernel(const float* __restrict__ logits, int ld, int vocab, const f
     }
     __syncthreads();                                 // (everyone knows how many were gathered, and the k-th key)
   }
-  if (!sorted && !given_up) {
-    uint32_t equals;
-    const unsigned wanted = radix_kth([&](int j) { return lk[j]; }, n_all, k, hist, sh, u_scratch, &kth, &equals);
-    // equals that straddle the cut would have to be taken by their ids, which come in no order here
-    given_up = wanted != equals;
-    __syncthreads();
-    if (tid == 0) sh[0] = 0u;
-    __syncthreads();
-    if (!given_up)
-      for (int j = tid; j < n_all; j += SS_THREADS)
-        if (lk[j] >= kth) {
-          const unsigned slot = atomicAdd(&sh[0], 1u);
-          cand_v[slot] = key_float(lk[j]);
-          cand_i[slot] = id_of(j);
-        }
-    __syncthreads();
-  }
+  uint32_t equals = 0u;
+  const unsigned wanted = sorted ? 0u : radix_kth([&](int j) { return lk[j]; }, n_all, k, hist, sh, u_scratch, &kth, &equals);
   // is anything that a stretch did not keep among the row's k largest?
-  if (tid < SS_SPLITS && k1 < k && __ldcg(Q.part_key + r * SS_SPLITS + tid) > kth) sh_owner = 1;
-  __syncthreads();
-  if (given_up || sh_owner) {
+  if (__syncthreads_or(tid < SS_SPLITS && k1 < k && __ldcg(Q.part_key + r * SS_SPLITS + tid) > kth)) {
     if (tid == 0) Q.redo[r] = 1;
     return;
+  }
+  if (!sorted) {
+    uint32_t last_id = 0u;                           // (ids turned round: of equals the lower id is the larger)
+    if (wanted != equals) {                          // equals straddle the cut: the lowest ids of them, by one more selection
+      uint32_t one;
+      radix_kth([&](int j) { return lk[j] == kth ? ~(uint32_t)id_of(j) : 0u; }, n_all, wanted, hist, sh, u_scratch, &last_id, &one);
+      __syncthreads();
+    }
+    if (tid == 0) sh[0] = 0u;
+    __syncthreads();
+    for (int j = tid; j < n_all; j += SS_THREADS)
+      if (lk[j] >= kth) {
+        const int id = id_of(j);
+        if (lk[j] == kth && ~(uint32_t)id < last_id) continue;
+        const unsigned slot = atomicAdd(&sh[0], 1u);
+        cand_v[slot] = key_float(lk[j]);
+        cand_i[slot] = id;
+      }
+    __syncthreads();
   }
   // pad to a power of two and sort: descending logit, ascending id among equals (bitonic, in shared memory)
   int n_sort = 1;

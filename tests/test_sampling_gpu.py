@@ -178,3 +178,27 @@ def test_rows_cut_over_blocks_pick_what_one_block_picks(vocab, k):
         got.append((ids.tolist(), vals.tolist()))
     assert got[0] == got[1]
     assert all(rows[r, i] == v for r, (i, v) in enumerate(zip(*got[0])))
+
+
+@pytest.mark.parametrize("vocab", [5000, 8192, 128256])
+@pytest.mark.parametrize("k,top_p", [(1, 1.0), (40, 0.9), (200, 1.0), (0, 0.9)])
+def test_filters_pass_over_the_lowest_nan(vocab, k, top_p):
+    """A NaN with its sign set (what x86 makes of an invalid operation) orders below everything, as it always has: a filtered
+    draw picks what it would with -inf in its place."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(vocab + k)
+    rows = rng.standard_normal((4, vocab)).astype(np.float32) * 3
+    at = rng.permutation(vocab)[:7]
+    rows[:, at] = -np.inf
+    holes = rows.copy()
+    holes.view(np.uint32)[:, at] = 0xFFC00000
+    u = _dev(rng.random(4), torch.float32)
+    for one_block in (False, True):
+        got = []
+        for logits in (rows, holes):
+            ids = torch.empty(4, dtype=torch.int32, device="cuda")
+            vals = torch.empty(4, dtype=torch.float32, device="cuda")
+            K.sample(torch.from_numpy(logits).cuda(), _dev([0.9] * 4, torch.float32), _dev([k] * 4, torch.int32),
+                     _dev([top_p] * 4, torch.float32), u, ids, vals, one_block_per_row=one_block)
+            got.append((ids.tolist(), vals.tolist()))
+        assert got[0] == got[1]
