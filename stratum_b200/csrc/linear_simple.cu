@@ -13,7 +13,7 @@
 //             fma.rn.f32x2, whose operands then are two neighbouring values of a row as they lie in memory, and the
 //             segments are what few rows of x, or few tiles, are spread over the GPU by.
 //
-// Epilogues: 0 store as T; 1 add into a float32 tensor in place (the residual stream);
+// Epilogues: 0 store as x's type; 1 add into a float32 tensor in place (the residual stream);
 //            2 store as float32 (logits).
 #include "common.cuh"
 
@@ -24,9 +24,9 @@
 #define LS_TM 4
 #define LS_TN 4
 
-template <typename T, int EPI>
+template <int EPI>
 __global__ void __launch_bounds__(256)
-linear_simple_kernel(const T* __restrict__ x, const T* __restrict__ w, const float* __restrict__ bias,
+linear_simple_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const float* __restrict__ bias,
                      void* __restrict__ out, int M, int N, int K, int ldx, int ldo, int x_step, long long w_step,
                      int o_step, int act) {
   __shared__ float xs[LS_BK][LS_BM + 1];
@@ -80,26 +80,25 @@ linear_simple_kernel(const T* __restrict__ x, const T* __restrict__ w, const flo
       float v = acc[i][j];
       if (bias) v += bias[n];
       const size_t o = (size_t)m * ldo + n + o_shift;
-      if (EPI == 0) ((T*)out)[o] = from_float<T>(activate(v, act));
+      if (EPI == 0) ((bf16*)out)[o] = __float2bfloat16_rn(activate(v, act));
       else if (EPI == 1) ((float*)out)[o] += v;
       else ((float*)out)[o] = v;
     }
   }
 }
 
-template <typename T>
 static int launch_linear_simple(const void* x, const void* w, const float* bias, void* out, int epilogue,
                                 int M, int N, int K, int ldx, int ldo, cudaStream_t stream, int heads = 1,
                                 int x_step = 0, long long w_step = 0, int o_step = 0, int act = 0) {
   dim3 grid((N + LS_BN - 1) / LS_BN, (M + LS_BM - 1) / LS_BM, heads);
   if (epilogue == 0)
-    linear_simple_kernel<T, 0><<<grid, 256, 0, stream>>>((const T*)x, (const T*)w, bias, out, M, N, K, ldx, ldo,
+    linear_simple_kernel<0><<<grid, 256, 0, stream>>>((const bf16*)x, (const bf16*)w, bias, out, M, N, K, ldx, ldo,
                                                       x_step, w_step, o_step, act);
   else if (epilogue == 1)
-    linear_simple_kernel<T, 1><<<grid, 256, 0, stream>>>((const T*)x, (const T*)w, bias, out, M, N, K, ldx, ldo,
+    linear_simple_kernel<1><<<grid, 256, 0, stream>>>((const bf16*)x, (const bf16*)w, bias, out, M, N, K, ldx, ldo,
                                                       x_step, w_step, o_step, act);
   else if (epilogue == 2)
-    linear_simple_kernel<T, 2><<<grid, 256, 0, stream>>>((const T*)x, (const T*)w, bias, out, M, N, K, ldx, ldo,
+    linear_simple_kernel<2><<<grid, 256, 0, stream>>>((const bf16*)x, (const bf16*)w, bias, out, M, N, K, ldx, ldo,
                                                       x_step, w_step, o_step, act);
   else
     return STRATUM_ERR_SHAPE;
@@ -534,7 +533,7 @@ STRATUM_EXPORT int stratum_linear_simple(const void* x, const void* w, const flo
   if (dtype == STRATUM_DT_F32)
     return launch_linear_f32(x, w, bias, out, epilogue, M, N, K, ldx, ldo, scratch, stream, 1, 0, 0, 0, act);
   if (dtype == STRATUM_DT_BF16)
-    return launch_linear_simple<bf16>(x, w, bias, out, epilogue, M, N, K, ldx, ldo, stream, 1, 0, 0, 0, act);
+    return launch_linear_simple(x, w, bias, out, epilogue, M, N, K, ldx, ldo, stream, 1, 0, 0, 0, act);
   return STRATUM_ERR_DTYPE;
 }
 
@@ -553,7 +552,7 @@ STRATUM_EXPORT int stratum_linear_heads(const void* x, const void* w, void* out,
     return launch_linear_f32(x, w, nullptr, out, epilogue, M, N, K, ldx, ldo, scratch, stream, heads, x_step, w_step,
                              o_step);
   if (dtype == STRATUM_DT_BF16)
-    return launch_linear_simple<bf16>(x, w, nullptr, out, epilogue, M, N, K, ldx, ldo, stream, heads, x_step, w_step,
+    return launch_linear_simple(x, w, nullptr, out, epilogue, M, N, K, ldx, ldo, stream, heads, x_step, w_step,
                                       o_step);
   return STRATUM_ERR_DTYPE;
 }
