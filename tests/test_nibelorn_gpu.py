@@ -44,6 +44,21 @@ def test_dynamic_tanh_kernel(dtype):
     assert torch.equal(part, out[[5, 0, 36]])
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("hidden", [4, 203, 1024, 1028, 4096])
+def test_dynamic_tanh_kernel_widths(dtype, hidden):
+    """Rows in 16-byte pieces over one block and over several, and rows that end between them."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(hidden)
+    x = rng.normal(size=(3, hidden)) * 3
+    w, b, alpha = rng.uniform(0.5, 1.5, hidden), rng.normal(size=hidden) * 0.2, 0.7
+    dev = lambda a: torch.tensor(a, dtype=torch.float32, device="cuda")                     # noqa: E731
+    out = torch.empty((3, hidden), dtype=torch.float32 if dtype == "float32" else torch.bfloat16, device="cuda")
+    K.dynamic_tanh(dev(x), dev([alpha]), dev(w), dev(b), out)
+    ref = N.dynamic_tanh(np.float32(x), np.float32(w), np.float32(b), np.float32(alpha))
+    assert np.max(np.abs(out.float().cpu().numpy() - ref)) <= (2e-6 if dtype == "float32" else 1e-2)
+
+
 def test_gelu_kernel_both_forms():
     from stratum_b200 import kernels as K
     z = np.linspace(-6, 6, 1001).astype(np.float32).reshape(7, 143)
@@ -414,6 +429,23 @@ def test_per_head_products(rows, heads, n, k, x_step, o_step):
         assert np.max(np.abs(got[:, j * o_step: j * o_step + n] - ref)) <= 2 ** -8 * max(1.0, np.max(np.abs(ref)))
     if o_step > n:                                         # columns between the heads' results are left alone
         assert np.all(got[:, n:o_step] == 7.0)
+
+
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17])
+@pytest.mark.parametrize("n,k", [(24, 520), (16, 1032), (72, 128), (8, 136)])
+def test_per_head_products_of_few_rows(rows, n, k):
+    """The kernel for up to 16 rows through one and several turns of its loop over k, and the row behind its last: the same
+    bits, since either adds in the order of k."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(rows + n)
+    x = torch.tensor(rng.normal(size=(rows, 3 * k)), dtype=torch.bfloat16, device="cuda")
+    w = torch.tensor(rng.normal(size=(3, n, k)) * 0.2, dtype=torch.bfloat16, device="cuda")
+    out, want = (torch.full((r, 3 * n), 7.0, dtype=torch.bfloat16, device="cuda") for r in (rows, 40))
+    K.head_gemm(x, w, out, k, n)
+    K.head_gemm(torch.cat([x, torch.zeros(40 - rows, 3 * k, dtype=x.dtype, device="cuda")]), w, want, k, n)
+    ref = np.einsum("mjk,jnk->mjn", x.double().cpu().numpy().reshape(rows, 3, k), w.double().cpu().numpy()).reshape(rows, -1)
+    assert np.max(np.abs(out.double().cpu().numpy() - ref)) <= 2 ** -8 * max(1.0, np.max(np.abs(ref)))
+    assert torch.equal(out, want[:rows])
 
 
 # ------------------------------------------------------------------------------------------ the programs

@@ -75,3 +75,6 @@ def test_shapes_and_picking_kinds():
     assert pick_kind(8, 0.7, 0, 1.0) == PICK_DRAW and pick_kind(64, 0.7, 0, 1.0) == PICK_DRAW
     assert pick_kind(32, 0.7, 50, 1.0) == PICK_DRAW               # up to 32 rows the 32-block kernel filters too
     assert pick_kind(40, 0.7, 50, 1.0) == PICK_FILTERED_MANY_ROWS and pick_kind(64, 0.7, 0, 0.9) == PICK_FILTERED_MANY_ROWS
+    # with longer rows up to a row per thousand logits (and 32 of any length)
+    assert pick_kind(128, 0.7, 50, 1.0, 128256) == PICK_DRAW and pick_kind(136, 0.7, 50, 1.0, 128256) == PICK_FILTERED_MANY_ROWS
+    assert pick_kind(32, 0.7, 50, 1.0, 8192) == PICK_DRAW and pick_kind(40, 0.7, 0, 0.9, 32000) == PICK_FILTERED_MANY_ROWS
