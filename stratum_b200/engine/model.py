@@ -19,6 +19,7 @@ from ..config.registry import find_architecture
 from ..parts import find_part
 from ..parts.base import Runtime
 from ..parts.spec import LayerSpec, ModelSpec, TensorSpec
+from .resident import ResidentSteps
 from ..weights.loader import check_tensors, load_weights, place, tensor_shapes
 
 
@@ -79,6 +80,8 @@ class Model:
                          if spec.position is not None else None)
         self.schedule = spec.schedule
         self.hidden, self.vocab = spec.hidden, spec.vocab
+        self._resident: Optional[ResidentSteps] = None      # made with the first step of single tokens (it needs the device)
+        self._resident_asked = False
 
     # ------------------------------------------------------------------ description
     def tensors(self) -> Dict[str, TensorSpec]:
@@ -126,6 +129,12 @@ class Model:
             parts += list(layer.parts()) + [layer.arrangement]
         return all(getattr(p, "replays_prompts", False) for p in parts)
 
+    def resident_steps(self) -> Optional[ResidentSteps]:
+        """How decode steps of a few rows run as one kernel; None where the model's parts are not the ones it knows."""
+        if not self._resident_asked:
+            self._resident, self._resident_asked = ResidentSteps.of(self), True
+        return self._resident
+
     # ------------------------------------------------------------------ forward
     def forward(self, step, cache) -> torch.Tensor:
         """Run the tokens of one step through every stop of the schedule; float32 logits at the wanted rows."""
@@ -135,6 +144,10 @@ class Model:
             self.position.add_to_embedding(x, step)
             if self.spec.keep_embedded:
                 self.position.add_to_embedding(step.embedded, step)
+        if step.all_single:
+            plan = self.resident_steps()
+            if plan is not None and plan.takes(step):
+                return plan.run(x, step, cache)
         carry = None                  # rows a layer's last product prepared for the next layer's first norm
         for stop, entry in enumerate(self.schedule):
             layer = self.layers[entry.layer]

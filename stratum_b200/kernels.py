@@ -491,7 +491,9 @@ def check_status() -> None:
     if code != 0:
         _status_word.zero_()
         where = {101: "the TMA producer waiting for a free stage", 102: "the MMA warp waiting for a free accumulator",
-                 103: "the MMA warp waiting for a loaded stage", 104: "the epilogue waiting for an accumulator"}
+                 103: "the MMA warp waiting for a loaded stage", 104: "the epilogue waiting for an accumulator",
+                 431: "the resident decode step's ring (a free stage)", 432: "the resident decode step's ring (a filled stage)",
+                 **{c: "a block of the resident decode step waiting for the others" for c in (401, 402, 403, 405, 411, 421)}}
         raise KernelError(f"a device-side wait ran out in {where.get(code, f'code {code}')}; results are invalid")
 
 
@@ -1653,6 +1655,102 @@ def attention_stream(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
              _ptr(status_word()),
              _stream()), "attention_stream")
     count_launches(1)
+
+
+# ------------------------------------------------------------------ a decode step's layers as one kernel
+DECODE_LAYERS_MAX, DECODE_LAYERS_MAX_ROWS = 96, 16
+
+
+class _DecodeLayer(ctypes.Structure):
+    """Mirror of struct DlLayer in csrc/decode_layers.cu."""
+    _fields_ = [(n, c_void_p) for n in ("w_qkv", "w_o", "w_gu", "w_down", "gain_ff", "gain_next", "k", "v")]
+
+
+class _DecodeLayers(ctypes.Structure):
+    """Mirror of struct DlParams in csrc/decode_layers.cu."""
+    _fields_ = [(n, c_void_p) for n in ("x", "gain_first", "w_head", "logits", "xb", "qb", "ob", "ab", "ss", "part_o",
+                                        "part_ml", "counters", "rope", "pos", "seq", "block_table", "status")] + \
+               [(n, c_int) for n in ("bt_stride", "n_layers", "M", "H", "F", "n_q", "n_kv", "D", "n_pairs", "window",
+                                     "vocab")] + \
+               [("eps", c_float), ("scale", c_float), ("layer", _DecodeLayer * DECODE_LAYERS_MAX)]
+
+
+def sm_count(device) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
+def decode_layers_sizes_ok(H: int, F: int, vocab: int, n_q: int, n_kv: int, head_dim: int, device) -> bool:
+    """Whether the resident kernel takes a model of these sizes: k in 128s, rows of x of the products over H and over the heads
+    in registers (4,096), two tiles of the stream and two rows of every matrix a block."""
+    blocks, KO = sm_count(device), n_q * head_dim
+    return (head_dim in (64, 128) and n_q // n_kv <= 8 and H % 128 == 0 and F % 128 == 0 and KO % 128 == 0 and H <= 4096
+            and KO <= 4096 and (H // 2 + blocks - 1) // blocks <= 16 and H >= 2 * blocks and F >= blocks
+            and vocab % 2 == 0 and vocab >= 2 * blocks and KO + 2 * n_kv * head_dim >= 2 * blocks)
+
+
+def decode_layers_takes(rows: int, n_kv: int, table_width: int, device) -> bool:
+    """Whether the resident kernel's lists of pages hold what page tables of that width may name (16 sequences of
+    65,536 tokens with 8 kv heads, on 148 SMs)."""
+    return rows * n_kv * table_width <= (1024 - 17) * sm_count(device)
+
+
+def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: torch.Tensor, logits: torch.Tensor,
+                  rope: Optional[torch.Tensor], token_pos: torch.Tensor, token_seq: torch.Tensor,
+                  block_table: torch.Tensor, n_q: int, n_kv: int, head_dim: int, window: int, scale: float,
+                  eps: float) -> None:
+    """All layers of a dense decoder and its head for a step of one new token per sequence, in one kernel that stays on
+    every SM: x float32 [rows, H] (embedded), layers a list of (w_qkv, w_o, w_gate_up, w_down, gain of the feed-forward's
+    norm, gain of the norm behind the layer, k_cache, v_cache), logits float32 [rows, vocab].  Weights bfloat16, gate and up
+    rows alternating, rotated pairs neighbours; rope: (cos, sin) [rows, pairs, 2] or None.  At most 16 rows."""
+    H, rows = x.shape[1], x.shape[0]
+    _need(x, "x", torch.float32); _need(gain_first, "gain_first", torch.float32)
+    _need(w_head, "w_head", torch.bfloat16); _need(logits, "logits", torch.float32)
+    _need(token_pos, "token_pos", torch.int32); _need(token_seq, "token_seq", torch.int32)
+    _need(block_table, "block_table", torch.int32, contiguous=False)
+    if len(layers) > DECODE_LAYERS_MAX or rows > DECODE_LAYERS_MAX_ROWS:
+        raise KernelError("decode_layers: more layers or rows than it takes")
+    if w_head.shape[1] != H or logits.shape != (rows, w_head.shape[0]) or gain_first.numel() != H:
+        raise KernelError("decode_layers: shapes disagree")
+    if token_pos.numel() != rows or token_seq.numel() != rows or block_table.shape[0] != rows or block_table.stride(1) != 1:
+        raise KernelError("decode_layers: the step's description has another number of rows")
+    F, KO = layers[0][3].shape[1], n_q * head_dim
+    p = _DecodeLayers()
+    for q, (w_qkv, w_o, w_gu, w_down, gain_ff, gain_next, k, v) in zip(p.layer, layers):
+        for t, shape in ((w_qkv, (KO + 2 * n_kv * head_dim, H)), (w_o, (H, KO)), (w_gu, (2 * F, H)), (w_down, (H, F))):
+            _need(t, "a layer's matrix", torch.bfloat16)
+            if tuple(t.shape) != shape:
+                raise KernelError("decode_layers: a layer's matrix has another shape")
+        for t in (gain_ff, gain_next):
+            _need(t, "a layer's gain", torch.float32)
+            if t.numel() != H:
+                raise KernelError("decode_layers: a layer's gain has another size")
+        for t in (k, v):
+            _need(t, "a layer's cache", torch.bfloat16)
+            if tuple(t.shape[1:]) != (n_kv, 64, head_dim):
+                raise KernelError("decode_layers: a layer's cache has another shape")
+        q.w_qkv, q.w_o, q.w_gu, q.w_down = w_qkv.data_ptr(), w_o.data_ptr(), w_gu.data_ptr(), w_down.data_ptr()
+        q.gain_ff, q.gain_next, q.k, q.v = gain_ff.data_ptr(), gain_next.data_ptr(), k.data_ptr(), v.data_ptr()
+    blocks, dev = sm_count(x.device), x.device
+    bf = lambda n: torch.empty(rows * n, dtype=torch.bfloat16, device=dev)          # noqa: E731
+    f32 = lambda n: torch.empty(n, dtype=torch.float32, device=dev)                 # noqa: E731
+    xb, qb, ob, ab = bf(H), bf(KO), bf(KO), bf(F)
+    ss, part_o, part_ml = f32(2 * blocks * 16), f32(2 * blocks * 8 * head_dim), f32(2 * blocks * 8 * 2)
+    counters = torch.zeros(1 + rows * n_kv, dtype=torch.int32, device=dev)          # (a step begins with zeros whatever came before)
+    p.x, p.gain_first, p.w_head, p.logits = x.data_ptr(), gain_first.data_ptr(), w_head.data_ptr(), logits.data_ptr()
+    p.xb, p.qb, p.ob, p.ab = xb.data_ptr(), qb.data_ptr(), ob.data_ptr(), ab.data_ptr()
+    p.ss, p.part_o, p.part_ml, p.counters = ss.data_ptr(), part_o.data_ptr(), part_ml.data_ptr(), counters.data_ptr()
+    if rope is not None:
+        _need(rope, "rope", torch.float32)
+        if rope.shape[0] != rows:
+            raise KernelError("decode_layers: the rotation table has another number of rows")
+        p.rope, p.n_pairs = rope.data_ptr(), rope.shape[1]
+    p.pos, p.seq, p.block_table = token_pos.data_ptr(), token_seq.data_ptr(), block_table.data_ptr()
+    p.status = status_word().data_ptr()
+    p.bt_stride, p.n_layers, p.M, p.H, p.F = block_table.stride(0), len(layers), rows, H, F
+    p.n_q, p.n_kv, p.D, p.window, p.vocab = n_q, n_kv, head_dim, int(window), w_head.shape[0]
+    p.eps, p.scale = float(eps), float(scale)
+    f = _fn("decode_layers", "stratum_decode_layers", [c_void_p, c_int, c_void_p])
+    _check(f(ctypes.addressof(p), blocks, _stream()), "decode_layers")
 
 
 # ------------------------------------------------------------------ sampling
