@@ -289,10 +289,20 @@ __device__ __forceinline__ void draw_from_candidates(const float* cand_v, const 
   else draw_from<16>(cand_v, cand_i, cand_e, n_cand, tp, u, r, ids, values);
 }
 
+// The rows' numbers as part of the launch itself, one temperature, top_k and top_p for all of them (rows > 0): a caller that
+// draws on the host then copies nothing to the device and does not wait for it (24 rows of 128,256 logits, a pick among
+// others: 31 us; with a copy of four numbers a row, which waited for the picks before, 58).
+#define SAMPLE_GIVEN_MAX 256
+struct SampleGiven {
+  int rows, top_k;
+  float temperature, top_p;
+  float uniform[SAMPLE_GIVEN_MAX];
+};
+
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_kernel(const float* __restrict__ logits, int ld, int vocab, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ uniform,
-              int* __restrict__ ids, float* __restrict__ values, const int* redo) {
+              int* __restrict__ ids, float* __restrict__ values, const int* redo, const __grid_constant__ SampleGiven given) {
   __shared__ MaxIdx mi_scratch[33];
   __shared__ float f_scratch[33];
   __shared__ unsigned u_scratch[33];
@@ -308,16 +318,16 @@ sample_kernel(const float* __restrict__ logits, int ld, int vocab, const float* 
   const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (redo && !__ldcg(redo + r)) return;       // behind the 32-block kernel: only the rows it marked
   const float* row = logits + (size_t)r * ld;
-  const float temp = temperature[r];
+  const float temp = given.rows ? given.temperature : temperature[r];
   const MaxIdx best = row_argmax(row, vocab, mi_scratch);
   if (!(temp > 0.f)) {
     if (tid == 0) { ids[r] = best.i; if (values) values[r] = best.v; }
     return;
   }
   const float inv_t = 1.0f / temp;
-  const float u = uniform[r];
-  int k = top_k[r];
-  const float tp = top_p[r];
+  const float u = given.rows ? given.uniform[r] : uniform[r];
+  int k = given.rows ? given.top_k : top_k[r];
+  const float tp = given.rows ? given.top_p : top_p[r];
   const bool filtered = (k > 0) || (tp < 1.0f);
 
   if (!filtered) {
@@ -664,7 +674,7 @@ __global__ void __launch_bounds__(SS_THREADS)
 sample_split_kernel(const float* __restrict__ logits, int ld, int vocab, const float* __restrict__ temperature,
                     const int* __restrict__ top_k, const float* __restrict__ top_p,
                     const float* __restrict__ uniform, int* __restrict__ ids, float* __restrict__ values,
-                    const SsScratch Q) {
+                    const SsScratch Q, const __grid_constant__ SampleGiven given) {
   extern __shared__ __align__(16) float lv[];      // the stretch's logits; in the last block, the lists: values, ids
   __shared__ MaxIdx mi_scratch[33];
   __shared__ float f_scratch[SS_THREADS + 2];
@@ -685,11 +695,11 @@ sample_split_kernel(const float* __restrict__ logits, int ld, int vocab, const f
   pdl_wait();
   const int r = blockIdx.x, sp = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float* row = logits + (size_t)r * ld;
-  const float temp = temperature[r];
+  const float temp = given.rows ? given.temperature : temperature[r];
   const bool sampled = temp > 0.f;
   const float inv_t = sampled ? 1.0f / temp : 0.f;
-  int k = top_k[r];
-  const float tp = top_p[r];
+  int k = given.rows ? given.top_k : top_k[r];
+  const float tp = given.rows ? given.top_p : top_p[r];
   const bool filtered = sampled && ((k > 0) || (tp < 1.0f));
   if (k <= 0 || k > SAMPLE_CAND_MAX) k = SAMPLE_CAND_MAX;
   if (k > vocab) k = vocab;
@@ -771,7 +781,7 @@ sample_split_kernel(const float* __restrict__ logits, int ld, int vocab, const f
     if (tid == 0) { ids[r] = best.i; if (values) values[r] = best.v; }
     return;
   }
-  const float u = uniform[r];
+  const float u = given.rows ? given.uniform[r] : uniform[r];
 
   if (!filtered) {
     // thread t: sub-stretch t % 8 of stretch t / 8; their sums brought to the row's maximum, added in id order
@@ -922,28 +932,50 @@ sample_split_kernel(const float* __restrict__ logits, int ld, int vocab, const f
   draw_from_candidates(cand_v, cand_i, cand_e, n_cand, tp, u, r, ids, values);
 }
 
+static int sample_rows(const float* logits, int ld, int n_rows, int vocab, const float* temperature, const int* top_k,
+                       const float* top_p, const float* uniform, int* ids, float* values, const SsScratch& Q,
+                       const SampleGiven& given, cudaStream_t stream) {
+  if (n_rows <= 0) return 0;
+  if (vocab < 1) return STRATUM_ERR_SHAPE;
+  if (Q.part_v && Q.part_i && Q.part_e && Q.part_key && Q.cand_v && Q.cand_i && Q.counters && Q.redo && vocab >= 8192 &&
+      vocab <= SS_SPLITS * SS_CHUNK_MAX) {
+    const size_t chunk_bytes = (size_t)((vocab + SS_SPLITS - 1) / SS_SPLITS) * sizeof(float);
+    const size_t list_bytes = (size_t)SS_LIST_MAX * sizeof(uint32_t);
+    const size_t smem = chunk_bytes > list_bytes ? chunk_bytes : list_bytes;
+    int st = launch_pdl(sample_split_kernel, dim3(n_rows, SS_SPLITS), SS_THREADS, smem, stream, logits, ld, vocab,
+                        temperature, top_k, top_p, uniform, ids, values, Q, given);
+    if (st != 0) return st;
+    return launch_pdl(sample_kernel, n_rows, SAMPLE_THREADS, 0, stream, logits, ld, vocab, temperature, top_k, top_p,
+                      uniform, ids, values, (const int*)Q.redo, given);
+  }
+  return launch_pdl(sample_kernel, n_rows, SAMPLE_THREADS, 0, stream, logits, ld, vocab, temperature, top_k, top_p,
+                    uniform, ids, values, (const int*)nullptr, given);
+}
+
 // scratch (optional, all eight or none): see SsScratch; with it, rows of 8,192 to 262,144 logits are cut over 32
 // blocks each, and the one-block kernel runs behind for the rows that were marked.
 STRATUM_EXPORT int stratum_sample(const float* logits, int ld, int n_rows, int vocab, const float* temperature,
                                   const int* top_k, const float* top_p, const float* uniform, int* ids,
                                   float* values, float* part_v, int* part_i, float* part_e, unsigned* part_key,
                                   float* cand_v, int* cand_i, unsigned* counters, int* redo, cudaStream_t stream) {
-  if (n_rows <= 0) return 0;
-  if (vocab < 1) return STRATUM_ERR_SHAPE;
-  if (part_v && part_i && part_e && part_key && cand_v && cand_i && counters && redo && vocab >= 8192 &&
-      vocab <= SS_SPLITS * SS_CHUNK_MAX) {
-    const size_t chunk_bytes = (size_t)((vocab + SS_SPLITS - 1) / SS_SPLITS) * sizeof(float);
-    const size_t list_bytes = (size_t)SS_LIST_MAX * sizeof(uint32_t);
-    const size_t smem = chunk_bytes > list_bytes ? chunk_bytes : list_bytes;
-    SsScratch Q{part_v, part_i, part_e, part_key, cand_v, cand_i, counters, redo};
-    int st = launch_pdl(sample_split_kernel, dim3(n_rows, SS_SPLITS), SS_THREADS, smem, stream, logits, ld, vocab,
-                        temperature, top_k, top_p, uniform, ids, values, Q);
-    if (st != 0) return st;
-    return launch_pdl(sample_kernel, n_rows, SAMPLE_THREADS, 0, stream, logits, ld, vocab, temperature, top_k, top_p,
-                      uniform, ids, values, (const int*)redo);
-  }
-  return launch_pdl(sample_kernel, n_rows, SAMPLE_THREADS, 0, stream, logits, ld, vocab, temperature, top_k, top_p,
-                    uniform, ids, values, (const int*)nullptr);
+  static const SampleGiven none = {};
+  return sample_rows(logits, ld, n_rows, vocab, temperature, top_k, top_p, uniform, ids, values,
+                     SsScratch{part_v, part_i, part_e, part_key, cand_v, cand_i, counters, redo}, none, stream);
+}
+
+// The same for up to 256 rows of one temperature, top_k and top_p, with the uniforms in host memory.
+STRATUM_EXPORT int stratum_sample_given(const float* logits, int ld, int n_rows, int vocab, float temperature, int top_k,
+                                        float top_p, const float* host_uniforms, int* ids, float* values, float* part_v,
+                                        int* part_i, float* part_e, unsigned* part_key, float* cand_v, int* cand_i,
+                                        unsigned* counters, int* redo, cudaStream_t stream) {
+  if (n_rows > SAMPLE_GIVEN_MAX) return STRATUM_ERR_LIMIT;
+  if (n_rows > 0 && !host_uniforms) return STRATUM_ERR_SHAPE;
+  SampleGiven given = {};
+  given.rows = n_rows;
+  given.temperature = temperature; given.top_k = top_k; given.top_p = top_p;
+  for (int i = 0; i < n_rows; i++) given.uniform[i] = host_uniforms[i];
+  return sample_rows(logits, ld, n_rows, vocab, nullptr, nullptr, nullptr, nullptr, ids, values,
+                     SsScratch{part_v, part_i, part_e, part_key, cand_v, cand_i, counters, redo}, given, stream);
 }
 
 // ---------------------------------------------------------------- feeding picked ids back on the device

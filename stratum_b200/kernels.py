@@ -1841,3 +1841,23 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
              _ptr(top_p), _ptr(uniform), _ptr(ids), _ptr(values), *[_ptr(t) for t in scratch], _stream()), "sample")
     if not one_block_per_row and 8192 <= logits.shape[1] <= 262144:
         count_launches(1)                      # the one-block kernel behind, for marked rows
+
+
+SAMPLE_GIVEN_MAX = 256
+
+
+def sample_given(logits: torch.Tensor, temperature: float, top_k: int, top_p: float, uniforms, ids: torch.Tensor,
+                 values: Optional[torch.Tensor] = None, one_block_per_row: bool = False) -> None:
+    """`sample` for up to 256 rows of one temperature, top_k and top_p, with a host list of uniforms: the numbers travel with
+    the launch, nothing is copied to the device."""
+    _need(logits, "logits", torch.float32, contiguous=False); _need(ids, "ids", torch.int32)
+    n = logits.shape[0]
+    if len(uniforms) != n or n > SAMPLE_GIVEN_MAX:
+        raise KernelError(f"sample_given: one uniform per row, at most {SAMPLE_GIVEN_MAX}")
+    scratch = (None,) * 8 if one_block_per_row else _sample_scratch_for(n, logits.device)
+    f = _fn("sampling", "stratum_sample_given",
+            [c_void_p, c_int, c_int, c_int, c_float, c_int, c_float, c_void_p, c_void_p, c_void_p] + [c_void_p] * 9)
+    _check(f(logits.data_ptr(), logits.stride(0), n, logits.shape[1], temperature, top_k, top_p, (c_float * n)(*uniforms),
+             ids.data_ptr(), _ptr(values), *[_ptr(t) for t in scratch], _stream()), "sample_given")
+    if not one_block_per_row and 8192 <= logits.shape[1] <= 262144:
+        count_launches(1)                      # the one-block kernel behind, for marked rows

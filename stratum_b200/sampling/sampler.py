@@ -35,13 +35,19 @@ class Sampler:
             return ids, values
         if streams is None or len(streams) != n:
             raise ValueError("sampling needs one random stream per row")
+        many_filtered = n > K.sample_split_rows(logits.shape[1]) and (params.top_k > 0 or params.top_p < 1.0)
+        # the numbers as arguments of the launch: a copy from host memory waits for the device.  (A capture would keep them:
+        # there the copy refuses, as it does for more rows.)
+        if n <= K.SAMPLE_GIVEN_MAX and not torch.cuda.is_current_stream_capturing():
+            K.sample_given(logits, params.temperature, int(np.int32(params.top_k)), params.top_p,
+                           [s.uniform() for s in streams], ids, values, one_block_per_row=many_filtered)
+            return ids, values
         host = np.empty((4, n), dtype=np.float32)
         host[0, :] = params.temperature
         host[1, :] = np.array([params.top_k], dtype=np.int32).view(np.float32)[0]
         host[2, :] = params.top_p
         host[3, :] = [s.uniform() for s in streams]
         dev = torch.from_numpy(host).to(self.device)
-        many_filtered = n > K.sample_split_rows(logits.shape[1]) and (params.top_k > 0 or params.top_p < 1.0)
         K.sample(logits, dev[0], dev[1].view(torch.int32), dev[2], dev[3], ids, values,
                  one_block_per_row=many_filtered)
         return ids, values

@@ -202,3 +202,27 @@ def test_filters_pass_over_the_lowest_nan(vocab, k, top_p):
                      _dev([top_p] * 4, torch.float32), u, ids, vals, one_block_per_row=one_block)
             got.append((ids.tolist(), vals.tolist()))
         assert got[0] == got[1]
+
+
+@pytest.mark.parametrize("vocab", [5000, 50001])
+@pytest.mark.parametrize("n,temp,top_k,top_p", [(1, 0.0, 0, 1.0), (1, 0.7, 0, 1.0), (24, 0.8, 50, 0.95), (256, 1.1, 0, 0.9)])
+def test_numbers_given_with_the_launch(vocab, n, temp, top_k, top_p):
+    """The numbers as arguments pick what the numbers in device memory pick, bit for bit."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(n + vocab)
+    L = _dev(rng.standard_normal((n, vocab)) * 2.0, torch.float32)
+    us = [float(np.float32(u)) for u in rng.random(n)]
+    out = []
+    for given in (False, True):
+        ids = torch.empty(n, dtype=torch.int32, device="cuda")
+        vals = torch.empty(n, dtype=torch.float32, device="cuda")
+        one = n > K.sample_split_rows(vocab)
+        if given:
+            K.sample_given(L, temp, top_k, top_p, us, ids, vals, one_block_per_row=one)
+        else:
+            K.sample(L, _dev([temp] * n, torch.float32), _dev([top_k] * n, torch.int32), _dev([top_p] * n, torch.float32),
+                     _dev(us, torch.float32), ids, vals, one_block_per_row=one)
+        out.append((ids.tolist(), vals.tolist()))
+    assert out[0] == out[1]
+    with pytest.raises(K.KernelError):
+        K.sample_given(L, temp, top_k, top_p, us + [0.5], ids, vals)
