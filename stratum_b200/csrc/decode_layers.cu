@@ -26,7 +26,8 @@
 // the threads that add to it, in float32.
 //
 // Attention.  The pages of all (sequence, kv head) pairs form one list, cut evenly over the blocks (pairs of few pages are not
-// cut); four warps take 16 keys of a page each, two pages at a time; scores and values as in attention_mma.cu (keys along M).
+// cut: a row's bits then do not depend on its batch); four warps take 16 keys of a page each, two pages at a time; scores and
+// values as in attention_mma.cu (keys along M).
 // A pair seen by several blocks is merged by whichever of them comes last, in the order of its keys.  The new token's key and
 // value, which another block may have written a phase ago, do not come through the ring: one warp takes them from L2.
 #include "common.cuh"
@@ -371,7 +372,7 @@ __device__ __forceinline__ void dl_attention(const DlParams& P, DlSmem& S, const
     for (int c = 0; c < CH; c++)
       qv[c] = g < gs ? ld_fresh(reinterpret_cast<const uint4*>(P.qb + ((size_t)b * P.n_q + kvh * gs + g) * HD + 32 * c + 8 * t)) : zero4;
     // the new key comes behind its pair's last page, as a block of 16 keys with one key; by a warp that has no part in that page
-    const bool has_new = end == s1 && warp == ((((s1 - 1 - p0) & 1) ^ 1) << 2);
+    const bool has_new = end == s1 && warp == ((n & 1) << 2);
     uint4 nk[CH], nv[CH];
     if (has_new) {
       const int page = P.block_table[(size_t)P.seq[b] * P.bt_stride + pos / DL_PAGE];
@@ -391,7 +392,7 @@ __device__ __forceinline__ void dl_attention(const DlParams& P, DlSmem& S, const
       uint32_t keys = 0;
       if (!fresh) {
         if (CH == 4 || (i & 1) == 0) held = W.ready();
-        mine = (warp >> 2) == (i & 1);
+        mine = (warp >> 2) == ((at - s0) & 1);           // (by the pair's pages: the same sums in any batch)
         keys = held + (CH == 4 ? 0 : (i & 1) * 2 * BYTES) + (16 * (warp & 3) + g) * PITCH + t * 16;
       } else {
         mine = has_new;

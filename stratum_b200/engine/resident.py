@@ -2,7 +2,8 @@
 
 A model whose every layer is the plain pre-norm decoder layer (RMSNorm, grouped-query attention without biases or head
 norms, RMSNorm, SwiGLU) and whose head is a plain matrix can take a step of a few rows, one new token each, in one launch
-for all layers and the head.  Everything else, and every step this does not take, runs part by part.
+for all layers and the head.  Captured decode steps run so (engine/graphs.py); everything else, and every step this does not
+take, runs part by part: launched from the host one after the other, the parts' kernels are the reference for it.
 """
 from __future__ import annotations
 
@@ -62,8 +63,8 @@ class ResidentSteps:
         return cls(model) if ok else None
 
     def takes(self, step) -> bool:
-        if not (step.all_single and 0 < step.n_tokens <= K.DECODE_LAYERS_MAX_ROWS and step.host
-                and step.host.get("want_all") and len(step.block_tables) == 1):
+        if not (step.resident and step.all_single and 0 < step.n_tokens <= K.DECODE_LAYERS_MAX_ROWS
+                and len(step.block_tables) == 1):
             return False
         width = next(iter(step.block_tables.values())).stride(0)
         return K.decode_layers_takes(step.n_tokens, self.att.n_kv_heads, width, self.model.runtime.device)

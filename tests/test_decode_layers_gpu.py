@@ -1,0 +1,122 @@
+"""Decode steps through the resident kernel (csrc/decode_layers.cu): against the plain oracle where its tiles, pages, pairs and
+rows end, against the part-by-part path for what the oracle has no word for, and which steps it leaves alone."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import assert_close, load_plain, make_model_dir, plain_logits, rand_tokens
+
+pytestmark = pytest.mark.gpu
+
+BASE = {
+    "architectures": ["LlamaForCausalLM"], "model_type": "llama", "num_hidden_layers": 2, "hidden_size": 512,
+    "intermediate_size": 1024, "num_attention_heads": 8, "num_key_value_heads": 2, "head_dim": 64, "vocab_size": 600,
+    "rms_norm_eps": 1e-5, "rope_theta": 10000.0, "max_position_embeddings": 4096, "tie_word_embeddings": False,
+    "attention_bias": False, "mlp_bias": False, "hidden_act": "silu",
+}
+MODELS = {
+    "heads of 64": BASE,
+    # one kv head for eight heads, k that ends inside a chunk of 1,024, shares of one and of two tiles
+    "heads of 128, one kv head": dict(BASE, hidden_size=1152, intermediate_size=1408, num_key_value_heads=1, head_dim=128,
+                                      vocab_size=2400, tie_word_embeddings=True),
+    "a kv head per head": dict(BASE, hidden_size=1024, intermediate_size=2688, num_key_value_heads=8, head_dim=128,
+                               num_hidden_layers=1),
+}
+# lengths in front of the decoded tokens: page and block edges, pairs that are cut over blocks, one to sixteen rows
+BATCHES = [(30,), (1,), (64, 63, 65), (16, 17, 128, 15, 1, 2, 127, 300), (700, 5), (1300,),
+           (9, 64, 200, 31, 32, 33, 70, 129, 4), tuple(range(3, 51, 3))]
+
+
+@pytest.fixture(scope="module", params=sorted(MODELS))
+def model(request, tmp_path_factory):
+    path = make_model_dir(str(tmp_path_factory.mktemp("resident")), MODELS[request.param], seed=3, dtype="bfloat16")
+    cfg, w = load_plain(path)
+    return path, cfg, w
+
+
+def _stratum(path, max_tokens):
+    from stratum_b200 import Stratum
+    return Stratum(path, dtype="bfloat16", max_tokens=max_tokens, max_seqs=20)
+
+
+def _fill(llm, prompts):
+    from stratum_b200 import StepEntry
+    slots = [llm.acquire() for _ in prompts]
+    for s, p in zip(slots, prompts):
+        llm.engine.step([StepEntry(s, p, [])])
+    return slots
+
+
+def _decode(llm, slots, tokens):
+    return llm.decode_step(slots, tokens, with_logits=True)[2].cpu().numpy()
+
+
+@pytest.mark.parametrize("lens", BATCHES, ids=lambda b: f"{len(b)} rows, {max(b)}")
+def test_against_the_oracle(model, lens):
+    path, cfg, w = model
+    llm = _stratum(path, sum(n + 128 for n in lens))
+    rng = np.random.default_rng(len(lens))
+    steps = 3
+    toks = [rand_tokens(rng, n + steps, cfg["vocab_size"]) for n in lens]
+    slots = _fill(llm, [t[:n] for t, n in zip(toks, lens)])
+    got = [_decode(llm, slots, [t[n + i] for t, n in zip(toks, lens)]) for i in range(steps)]
+    assert llm.model.resident_steps() is not None
+    for j, (t, n) in enumerate(zip(toks, lens)):
+        ref = plain_logits(cfg, w, t)
+        assert_close(np.stack([g[j] for g in got]), ref[n:], "bfloat16", f"row {j} of {n} tokens")
+
+
+def test_window_and_rows_alone(model, monkeypatch):
+    """A sliding window (the same attribute both paths read) against the part-by-part path, and a row's bits in another batch."""
+    path, cfg, _ = model
+    lens = [200, 64, 10, 130]
+    rng = np.random.default_rng(1)
+    toks = [rand_tokens(rng, n + 1, cfg["vocab_size"]) for n in lens]
+    out = []
+    for on in ("1", "0"):
+        monkeypatch.setenv("STRATUM_RESIDENT_STEPS", on)
+        llm = _stratum(path, 2048)
+        slots = _fill(llm, [t[:-1] for t in toks])
+        for layer in llm.model.layers:
+            layer.part("mixer").window = 70
+        out.append(_decode(llm, slots, [t[-1] for t in toks]))
+        assert (llm.model.resident_steps() is not None) == (on == "1")
+    assert_close(out[0], out[1], "bfloat16", "window")
+    monkeypatch.setenv("STRATUM_RESIDENT_STEPS", "1")
+    llm = _stratum(path, 2048)
+    alone = []
+    for t in toks:
+        slots = _fill(llm, [t[:-1]])
+        alone.append(_decode(llm, slots, [t[-1]])[0])
+        llm.release(slots[0])
+    slots = _fill(llm, [t[:-1] for t in toks])
+    both = _decode(llm, slots, [t[-1] for t in toks])
+    # (pairs of up to eight pages are never cut, so the order of every sum is the same)
+    assert np.array_equal(both, np.stack(alone))
+
+
+def test_steps_it_leaves_alone(model):
+    """More rows than sixteen, and steps launched from the host, run part by part."""
+    from stratum_b200 import StepEntry
+    path, cfg, w = model
+    llm = _stratum(path, 4096)
+    rng = np.random.default_rng(2)
+    toks = [rand_tokens(rng, 21, cfg["vocab_size"]) for _ in range(17)]
+    slots = _fill(llm, [t[:19] for t in toks])
+    got = llm.engine.step([StepEntry(s, [t[19]], [0]) for s, t in zip(slots, toks)]).cpu().numpy()
+    ref = [plain_logits(cfg, w, t) for t in toks[:3]]
+    assert_close(got[:3], np.stack([r[19] for r in ref]), "bfloat16", "launched from the host")
+    got = _decode(llm, slots, [t[20] for t in toks])
+    assert_close(got[:3], np.stack([r[20] for r in ref]), "bfloat16", "seventeen rows")
+
+
+def test_sizes_it_refuses():
+    """The launcher refuses what its shares and registers do not hold; the plan asks the same questions."""
+    from stratum_b200 import kernels as K
+    dev = torch.device("cuda")
+    ok = dict(H=2048, F=8192, vocab=128256, n_q=32, n_kv=8, head_dim=64, device=dev)
+    assert K.decode_layers_sizes_ok(**ok)
+    for bad in (dict(H=8192), dict(H=2080), dict(F=8200), dict(head_dim=80), dict(n_q=72, n_kv=8), dict(vocab=128257),
+                dict(H=128), dict(n_q=128)):
+        assert not K.decode_layers_sizes_ok(**dict(ok, **bad)), bad
+    assert K.decode_layers_takes(16, 8, 1024, dev) and not K.decode_layers_takes(16, 32, 1024, dev)
