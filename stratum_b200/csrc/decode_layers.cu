@@ -544,18 +544,19 @@ __global__ void __launch_bounds__(DL_THREADS, 1)
 decode_layers_kernel(const __grid_constant__ DlParams P) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   DlSmem& S = *reinterpret_cast<DlSmem*>(smem_raw);
+  constexpr int HD = 32 * CH;
   constexpr int TG = 4 / MT;                    // tiles whose partial sums meet at a time
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = gridDim.x;
 
   if (tid < PH_COUNT) {
-    const int NQ = (P.n_q + 2 * P.n_kv) * P.D;
+    const int NQ = (P.n_q + 2 * P.n_kv) * HD;
     const int N = tid == PH_QKV ? NQ : tid == PH_O ? P.H : tid == PH_GU ? 2 * P.F : tid == PH_DOWN ? P.H : P.vocab;
     DlShare s;
     s.row0 = 2 * (int)((long long)blockIdx.x * (N / 2) / G);
     s.rows = 2 * (int)((long long)(blockIdx.x + 1) * (N / 2) / G) - s.row0;
     s.tiles = (s.rows + 15) / 16;
-    s.K = tid == PH_O ? P.n_q * P.D : tid == PH_DOWN ? P.F : P.H;
+    s.K = tid == PH_O ? P.n_q * HD : tid == PH_DOWN ? P.F : P.H;
     s.chunks = (s.K + DL_CHUNK - 1) / DL_CHUNK;
     S.share[tid] = s;
   }
@@ -662,23 +663,23 @@ decode_layers_kernel(const __grid_constant__ DlParams P) {
     ok = wide(PH_QKV, P.xb, ss_of[0],
               [&](int t0) {
                 const int n = S.share[PH_QKV].row0 + (t0 + etl) * 16 + 2 * ep;
-                const int d = (n % P.D) >> 1;
+                const int d = (n % HD) >> 1;
                 turn = make_float2(1.f, 0.f);
-                if (m_ok && n < (P.n_q + P.n_kv) * P.D && d < P.n_pairs) turn = P.rope[em * P.n_pairs + d];
+                if (m_ok && n < (P.n_q + P.n_kv) * HD && d < P.n_pairs) turn = P.rope[em * P.n_pairs + d];
               },
               [&](bool on, int n, float2 v) {
                 if (!on) return;
                 const float inv = S.inv[em];
                 v.x *= inv; v.y *= inv;
                 const __nv_bfloat162 y = __floats2bfloat162_rn(v.x * turn.x - v.y * turn.y, v.x * turn.y + v.y * turn.x);
-                const int head = n / P.D, d = n % P.D;
+                const int head = n / HD, d = n % HD;
                 if (head < P.n_q) {
-                  *reinterpret_cast<__nv_bfloat162*>(P.qb + (size_t)em * P.n_q * P.D + n) = y;
+                  *reinterpret_cast<__nv_bfloat162*>(P.qb + (size_t)em * P.n_q * HD + n) = y;
                 } else if (my_seq >= 0) {
                   const int h = head - P.n_q;
                   bf16* c = h < P.n_kv ? L.k : L.v;
                   const int kvh = h < P.n_kv ? h : h - P.n_kv;
-                  *reinterpret_cast<__nv_bfloat162*>(c + (((size_t)my_page * P.n_kv + kvh) * DL_PAGE + my_pos % DL_PAGE) * P.D + d) = y;
+                  *reinterpret_cast<__nv_bfloat162*>(c + (((size_t)my_page * P.n_kv + kvh) * DL_PAGE + my_pos % DL_PAGE) * HD + d) = y;
                 }
               });
     if (!ok) break;

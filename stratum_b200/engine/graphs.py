@@ -115,9 +115,7 @@ class DecodeGraphs:
     # ------------------------------------------------------------------ building blocks
     def _forward_and_pick(self, c: _Captured) -> None:
         d = c.desc
-        step = d.batch(c.width * PAGE_TOKENS)
-        step.resident = True
-        logits = self.engine.model.forward(step, self.engine.cache)
+        logits = self.engine.model.forward(d.batch(c.width * PAGE_TOKENS), self.engine.cache)
         f32 = lambda name: d.field(name).view(torch.float32)                     # noqa: E731
         if c.greedy:
             K.argmax(logits, c.out_ids, c.out_vals)

@@ -80,7 +80,7 @@ class Model:
                          if spec.position is not None else None)
         self.schedule = spec.schedule
         self.hidden, self.vocab = spec.hidden, spec.vocab
-        self._resident: Optional[ResidentSteps] = None      # made with the first captured decode step (it needs the device)
+        self._resident: Optional[ResidentSteps] = None      # made with the first step of single tokens (it needs the device)
         self._resident_asked = False
 
     # ------------------------------------------------------------------ description
@@ -144,7 +144,7 @@ class Model:
             self.position.add_to_embedding(x, step)
             if self.spec.keep_embedded:
                 self.position.add_to_embedding(step.embedded, step)
-        if step.resident:
+        if step.all_single:
             plan = self.resident_steps()
             if plan is not None and plan.takes(step):
                 return plan.run(x, step, cache)

@@ -2,8 +2,8 @@
 
 A model whose every layer is the plain pre-norm decoder layer (RMSNorm, grouped-query attention without biases or head
 norms, RMSNorm, SwiGLU) and whose head is a plain matrix can take a step of a few rows, one new token each, in one launch
-for all layers and the head.  Captured decode steps run so (engine/graphs.py); everything else, and every step this does not
-take, runs part by part: launched from the host one after the other, the parts' kernels are the reference for it.
+for all layers and the head, replayed or launched from the host alike (the same bits).  Everything else, and every step this
+does not take, runs part by part.
 """
 from __future__ import annotations
 
@@ -19,6 +19,13 @@ from ..parts.block import PreNormResidual
 from ..parts.embedding import LinearHead
 from ..parts.mlp import SwiGLU
 from ..parts.norm import RMSNorm
+
+
+# Models of fewer layers run part by part: the kernel's set-up (lists of pages, the ring's first filling, the head's tiles) is a
+# large share of so short a step.  A step in us, parts / kernel, behind 200 tokens with a vocabulary of 2,048, at one, two and
+# four layers: width 512, 8 rows 29 / 33, 47 / 49, 86 / 82; 1 row 36 / 33, 64 / 49, 117 / 82; width 4,096 (8B shape), 8 rows
+# 122 / 112, 218 / 194, 409 / 361.
+MIN_LAYERS = 4
 
 
 class ResidentSteps:
@@ -39,7 +46,7 @@ class ResidentSteps:
             return None
         if type(model.final_norm) is not RMSNorm or type(model.head) is not LinearHead or model.spec.keep_embedded:
             return None
-        if any(e.cache_of is not None for e in model.schedule) or len(model.schedule) > K.DECODE_LAYERS_MAX:
+        if any(e.cache_of is not None for e in model.schedule) or not MIN_LAYERS <= len(model.schedule) <= K.DECODE_LAYERS_MAX:
             return None
         eps, shapes = model.final_norm.eps, set()
         for e in model.schedule:
@@ -63,8 +70,8 @@ class ResidentSteps:
         return cls(model) if ok else None
 
     def takes(self, step) -> bool:
-        if not (step.resident and step.all_single and 0 < step.n_tokens <= K.DECODE_LAYERS_MAX_ROWS
-                and len(step.block_tables) == 1):
+        if not (step.all_single and 0 < step.n_tokens <= K.DECODE_LAYERS_MAX_ROWS and step.host
+                and step.host.get("want_all") and len(step.block_tables) == 1):
             return False
         width = next(iter(step.block_tables.values())).stride(0)
         return K.decode_layers_takes(step.n_tokens, self.att.n_kv_heads, width, self.model.runtime.device)

@@ -55,7 +55,6 @@ class StepBatch:
     fixed_qblocks: Optional[Dict[int, tuple]] = None   # a captured prompt step: its query blocks, padded lists
     sizes_seen: Optional[set] = None  # when set: the block sizes `query_blocks` was asked for are noted here
     kept: Dict[str, torch.Tensor] = field(default_factory=dict)   # rows a layer leaves for later layers of the same step
-    resident: bool = False            # a captured decode step, every row's logits wanted: one kernel may take all its layers
     embedded: Optional[torch.Tensor] = None   # float32 [T, hidden]: the embedded tokens, for models that re-read them
     _qblocks: Dict[int, tuple] = field(default_factory=dict)
     _rotation: Dict[object, torch.Tensor] = field(default_factory=dict)
@@ -131,6 +130,7 @@ class StepDescription:
         self.n_new: List[int] = []
         self.single = True
         self.before: Optional[List[int]] = None
+        self.want_all = False             # the wanted rows are all rows, in their order
 
     def write_membership(self, slots: Sequence[int], n_new: Sequence[int], wants: Optional[Sequence[Sequence[int]]]):
         """Who is in the step, with how many tokens each, whose logits are wanted and which pages they hold:
@@ -159,12 +159,14 @@ class StepDescription:
         slot[B:] = cache.max_seqs
         if wants is None:
             v["want"][:] = np.arange(self.n_want, dtype=np.int32)
+            self.want_all = self.n_want == self.n_tokens
         else:
             w = 0
             for i, ws in enumerate(wants):
                 for p in ws:
                     v["want"][w] = start[i] + int(p)
                     w += 1
+            self.want_all = pad == 0 and all(n == 1 for n in n_new) and all(len(ws) == 1 for ws in wants)
         if self.groups:
             tb = v["tables"].reshape(len(self.groups), self.n_seqs, self.width)
             tb.fill(-1)
@@ -271,7 +273,8 @@ class StepDescription:
                          token_seq=self.field("seq"), want_rows=self.field("want"), seq_slot=self.field("slot"),
                          seq_start=self.field("start"), seq_len=self.field("len"), block_tables=tables,
                          max_new=max(self.n_new, default=0), max_len=max_len, all_single=self.single,
-                         host={"n_new": list(self.n_new), "before": self.before}, fixed_qblocks=fixed)
+                         host={"n_new": list(self.n_new), "before": self.before, "want_all": self.want_all},
+                         fixed_qblocks=fixed)
 
 
 class Engine:

@@ -9,7 +9,7 @@ from helpers import assert_close, load_plain, make_model_dir, plain_logits, rand
 pytestmark = pytest.mark.gpu
 
 BASE = {
-    "architectures": ["LlamaForCausalLM"], "model_type": "llama", "num_hidden_layers": 2, "hidden_size": 512,
+    "architectures": ["LlamaForCausalLM"], "model_type": "llama", "num_hidden_layers": 4, "hidden_size": 512,
     "intermediate_size": 1024, "num_attention_heads": 8, "num_key_value_heads": 2, "head_dim": 64, "vocab_size": 600,
     "rms_norm_eps": 1e-5, "rope_theta": 10000.0, "max_position_embeddings": 4096, "tie_word_embeddings": False,
     "attention_bias": False, "mlp_bias": False, "hidden_act": "silu",
@@ -19,8 +19,7 @@ MODELS = {
     # one kv head for eight heads, k that ends inside a chunk of 1,024, shares of one and of two tiles
     "heads of 128, one kv head": dict(BASE, hidden_size=1152, intermediate_size=1408, num_key_value_heads=1, head_dim=128,
                                       vocab_size=2400, tie_word_embeddings=True),
-    "a kv head per head": dict(BASE, hidden_size=1024, intermediate_size=2688, num_key_value_heads=8, head_dim=128,
-                               num_hidden_layers=1),
+    "a kv head per head": dict(BASE, hidden_size=1024, intermediate_size=2688, num_key_value_heads=8, head_dim=128),
 }
 # lengths in front of the decoded tokens: page and block edges, pairs that are cut over blocks, one to sixteen rows
 BATCHES = [(30,), (1,), (64, 63, 65), (16, 17, 128, 15, 1, 2, 127, 300), (700, 5), (1300,),
@@ -96,18 +95,26 @@ def test_window_and_rows_alone(model, monkeypatch):
 
 
 def test_steps_it_leaves_alone(model):
-    """More rows than sixteen, and steps launched from the host, run part by part."""
+    """Rows whose logits nobody wants, and more rows than sixteen, run part by part; a step launched from the host gives a
+    replayed one's bits."""
     from stratum_b200 import StepEntry
     path, cfg, w = model
     llm = _stratum(path, 4096)
     rng = np.random.default_rng(2)
-    toks = [rand_tokens(rng, 21, cfg["vocab_size"]) for _ in range(17)]
-    slots = _fill(llm, [t[:19] for t in toks])
-    got = llm.engine.step([StepEntry(s, [t[19]], [0]) for s, t in zip(slots, toks)]).cpu().numpy()
+    toks = [rand_tokens(rng, 22, cfg["vocab_size"]) for _ in range(17)]
     ref = [plain_logits(cfg, w, t) for t in toks[:3]]
-    assert_close(got[:3], np.stack([r[19] for r in ref]), "bfloat16", "launched from the host")
+    slots = _fill(llm, [t[:19] for t in toks])
+    got = llm.engine.step([StepEntry(s, [t[19]], [0] if i != 1 else []) for i, (s, t) in enumerate(zip(slots, toks[:3]))])
+    assert_close(got.cpu().numpy(), np.stack([ref[0][19], ref[2][19]]), "bfloat16", "wanted rows")
+    _decode(llm, slots[3:], [t[19] for t in toks[3:]])
     got = _decode(llm, slots, [t[20] for t in toks])
     assert_close(got[:3], np.stack([r[20] for r in ref]), "bfloat16", "seventeen rows")
+    for s in slots:
+        llm.release(s)
+    a, b = _fill(llm, [t[:19] for t in toks[:2]]), _fill(llm, [t[:19] for t in toks[:2]])
+    replayed = _decode(llm, a, [t[19] for t in toks[:2]])
+    launched = llm.engine.step([StepEntry(s, [t[19]], [0]) for s, t in zip(b, toks)]).cpu().numpy()
+    assert np.array_equal(replayed, launched)
 
 
 def test_sizes_it_refuses():
