@@ -147,7 +147,7 @@ class Model:
         if step.all_single:
             plan = self.resident_steps()
             if plan is not None and plan.takes(step):
-                return plan.run(x, step, cache)
+                return plan.run(self, x, step, cache)
         carry = None                  # rows a layer's last product prepared for the next layer's first norm
         for stop, entry in enumerate(self.schedule):
             layer = self.layers[entry.layer]

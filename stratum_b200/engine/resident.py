@@ -29,10 +29,10 @@ MIN_LAYERS = 4
 
 
 class ResidentSteps:
-    """The plan of one model: which of its steps the kernel takes, and how it is called."""
+    """The plan of one model: which of its steps the kernel takes, and how it is called.  (It does not hold the model, which
+    holds it: a model's weights go when the last reference to it goes.)"""
 
     def __init__(self, model):
-        self.model = model
         self.att = model.layers[model.schedule[0].layer].part("mixer")
         self.rot = self.att.position.rotary() if self.att.position is not None else None
 
@@ -74,11 +74,11 @@ class ResidentSteps:
                 and step.host.get("want_all") and len(step.block_tables) == 1):
             return False
         width = next(iter(step.block_tables.values())).stride(0)
-        return K.decode_layers_takes(step.n_tokens, self.att.n_kv_heads, width, self.model.runtime.device)
+        return K.decode_layers_takes(step.n_tokens, self.att.n_kv_heads, width, step.token_ids.device)
 
-    def run(self, x: torch.Tensor, step, cache) -> torch.Tensor:
+    def run(self, model, x: torch.Tensor, step, cache) -> torch.Tensor:
         """Float32 logits of all rows of a step that `takes` accepted; x: the embedded tokens."""
-        m, att = self.model, self.att
+        m, att = model, self.att
         gains = [m.layers[e.layer].part("mixer_norm").gain for e in m.schedule] + [m.final_norm.gain]
         layers, table = [], None
         for i, e in enumerate(m.schedule):

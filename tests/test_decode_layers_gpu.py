@@ -117,6 +117,23 @@ def test_steps_it_leaves_alone(model):
     assert np.array_equal(replayed, launched)
 
 
+def test_a_model_goes_with_its_last_reference(model):
+    """The plan holds nothing that holds the model: no collector is needed to give its weights back."""
+    import gc
+    import weakref
+    path, cfg, _ = model
+    llm = _stratum(path, 256)
+    _decode(llm, _fill(llm, [[1, 2, 3]]), [4])
+    assert llm.model.resident_steps() is not None
+    ref = weakref.ref(llm.model)
+    gc.disable()
+    try:
+        del llm
+        assert ref() is None
+    finally:
+        gc.enable()
+
+
 def test_sizes_it_refuses():
     """The launcher refuses what its shares and registers do not hold; the plan asks the same questions."""
     from stratum_b200 import kernels as K
