@@ -7,7 +7,6 @@ does not take, runs part by part.
 """
 from __future__ import annotations
 
-import os
 from typing import Optional
 
 import torch
@@ -41,8 +40,6 @@ class ResidentSteps:
         """The plan, or None where the model is not made of the parts the kernel knows, in sizes it takes."""
         rt = model.runtime
         if rt is None or rt.dtype != torch.bfloat16 or rt.device.type != "cuda" or PAGE_TOKENS != 64:
-            return None
-        if os.environ.get("STRATUM_RESIDENT_STEPS", "1") == "0":             # (measurements)
             return None
         if type(model.final_norm) is not RMSNorm or type(model.head) is not LinearHead or model.spec.keep_embedded:
             return None

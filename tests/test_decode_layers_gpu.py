@@ -65,23 +65,23 @@ def test_against_the_oracle(model, lens):
         assert_close(np.stack([g[j] for g in got]), ref[n:], "bfloat16", f"row {j} of {n} tokens")
 
 
-def test_window_and_rows_alone(model, monkeypatch):
+def test_window_and_rows_alone(model):
     """A sliding window (the same attribute both paths read) against the part-by-part path, and a row's bits in another batch."""
     path, cfg, _ = model
     lens = [200, 64, 10, 130]
     rng = np.random.default_rng(1)
     toks = [rand_tokens(rng, n + 1, cfg["vocab_size"]) for n in lens]
     out = []
-    for on in ("1", "0"):
-        monkeypatch.setenv("STRATUM_RESIDENT_STEPS", on)
+    for on in (True, False):
         llm = _stratum(path, 2048)
+        if not on:                                           # (this model runs part by part)
+            llm.model._resident, llm.model._resident_asked = None, True
         slots = _fill(llm, [t[:-1] for t in toks])
         for layer in llm.model.layers:
             layer.part("mixer").window = 70
         out.append(_decode(llm, slots, [t[-1] for t in toks]))
-        assert (llm.model.resident_steps() is not None) == (on == "1")
+        assert (llm.model.resident_steps() is not None) == on
     assert_close(out[0], out[1], "bfloat16", "window")
-    monkeypatch.setenv("STRATUM_RESIDENT_STEPS", "1")
     llm = _stratum(path, 2048)
     alone = []
     for t in toks:
