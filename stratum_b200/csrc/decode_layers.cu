@@ -59,7 +59,7 @@ struct DlLayer {
 struct DlParams {
   const float* x;                     // [M][H] embedded tokens
   const float* gain_first;
-  const bf16* w_head; float* logits;  // [vocab][H]; [M][vocab]
+  const bf16* w_head; float* logits;  // [vocab][H]; [M][vocab]  (vocab 0: a step that wants no logits)
   bf16 *xb, *qb, *ob, *ab;            // [M][H], [M][n_q D], [M][n_q D], [M][F]
   float *ss;                          // [2][blocks][16]
   float *part_o, *part_ml;            // [2 blocks][8][D], [2 blocks][8][2]
@@ -739,7 +739,7 @@ decode_layers_kernel(const __grid_constant__ DlParams P) {
     dl_arrive(P);
   }
   // ------------------------------------------------------------------ the head
-  if (ok)
+  if (ok && P.vocab > 0)
     wide(PH_HEAD, P.xb, ss_of[0], [&](int) {},
          [&](bool on, int n, float2 v) {
            if (!on) return;
@@ -782,11 +782,12 @@ STRATUM_EXPORT int stratum_decode_layers(const DlParams* p, int blocks, cudaStre
   if (P.H % 128 || P.F % 128 || KO % 128 || P.H > 4 * DL_CHUNK || KO > 4 * DL_CHUNK) return STRATUM_ERR_SHAPE;
   // two rows of every matrix for each block, two tiles of 16 of the stream at most
   if (P.H < 2 * blocks || 2 * P.F < 2 * blocks || (P.H / 2 + blocks - 1) / blocks > 16) return STRATUM_ERR_SHAPE;
-  if ((P.n_q + 2 * P.n_kv) * P.D < 2 * blocks || P.vocab % 2 || P.vocab < 2 * blocks) return STRATUM_ERR_SHAPE;
+  if ((P.n_q + 2 * P.n_kv) * P.D < 2 * blocks || P.vocab < 0 || P.vocab % 2 || (P.vocab && P.vocab < 2 * blocks)) return STRATUM_ERR_SHAPE;
   // a block's list of pages (the table's width bounds the sequences' lengths)
   if (P.bt_stride < 1 || (long long)P.M * P.n_kv * P.bt_stride > (long long)(DL_MAX_PAGES - 2 * DL_WHOLE - 1) * blocks)
     return STRATUM_ERR_LIMIT;
-  if (!P.x || !P.gain_first || !P.w_head || !P.logits || !P.pos || !P.seq || !P.block_table || (P.n_pairs && !P.rope))
+  if (P.vocab && (!P.w_head || !P.logits)) return STRATUM_ERR_SHAPE;
+  if (!P.x || !P.gain_first || !P.pos || !P.seq || !P.block_table || (P.n_pairs && !P.rope))
     return STRATUM_ERR_SHAPE;
   if (!P.status || !P.counters || !P.xb || !P.qb || !P.ob || !P.ab || !P.ss || !P.part_o || !P.part_ml) return STRATUM_ERR_SHAPE;
   if (((uintptr_t)P.x | (uintptr_t)P.gain_first | (uintptr_t)P.w_head | (uintptr_t)P.logits | (uintptr_t)P.xb | (uintptr_t)P.qb |

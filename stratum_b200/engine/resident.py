@@ -67,14 +67,15 @@ class ResidentSteps:
         return cls(model) if ok else None
 
     def takes(self, step) -> bool:
-        if not (step.all_single and 0 < step.n_tokens <= K.DECODE_LAYERS_MAX_ROWS and step.host
-                and step.host.get("want_all") and len(step.block_tables) == 1):
+        # (not by whose logits are wanted: what a step leaves in the cache does not depend on that)
+        if not (step.all_single and 0 < step.n_tokens <= K.DECODE_LAYERS_MAX_ROWS and step.n_seqs == step.n_tokens
+                and len(step.block_tables) == 1):
             return False
         width = next(iter(step.block_tables.values())).stride(0)
         return K.decode_layers_takes(step.n_tokens, self.att.n_kv_heads, width, step.token_ids.device)
 
     def run(self, model, x: torch.Tensor, step, cache) -> torch.Tensor:
-        """Float32 logits of all rows of a step that `takes` accepted; x: the embedded tokens."""
+        """Float32 logits of the wanted rows of a step that `takes` accepted; x: the embedded tokens."""
         m, att = model, self.att
         gains = [m.layers[e.layer].part("mixer_norm").gain for e in m.schedule] + [m.final_norm.gain]
         layers, table = [], None
@@ -85,8 +86,13 @@ class ResidentSteps:
             table = view.block_table
             layers.append((mix.qkv.weight, mix.o.weight, ff.gate_up.weight, ff.down.weight,
                            layer.part("feed_forward_norm").gain, gains[i + 1], view.k, view.v))
-        logits = torch.empty((step.n_tokens, m.vocab), dtype=torch.float32, device=x.device)
+        n_want = step.want_rows.numel()
+        logits = torch.empty((step.n_tokens, m.vocab), dtype=torch.float32, device=x.device) if n_want else None
         K.decode_layers(x, layers, gains[0], m.head.proj.weight, logits,
                         None if self.rot is None else step.rotation_table(self.rot), step.token_pos, step.token_seq, table,
                         att.n_heads, att.n_kv_heads, att.head_dim, att.window, att.scale, m.final_norm.eps)
-        return logits
+        if logits is None:
+            return torch.empty((0, m.vocab), dtype=torch.float32, device=x.device)
+        if step.host and step.host.get("want_all"):
+            return logits
+        return logits.index_select(0, step.want_rows)      # (the head's matrix is read once for all rows anyway)

@@ -1694,22 +1694,24 @@ def decode_layers_takes(rows: int, n_kv: int, table_width: int, device) -> bool:
     return rows * n_kv * table_width <= (1024 - 17) * sm_count(device)
 
 
-def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: torch.Tensor, logits: torch.Tensor,
+def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: torch.Tensor, logits: Optional[torch.Tensor],
                   rope: Optional[torch.Tensor], token_pos: torch.Tensor, token_seq: torch.Tensor,
                   block_table: torch.Tensor, n_q: int, n_kv: int, head_dim: int, window: int, scale: float,
                   eps: float) -> None:
     """All layers of a dense decoder and its head for a step of one new token per sequence, in one kernel that stays on
     every SM: x float32 [rows, H] (embedded), layers a list of (w_qkv, w_o, w_gate_up, w_down, gain of the feed-forward's
-    norm, gain of the norm behind the layer, k_cache, v_cache), logits float32 [rows, vocab].  Weights bfloat16, gate and up
+    norm, gain of the norm behind the layer, k_cache, v_cache), logits float32 [rows, vocab] (None: no head).  Weights bfloat16, gate and up
     rows alternating, rotated pairs neighbours; rope: (cos, sin) [rows, pairs, 2] or None.  At most 16 rows."""
     H, rows = x.shape[1], x.shape[0]
     _need(x, "x", torch.float32); _need(gain_first, "gain_first", torch.float32)
-    _need(w_head, "w_head", torch.bfloat16); _need(logits, "logits", torch.float32)
+    _need(w_head, "w_head", torch.bfloat16)
+    if logits is not None:
+        _need(logits, "logits", torch.float32)
     _need(token_pos, "token_pos", torch.int32); _need(token_seq, "token_seq", torch.int32)
     _need(block_table, "block_table", torch.int32, contiguous=False)
     if len(layers) > DECODE_LAYERS_MAX or rows > DECODE_LAYERS_MAX_ROWS:
         raise KernelError("decode_layers: more layers or rows than it takes")
-    if w_head.shape[1] != H or logits.shape != (rows, w_head.shape[0]) or gain_first.numel() != H:
+    if w_head.shape[1] != H or (logits is not None and logits.shape != (rows, w_head.shape[0])) or gain_first.numel() != H:
         raise KernelError("decode_layers: shapes disagree")
     if token_pos.numel() != rows or token_seq.numel() != rows or block_table.shape[0] != rows or block_table.stride(1) != 1:
         raise KernelError("decode_layers: the step's description has another number of rows")
@@ -1736,7 +1738,9 @@ def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: tor
     xb, qb, ob, ab = bf(H), bf(KO), bf(KO), bf(F)
     ss, part_o, part_ml = f32(2 * blocks * 16), f32(2 * blocks * 8 * head_dim), f32(2 * blocks * 8 * 2)
     counters = torch.zeros(1 + rows * n_kv, dtype=torch.int32, device=dev)          # (a step begins with zeros whatever came before)
-    p.x, p.gain_first, p.w_head, p.logits = x.data_ptr(), gain_first.data_ptr(), w_head.data_ptr(), logits.data_ptr()
+    p.x, p.gain_first = x.data_ptr(), gain_first.data_ptr()
+    if logits is not None:
+        p.w_head, p.logits, p.vocab = w_head.data_ptr(), logits.data_ptr(), w_head.shape[0]
     p.xb, p.qb, p.ob, p.ab = xb.data_ptr(), qb.data_ptr(), ob.data_ptr(), ab.data_ptr()
     p.ss, p.part_o, p.part_ml, p.counters = ss.data_ptr(), part_o.data_ptr(), part_ml.data_ptr(), counters.data_ptr()
     if rope is not None:
@@ -1747,7 +1751,7 @@ def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: tor
     p.pos, p.seq, p.block_table = token_pos.data_ptr(), token_seq.data_ptr(), block_table.data_ptr()
     p.status = status_word().data_ptr()
     p.bt_stride, p.n_layers, p.M, p.H, p.F = block_table.stride(0), len(layers), rows, H, F
-    p.n_q, p.n_kv, p.D, p.window, p.vocab = n_q, n_kv, head_dim, int(window), w_head.shape[0]
+    p.n_q, p.n_kv, p.D, p.window = n_q, n_kv, head_dim, int(window)
     p.eps, p.scale = float(eps), float(scale)
     f = _fn("decode_layers", "stratum_decode_layers", [c_void_p, c_int, c_void_p])
     _check(f(ctypes.addressof(p), blocks, _stream()), "decode_layers")

@@ -95,8 +95,8 @@ def test_window_and_rows_alone(model):
 
 
 def test_steps_it_leaves_alone(model):
-    """Rows whose logits nobody wants, and more rows than sixteen, run part by part; a step launched from the host gives a
-    replayed one's bits."""
+    """Some rows' logits only; more rows than sixteen run part by part; a step launched from the host gives a replayed one's
+    bits."""
     from stratum_b200 import StepEntry
     path, cfg, w = model
     llm = _stratum(path, 4096)
@@ -115,6 +115,34 @@ def test_steps_it_leaves_alone(model):
     replayed = _decode(llm, a, [t[19] for t in toks[:2]])
     launched = llm.engine.step([StepEntry(s, [t[19]], [0]) for s, t in zip(b, toks)]).cpu().numpy()
     assert np.array_equal(replayed, launched)
+
+
+def test_the_cache_does_not_follow_from_the_wanted_rows(model):
+    """Whose logits a caller asks for changes neither a step's keys and values nor the logits it gives."""
+    from stratum_b200 import StepEntry
+    path, cfg, _ = model
+    llm = _stratum(path, 4096)
+    rng = np.random.default_rng(4)
+    toks = [rand_tokens(rng, n + 2, cfg["vocab_size"]) for n in (70, 19, 130)]
+    group = llm.engine.cache.groups[0]
+    left = []
+    for wants in ([[0], [0], [0]], [[], [0], []], [[], [], []]):
+        slots = _fill(llm, [t[:-2] for t in toks])
+        got = llm.engine.step([StepEntry(s, [t[-2]], w) for s, t, w in zip(slots, toks, wants)])
+        assert got.shape == (sum(map(len, wants)), cfg["vocab_size"])
+        pages = [llm.engine.cache.page_table_rows([s], 0)[0] for s in slots]
+        kv = [(group.k[:, p, :, (len(t) - 2) % 64].cpu(), group.v[:, p, :, (len(t) - 2) % 64].cpu())
+              for p, t in zip([row[-1] for row in pages], toks)]
+        nxt = _decode(llm, slots, [t[-1] for t in toks])
+        left.append((got.cpu(), kv, nxt))
+        for s in slots:
+            llm.release(s)
+    full = left[0][0]
+    assert torch.equal(left[1][0], full[1:2])
+    for _, kv, nxt in left[1:]:
+        for (k0, v0), (k1, v1) in zip(left[0][1], kv):
+            assert torch.equal(k0, k1) and torch.equal(v0, v1)
+        assert np.array_equal(left[0][2], nxt)
 
 
 def test_a_model_goes_with_its_last_reference(model):
