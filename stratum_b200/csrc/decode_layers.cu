@@ -34,6 +34,8 @@
 #include "mma_common.cuh"
 #include "tc_common.cuh"
 
+#define STRATUM_ERR_RESIDENT (-6)     // the blocks cannot all be resident: nothing was launched
+
 #define DL_WARPS 8                    // that compute; one more fills the ring (of a group of four: registers are dealt by fours)
 #define DL_COMPUTE (DL_WARPS * 32)
 #define DL_THREADS (DL_COMPUTE + 128)
@@ -754,6 +756,14 @@ static int launch_decode_layers(const DlParams& P, int blocks, cudaStream_t stre
   const int smem = (int)sizeof(DlSmem);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
+  // the blocks meet, so all of them must be resident: where the device or this context cannot hold them the caller runs
+  // the step another way
+  int dev = 0, cooperative = 0, sms = 0, per_sm = 0;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
+  if ((e = cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev)) != cudaSuccess) return (int)e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, DL_THREADS, smem)) != cudaSuccess) return (int)e;
+  if (!cooperative || per_sm * sms < blocks) return STRATUM_ERR_RESIDENT;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(DL_THREADS);
@@ -764,7 +774,12 @@ static int launch_decode_layers(const DlParams& P, int blocks, cudaStream_t stre
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, kern, P);
+  e = cudaLaunchKernelEx(&cfg, kern, P);
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+    cudaGetLastError();                          // (nothing ran; the error is this launch's alone)
+    return STRATUM_ERR_RESIDENT;
+  }
+  return (int)e;
 }
 
 // Bytes of DlParams, for callers that mirror it.

@@ -147,7 +147,10 @@ class Model:
         if step.all_single:
             plan = self.resident_steps()
             if plan is not None and plan.takes(step):
-                return plan.run(self, x, step, cache)
+                logits = plan.run(self, x, step, cache)
+                if logits is not None:
+                    return logits
+                self._resident = None             # refused once, before anything is captured: this model runs part by part
         carry = None                  # rows a layer's last product prepared for the next layer's first norm
         for stop, entry in enumerate(self.schedule):
             layer = self.layers[entry.layer]

@@ -74,8 +74,9 @@ class ResidentSteps:
         width = next(iter(step.block_tables.values())).stride(0)
         return K.decode_layers_takes(step.n_tokens, self.att.n_kv_heads, width, step.token_ids.device)
 
-    def run(self, model, x: torch.Tensor, step, cache) -> torch.Tensor:
-        """Float32 logits of the wanted rows of a step that `takes` accepted; x: the embedded tokens."""
+    def run(self, model, x: torch.Tensor, step, cache) -> Optional[torch.Tensor]:
+        """Float32 logits of the wanted rows of a step that `takes` accepted; x: the embedded tokens.  None where the launch was
+        refused because not all of its blocks can be resident (x is as it was)."""
         m, att = model, self.att
         gains = [m.layers[e.layer].part("mixer_norm").gain for e in m.schedule] + [m.final_norm.gain]
         layers, table = [], None
@@ -88,9 +89,10 @@ class ResidentSteps:
                            layer.part("feed_forward_norm").gain, gains[i + 1], view.k, view.v))
         n_want = step.want_rows.numel()
         logits = torch.empty((step.n_tokens, m.vocab), dtype=torch.float32, device=x.device) if n_want else None
-        K.decode_layers(x, layers, gains[0], m.head.proj.weight, logits,
-                        None if self.rot is None else step.rotation_table(self.rot), step.token_pos, step.token_seq, table,
-                        att.n_heads, att.n_kv_heads, att.head_dim, att.window, att.scale, m.final_norm.eps)
+        if not K.decode_layers(x, layers, gains[0], m.head.proj.weight, logits,
+                               None if self.rot is None else step.rotation_table(self.rot), step.token_pos, step.token_seq,
+                               table, att.n_heads, att.n_kv_heads, att.head_dim, att.window, att.scale, m.final_norm.eps):
+            return None
         if logits is None:
             return torch.empty((0, m.vocab), dtype=torch.float32, device=x.device)
         if step.host and step.host.get("want_all"):

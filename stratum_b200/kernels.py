@@ -17,7 +17,8 @@ from .csrc import build
 
 DT_F32, DT_BF16 = 0, 1
 _STATUS = {-1: "unsupported dtype", -2: "unsupported shape", -3: "misaligned pointer or stride",
-           -4: "size beyond the kernel's limit", -5: "device-side wait ran out"}
+           -4: "size beyond the kernel's limit", -5: "device-side wait ran out",
+           -6: "the launch's blocks cannot all be resident"}
 
 
 class KernelError(RuntimeError):
@@ -1658,7 +1659,7 @@ def attention_stream(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
 
 
 # ------------------------------------------------------------------ a decode step's layers as one kernel
-DECODE_LAYERS_MAX, DECODE_LAYERS_MAX_ROWS = 96, 16
+DECODE_LAYERS_MAX, DECODE_LAYERS_MAX_ROWS, DECODE_LAYERS_MAX_BLOCKS = 96, 16, 160
 
 
 class _DecodeLayer(ctypes.Structure):
@@ -1681,9 +1682,9 @@ def sm_count(device) -> int:
 
 def decode_layers_sizes_ok(H: int, F: int, vocab: int, n_q: int, n_kv: int, head_dim: int, device) -> bool:
     """Whether the resident kernel takes a model of these sizes: k in 128s, rows of x of the products over H and over the heads
-    in registers (4,096), two tiles of the stream and two rows of every matrix a block."""
+    in registers (4,096), two tiles of the stream and two rows of every matrix a block, a block per SM."""
     blocks, KO = sm_count(device), n_q * head_dim
-    return (head_dim in (64, 128) and n_q // n_kv <= 8 and H % 128 == 0 and F % 128 == 0 and KO % 128 == 0 and H <= 4096
+    return (blocks <= DECODE_LAYERS_MAX_BLOCKS and head_dim in (64, 128) and n_q // n_kv <= 8 and H % 128 == 0 and F % 128 == 0 and KO % 128 == 0 and H <= 4096
             and KO <= 4096 and (H // 2 + blocks - 1) // blocks <= 16 and H >= 2 * blocks and F >= blocks
             and vocab % 2 == 0 and vocab >= 2 * blocks and KO + 2 * n_kv * head_dim >= 2 * blocks)
 
@@ -1697,11 +1698,12 @@ def decode_layers_takes(rows: int, n_kv: int, table_width: int, device) -> bool:
 def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: torch.Tensor, logits: Optional[torch.Tensor],
                   rope: Optional[torch.Tensor], token_pos: torch.Tensor, token_seq: torch.Tensor,
                   block_table: torch.Tensor, n_q: int, n_kv: int, head_dim: int, window: int, scale: float,
-                  eps: float) -> None:
+                  eps: float) -> bool:
     """All layers of a dense decoder and its head for a step of one new token per sequence, in one kernel that stays on
     every SM: x float32 [rows, H] (embedded), layers a list of (w_qkv, w_o, w_gate_up, w_down, gain of the feed-forward's
     norm, gain of the norm behind the layer, k_cache, v_cache), logits float32 [rows, vocab] (None: no head).  Weights bfloat16, gate and up
-    rows alternating, rotated pairs neighbours; rope: (cos, sin) [rows, pairs, 2] or None.  At most 16 rows."""
+    rows alternating, rotated pairs neighbours; rope: (cos, sin) [rows, pairs, 2] or None.  At most 16 rows.
+    False where the device or the context cannot hold one block per SM at a time: nothing was launched."""
     H, rows = x.shape[1], x.shape[0]
     _need(x, "x", torch.float32); _need(gain_first, "gain_first", torch.float32)
     _need(w_head, "w_head", torch.bfloat16)
@@ -1754,7 +1756,11 @@ def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: tor
     p.n_q, p.n_kv, p.D, p.window = n_q, n_kv, head_dim, int(window)
     p.eps, p.scale = float(eps), float(scale)
     f = _fn("decode_layers", "stratum_decode_layers", [c_void_p, c_int, c_void_p])
-    _check(f(ctypes.addressof(p), blocks, _stream()), "decode_layers")
+    status = f(ctypes.addressof(p), blocks, _stream())
+    if status == -6:
+        return False
+    _check(status, "decode_layers")
+    return True
 
 
 # ------------------------------------------------------------------ sampling

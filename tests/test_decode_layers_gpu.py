@@ -162,6 +162,31 @@ def test_a_model_goes_with_its_last_reference(model):
         gc.enable()
 
 
+def test_a_launch_that_is_refused(model, monkeypatch):
+    """Where the blocks cannot all be resident the step runs part by part, launched and replayed, with the same bits as a model
+    that never took the kernel."""
+    from stratum_b200 import StepEntry
+    from stratum_b200 import kernels as K
+    path, cfg, _ = model
+    rng = np.random.default_rng(6)
+    toks = [rand_tokens(rng, n + 2, cfg["vocab_size"]) for n in (33, 5)]
+    asked, real, out = [], K._fn, []
+    for refused in (True, False):
+        llm = _stratum(path, 1024)
+        if refused:
+            monkeypatch.setattr(K, "_fn", lambda lib, name, types: (lambda *a: asked.append(name) or -6)
+                                if name == "stratum_decode_layers" else real(lib, name, types))
+        else:
+            monkeypatch.setattr(K, "_fn", real)
+            llm.model._resident, llm.model._resident_asked = None, True
+        slots = _fill(llm, [t[:-2] for t in toks])
+        first = llm.engine.step([StepEntry(s, [t[-2]], [0]) for s, t in zip(slots, toks)]).cpu().numpy()
+        out.append((first, _decode(llm, slots, [t[-1] for t in toks])))
+    assert asked == ["stratum_decode_layers"]             # asked once, and not inside a capture
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
 def test_sizes_it_refuses():
     """The launcher refuses what its shares and registers do not hold; the plan asks the same questions."""
     from stratum_b200 import kernels as K

@@ -150,3 +150,11 @@ def test_shared_memory_is_opted_into_at_every_launch():
     for path in sources:
         with open(path) as f:
             assert not re.search(r"static\b[^;{}]*=[^;{}]*cudaFuncSetAttribute", f.read()), path
+
+
+def test_resident_steps_ask_for_a_block_per_sm(monkeypatch):
+    """What the resident kernel's launcher refuses its plan refuses too: devices of more SMs than its tables hold."""
+    from stratum_b200 import kernels as K
+    for sms, takes in ((132, True), (148, True), (160, True), (161, False), (192, False)):
+        monkeypatch.setattr(K, "sm_count", lambda device, n=sms: n)
+        assert K.decode_layers_sizes_ok(4096, 14336, 128256, 32, 8, 128, None) == takes
