@@ -146,11 +146,9 @@ class Model:
                 self.position.add_to_embedding(step.embedded, step)
         if step.all_single:
             plan = self.resident_steps()
-            if plan is not None and plan.takes(step):
-                logits = plan.run(self, x, step, cache)
-                if logits is not None:
-                    return logits
-                self._resident = None             # refused once, before anything is captured: this model runs part by part
+            logits = plan.run(self, x, step, cache) if plan is not None and not plan.refused else None
+            if logits is not None:
+                return logits
         carry = None                  # rows a layer's last product prepared for the next layer's first norm
         for stop, entry in enumerate(self.schedule):
             layer = self.layers[entry.layer]

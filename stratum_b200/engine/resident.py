@@ -7,7 +7,7 @@ does not take, runs part by part.
 """
 from __future__ import annotations
 
-from typing import Optional
+from typing import NamedTuple, Optional
 
 import torch
 
@@ -16,8 +16,10 @@ from ..cache.pages import PAGE_TOKENS
 from ..parts.attention import GQAAttention
 from ..parts.block import PreNormResidual
 from ..parts.embedding import LinearHead
+from ..parts.linear import Linear
 from ..parts.mlp import SwiGLU
 from ..parts.norm import RMSNorm
+from ..parts.rope import RotaryTable
 
 
 # Models of fewer layers run part by part: the kernel's set-up (lists of pages, the ring's first filling, the head's tiles) is a
@@ -27,71 +29,97 @@ from ..parts.norm import RMSNorm
 MIN_LAYERS = 4
 
 
-class ResidentSteps:
-    """The plan of one model: which of its steps the kernel takes, and how it is called.  (It does not hold the model, which
-    holds it: a model's weights go when the last reference to it goes.)"""
+class Decoder(NamedTuple):
+    """A model's parts as the kernel takes them."""
+    att: GQAAttention                 # any layer's: the sizes, window, scale and rotation that all have
+    rot: Optional[RotaryTable]
+    stops: list                       # of every stop of the schedule: (mixer_norm, mixer, feed_forward_norm, feed_forward)
 
-    def __init__(self, model):
-        self.att = model.layers[model.schedule[0].layer].part("mixer")
-        self.rot = self.att.position.rotary() if self.att.position is not None else None
+
+def _is(part, kind) -> bool:
+    """Exactly that part, run as it was written (not a subclass, no `forward` of the object's own)."""
+    return type(part) is kind and "forward" not in vars(part)
+
+
+def _plain(linear) -> bool:
+    return type(linear) is Linear and linear.bias is None
+
+
+class ResidentSteps:
+    """Which of a model's steps the kernel takes, and how it is called.  Nothing of the model is kept: its parts are looked at
+    anew at every step that is not replayed, as the part-by-part path does."""
+
+    refused = False
 
     @classmethod
     def of(cls, model) -> Optional["ResidentSteps"]:
-        """The plan, or None where the model is not made of the parts the kernel knows, in sizes it takes."""
+        """None where the model is not made of the parts the kernel knows, in sizes it takes."""
+        return cls() if cls.describe(model) is not None else None
+
+    @staticmethod
+    def describe(model) -> Optional[Decoder]:
         rt = model.runtime
         if rt is None or rt.dtype != torch.bfloat16 or rt.device.type != "cuda" or PAGE_TOKENS != 64:
             return None
-        if type(model.final_norm) is not RMSNorm or type(model.head) is not LinearHead or model.spec.keep_embedded:
+        if not _is(model.final_norm, RMSNorm) or not _is(model.head, LinearHead) or model.spec.keep_embedded:
             return None
         if any(e.cache_of is not None for e in model.schedule) or not MIN_LAYERS <= len(model.schedule) <= K.DECODE_LAYERS_MAX:
             return None
-        eps, shapes = model.final_norm.eps, set()
+        eps, shapes, stops = model.final_norm.eps, set(), []
         for e in model.schedule:
             layer = model.layers[e.layer]
             norm_a, att = layer.part("mixer_norm"), layer.part("mixer")
             norm_b, ff = layer.part("feed_forward_norm"), layer.part("feed_forward")
-            if (type(layer.arrangement) is not PreNormResidual or type(norm_a) is not RMSNorm or type(norm_b) is not RMSNorm
-                    or type(att) is not GQAAttention or type(ff) is not SwiGLU):
+            if not (_is(layer.arrangement, PreNormResidual) and _is(norm_a, RMSNorm) and _is(norm_b, RMSNorm)
+                    and _is(att, GQAAttention) and _is(ff, SwiGLU)):
                 return None
             if norm_a.eps != eps or norm_b.eps != eps or att.bias or att.q_norm is not None or att.k_norm is not None:
                 return None
             if ff.bias or ff.act != K.ACT_NONE or att.hidden != model.hidden:
                 return None
+            if not (_plain(att.qkv) and _plain(att.o) and _plain(ff.gate_up) and _plain(ff.down)):
+                return None
             rot = att.position.rotary() if att.position is not None else None
             shapes.add((att.n_heads, att.n_kv_heads, att.head_dim, att.window, att.scale, ff.intermediate,
                         None if rot is None else rot.key))
-        if len(shapes) != 1:
+            stops.append((norm_a, att, norm_b, ff))
+        if len(shapes) != 1 or not _plain(model.head.proj):
             return None
-        ok = K.decode_layers_sizes_ok(model.hidden, ff.intermediate, model.vocab, att.n_heads, att.n_kv_heads, att.head_dim,
-                                      rt.device)
-        return cls(model) if ok else None
+        if not K.decode_layers_sizes_ok(model.hidden, ff.intermediate, model.vocab, att.n_heads, att.n_kv_heads, att.head_dim,
+                                        rt.device):
+            return None
+        return Decoder(att, rot, stops)
 
-    def takes(self, step) -> bool:
+    @staticmethod
+    def takes(decoder: Decoder, step) -> bool:
+        """Whether the kernel takes this step of a model it knows."""
+        width = next(iter(step.block_tables.values())).stride(0)
+        return K.decode_layers_takes(step.n_tokens, decoder.att.n_kv_heads, width, step.token_ids.device)
+
+    def run(self, model, x: torch.Tensor, step, cache) -> Optional[torch.Tensor]:
+        """Float32 logits of the step's wanted rows; x: the embedded tokens.  None where the step is not one the kernel takes, or
+        the launch was refused because not all of its blocks can be resident (`refused` is then set); x is as it was."""
         # (not by whose logits are wanted: what a step leaves in the cache does not depend on that)
         if not (step.all_single and 0 < step.n_tokens <= K.DECODE_LAYERS_MAX_ROWS and step.n_seqs == step.n_tokens
                 and len(step.block_tables) == 1):
-            return False
-        width = next(iter(step.block_tables.values())).stride(0)
-        return K.decode_layers_takes(step.n_tokens, self.att.n_kv_heads, width, step.token_ids.device)
-
-    def run(self, model, x: torch.Tensor, step, cache) -> Optional[torch.Tensor]:
-        """Float32 logits of the wanted rows of a step that `takes` accepted; x: the embedded tokens.  None where the launch was
-        refused because not all of its blocks can be resident (x is as it was)."""
-        m, att = model, self.att
-        gains = [m.layers[e.layer].part("mixer_norm").gain for e in m.schedule] + [m.final_norm.gain]
+            return None
+        d = self.describe(model)
+        if d is None or not self.takes(d, step):
+            return None
+        m, att = model, d.att
+        gains = [stop[0].gain for stop in d.stops] + [m.final_norm.gain]
         layers, table = [], None
-        for i, e in enumerate(m.schedule):
-            layer = m.layers[e.layer]
-            mix, ff = layer.part("mixer"), layer.part("feed_forward")
+        for i, (_, mix, norm_b, ff) in enumerate(d.stops):
             view = cache.layer_view(i, True, step.block_tables)
             table = view.block_table
-            layers.append((mix.qkv.weight, mix.o.weight, ff.gate_up.weight, ff.down.weight,
-                           layer.part("feed_forward_norm").gain, gains[i + 1], view.k, view.v))
+            layers.append((mix.qkv.weight, mix.o.weight, ff.gate_up.weight, ff.down.weight, norm_b.gain, gains[i + 1],
+                           view.k, view.v))
         n_want = step.want_rows.numel()
         logits = torch.empty((step.n_tokens, m.vocab), dtype=torch.float32, device=x.device) if n_want else None
         if not K.decode_layers(x, layers, gains[0], m.head.proj.weight, logits,
-                               None if self.rot is None else step.rotation_table(self.rot), step.token_pos, step.token_seq,
+                               None if d.rot is None else step.rotation_table(d.rot), step.token_pos, step.token_seq,
                                table, att.n_heads, att.n_kv_heads, att.head_dim, att.window, att.scale, m.final_norm.eps):
+            self.refused = True                            # (before anything is captured: a first launch warms up)
             return None
         if logits is None:
             return torch.empty((0, m.vocab), dtype=torch.float32, device=x.device)

@@ -187,6 +187,37 @@ def test_a_launch_that_is_refused(model, monkeypatch):
         assert np.array_equal(a, b)
 
 
+EDITS = {
+    "one layer's window": lambda m: setattr(m.layers[2].part("mixer"), "window", 24),
+    "one layer's scale": lambda m: setattr(m.layers[1].part("mixer"), "scale", 0.02),
+    "every layer's scale": lambda m: [setattr(la.part("mixer"), "scale", 0.02) for la in m.layers],
+    "one layer's eps": lambda m: setattr(m.layers[3].part("feed_forward_norm"), "eps", 0.5),
+    "a part's own forward": lambda m: setattr(m.layers[0].part("feed_forward"), "forward", lambda xn, x, step, emit=None: None),
+    "an output bias": lambda m: setattr(m.layers[0].part("mixer").o, "bias", torch.ones(m.hidden, device="cuda")),
+}
+
+
+@pytest.mark.parametrize("edit", sorted(EDITS))
+def test_parts_edited_after_the_first_step(model, edit):
+    """A step that is launched runs the parts as they are then, not as they were when the model's first step ran."""
+    from stratum_b200 import StepEntry
+    path, cfg, _ = model
+    rng = np.random.default_rng(8)
+    toks = [rand_tokens(rng, n + 3, cfg["vocab_size"]) for n in (90, 41)]
+    out = []
+    for on in (True, False):
+        llm = _stratum(path, 1024)
+        if not on:
+            llm.model._resident, llm.model._resident_asked = None, True
+        slots = _fill(llm, [t[:-3] for t in toks])
+        step = lambda i: llm.engine.step([StepEntry(s, [t[i]], [0]) for s, t in zip(slots, toks)]).cpu().numpy()   # noqa: E731
+        before = step(-3)
+        EDITS[edit](llm.model)
+        out.append((before, step(-2), step(-1)))
+    for a, b in zip(*out):
+        assert_close(a, b, "bfloat16", edit)
+
+
 def test_sizes_it_refuses():
     """The launcher refuses what its shares and registers do not hold; the plan asks the same questions."""
     from stratum_b200 import kernels as K
