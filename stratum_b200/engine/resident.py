@@ -41,8 +41,13 @@ def _is(part, kind) -> bool:
     return type(part) is kind and "forward" not in vars(part)
 
 
+def _copies(t) -> bool:
+    """Whether the kernel's 16-byte copies can read it (the parts have kernels for what they cannot)."""
+    return t.is_contiguous() and t.data_ptr() % 16 == 0
+
+
 def _plain(linear) -> bool:
-    return type(linear) is Linear and linear.bias is None
+    return type(linear) is Linear and linear.bias is None and _copies(linear.weight)
 
 
 class ResidentSteps:
@@ -77,13 +82,14 @@ class ResidentSteps:
                 return None
             if ff.bias or ff.act != K.ACT_NONE or att.hidden != model.hidden:
                 return None
-            if not (_plain(att.qkv) and _plain(att.o) and _plain(ff.gate_up) and _plain(ff.down)):
+            if not (_plain(att.qkv) and _plain(att.o) and _plain(ff.gate_up) and _plain(ff.down)
+                    and _copies(norm_a.gain) and _copies(norm_b.gain)):
                 return None
             rot = att.position.rotary() if att.position is not None else None
             shapes.add((att.n_heads, att.n_kv_heads, att.head_dim, att.window, att.scale, ff.intermediate,
                         None if rot is None else rot.key))
             stops.append((norm_a, att, norm_b, ff))
-        if len(shapes) != 1 or not _plain(model.head.proj):
+        if len(shapes) != 1 or not _plain(model.head.proj) or not _copies(model.final_norm.gain):
             return None
         if not K.decode_layers_sizes_ok(model.hidden, ff.intermediate, model.vocab, att.n_heads, att.n_kv_heads, att.head_dim,
                                         rt.device):

@@ -218,6 +218,27 @@ def test_parts_edited_after_the_first_step(model, edit):
         assert_close(a, b, "bfloat16", edit)
 
 
+def _moved(t):
+    """The same values, one element behind a 16-byte boundary."""
+    out = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view(t.shape)
+    return out.copy_(t)
+
+
+@pytest.mark.parametrize("which", ["output projection", "down projection", "head", "a norm's gain", "last gain"])
+def test_weights_that_no_16_byte_copy_can_read(model, which):
+    """A model bound to such tensors runs part by part; nothing is refused."""
+    path, cfg, w = model
+    llm = _stratum(path, 1024)
+    m, layer = llm.model, llm.model.layers[1]
+    owner, name = {"output projection": (layer.part("mixer").o, "weight"), "down projection": (layer.part("feed_forward").down, "weight"),
+                   "head": (m.head.proj, "weight"), "a norm's gain": (layer.part("feed_forward_norm"), "gain"),
+                   "last gain": (m.final_norm, "gain")}[which]
+    setattr(owner, name, _moved(getattr(owner, name)))
+    t = rand_tokens(np.random.default_rng(9), 40, cfg["vocab_size"])
+    slots = _fill(llm, [t[:-1]])
+    assert_close(_decode(llm, slots, t[-1:]), plain_logits(cfg, w, t)[-1:], "bfloat16", which)
+
+
 def test_sizes_it_refuses():
     """The launcher refuses what its shares and registers do not hold; the plan asks the same questions."""
     from stratum_b200 import kernels as K
