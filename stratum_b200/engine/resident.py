@@ -98,9 +98,11 @@ class ResidentSteps:
 
     @staticmethod
     def takes(decoder: Decoder, step) -> bool:
-        """Whether the kernel takes this step of a model it knows."""
-        width = next(iter(step.block_tables.values())).stride(0)
-        return K.decode_layers_takes(step.n_tokens, decoder.att.n_kv_heads, width, step.token_ids.device)
+        """Whether the kernel takes this step of a model it knows.  Asked of the sizes that a replay of the step has, so that a
+        step takes the same way, and gives the same bits, replayed or launched."""
+        from .graphs import padded_rows, width_bucket
+        rows, width = padded_rows(step.n_tokens), width_bucket(next(iter(step.block_tables.values())).stride(0))
+        return K.decode_layers_takes(rows, decoder.att.n_kv_heads, width, step.token_ids.device)
 
     def run(self, model, x: torch.Tensor, step, cache) -> Optional[torch.Tensor]:
         """Float32 logits of the step's wanted rows; x: the embedded tokens.  None where the step is not one the kernel takes, or

@@ -158,3 +158,29 @@ def test_resident_steps_ask_for_a_block_per_sm(monkeypatch):
     for sms, takes in ((132, True), (148, True), (160, True), (161, False), (192, False)):
         monkeypatch.setattr(K, "sm_count", lambda device, n=sms: n)
         assert K.decode_layers_sizes_ok(4096, 14336, 128256, 32, 8, 128, None) == takes
+
+
+def _step_of(rows, width):
+    tables = {0: torch.zeros(rows, width, dtype=torch.int32)}
+    return types.SimpleNamespace(n_tokens=rows, block_tables=tables, token_ids=torch.zeros(rows, dtype=torch.int32))
+
+
+def test_resident_steps_go_the_same_way_launched_and_replayed(monkeypatch):
+    """The rule sees a launched step's own rows and pages and a replay's padded ones: it must not tell them apart, up to the
+    kernel's limit on pages (1,007 a block) and beyond it."""
+    from stratum_b200 import kernels as K
+    from stratum_b200.engine.graphs import padded_rows, width_bucket
+    from stratum_b200.engine.resident import ResidentSteps
+    monkeypatch.setattr(K, "sm_count", lambda device: 148)
+    seen = set()
+    for heads in ((32, 8, 128), (32, 32, 128), (32, 8, 64), (16, 16, 64)):
+        att = types.SimpleNamespace(n_heads=heads[0], n_kv_heads=heads[1], head_dim=heads[2], hidden=4096)
+        decoder = types.SimpleNamespace(att=att)
+        for rows in range(1, 17):
+            for width in (1, 3, 8, 9, 16, 17, 257, 291, 292, 512, 580, 582, 583, 1000, 1024, 1025):
+                launched = ResidentSteps.takes(decoder, _step_of(rows, width))
+                assert launched == ResidentSteps.takes(decoder, _step_of(padded_rows(rows), width_bucket(width)))
+                # what it takes, the launcher takes
+                assert not launched or K.decode_layers_takes(rows, heads[1], width, None)
+                seen.add(launched)
+    assert seen == {True, False}
