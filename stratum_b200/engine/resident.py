@@ -25,8 +25,36 @@ from ..parts.rope import RotaryTable
 # Models of fewer layers run part by part: the kernel's set-up (lists of pages, the ring's first filling, the head's tiles) is a
 # large share of so short a step.  A step in us, parts / kernel, behind 200 tokens with a vocabulary of 2,048, at one, two and
 # four layers: width 512, 8 rows 29 / 33, 47 / 49, 86 / 82; 1 row 36 / 33, 64 / 49, 117 / 82; width 4,096 (8B shape), 8 rows
-# 122 / 112, 218 / 194, 409 / 361.
+# 122 / 112, 218 / 194, 409 / 361: wide models would gain with fewer layers too, but they have more.
 MIN_LAYERS = 4
+WHOLE_PAGES = 8                       # pages of a (sequence, kv head) pair up to which the kernel leaves it to one block
+
+
+def pays(rows: int, width: int, n_kv: int, head_dim: int, hidden: int, heads_width: int, blocks: int) -> bool:
+    """Whether a step is shorter in the kernel than part by part; `width`: pages it may read of a sequence.  Both were
+    measured as replayed steps of 16 layers (us, parts / kernel), 14 shapes behind 200 to 32,000 keys.
+
+    Up to 8 rows, short sequences (no pair is cut): always (Llama-3.2-1B shape, 1 and 8 rows behind 500 keys 862 / 667 and
+    934 / 720; 8B 1,713 / 1,494 and 1,754 / 1,563; width 768, 12 layers, 8 rows 322 / 292).
+    9 to 16 rows, a second accumulator and twice the rows of x a phase: up to a width of 3,072 (16 rows behind 500: 1B
+    989 / 909, 3,072 wide 1,309 / 1,206, but 7B 1,880 / 1,970 and 8B behind 200 1,772 / 1,825), and cut pairs only up to 16
+    pages of 8 kv heads or more (behind 1,000: 1B 1,059 / 1,032, four kv heads 927 / 950; behind 8,000: 1B 1,604 / 1,615).
+    Up to 8 rows, cut pairs: the block that merges a pair reads its pieces four at a time, behind an atomic (5 to 8 us a layer),
+    and what that is taken from must be there.
+    * Narrow models have too little to stream in the meantime: width 768, 12 layers, 8 rows behind 2,500 417 / 452; width
+      1,024, 8 rows behind 8,000 816 / 857; 2,048 wide (1B) 1,261 / 1,128.
+    * Few kv heads make many pieces of a pair: up to one a page, and to all blocks over the kv heads.  1 row: one kv head of
+      128 behind 1,000 (16 pieces) 1,013 / 685, behind 8,000 (125) 1,122 / 1,849; four kv heads behind 8,000 (32) 875 / 892;
+      eight (18) 928 / 858.  From four rows on 37 pieces are still covered: four kv heads, 4 rows behind 8,000 907 / 802.
+    * Heads of 64 in quarter pages draw less than attention_stream.cu's whole pages: 32 kv heads, 8 rows, 111 pages a block
+      (behind 2,500) 1,258 / 1,132, 221 (behind 8,000) 2,087 / 2,124; 8 kv heads, 8 rows behind 32,000 2,185 / 2,209."""
+    if rows > 8:
+        return max(hidden, heads_width) <= 3072 and width <= (16 if n_kv >= 8 else WHOLE_PAGES)
+    if width <= WHOLE_PAGES:
+        return True
+    if hidden < 2048 or min(width, blocks // n_kv) > (40 if rows >= 4 else 20):
+        return False
+    return head_dim != 64 or rows * n_kv * width <= 111 * blocks
 
 
 class Decoder(NamedTuple):
@@ -102,7 +130,10 @@ class ResidentSteps:
         step takes the same way, and gives the same bits, replayed or launched."""
         from .graphs import padded_rows, width_bucket
         rows, width = padded_rows(step.n_tokens), width_bucket(next(iter(step.block_tables.values())).stride(0))
-        return K.decode_layers_takes(rows, decoder.att.n_kv_heads, width, step.token_ids.device)
+        att, device = decoder.att, step.token_ids.device
+        seen = min(width, att.window // PAGE_TOKENS + 2) if att.window > 0 else width
+        return (K.decode_layers_takes(rows, att.n_kv_heads, width, device)
+                and pays(rows, seen, att.n_kv_heads, att.head_dim, att.hidden, att.n_heads * att.head_dim, K.sm_count(device)))
 
     def run(self, model, x: torch.Tensor, step, cache) -> Optional[torch.Tensor]:
         """Float32 logits of the step's wanted rows; x: the embedded tokens.  None where the step is not one the kernel takes, or

@@ -26,6 +26,13 @@ BATCHES = [(30,), (1,), (64, 63, 65), (16, 17, 128, 15, 1, 2, 127, 300), (700, 5
            (9, 64, 200, 31, 32, 33, 70, 129, 4), tuple(range(3, 51, 3))]
 
 
+@pytest.fixture(autouse=True)
+def wherever_it_can(monkeypatch):
+    """These tests are of the kernel: it takes every step it can run, not only those that are shorter in it."""
+    from stratum_b200.engine import resident
+    monkeypatch.setattr(resident, "pays", lambda *a: True)
+
+
 @pytest.fixture(scope="module", params=sorted(MODELS))
 def model(request, tmp_path_factory):
     path = make_model_dir(str(tmp_path_factory.mktemp("resident")), MODELS[request.param], seed=3, dtype="bfloat16")

@@ -174,7 +174,7 @@ def test_resident_steps_go_the_same_way_launched_and_replayed(monkeypatch):
     monkeypatch.setattr(K, "sm_count", lambda device: 148)
     seen = set()
     for heads in ((32, 8, 128), (32, 32, 128), (32, 8, 64), (16, 16, 64)):
-        att = types.SimpleNamespace(n_heads=heads[0], n_kv_heads=heads[1], head_dim=heads[2], hidden=4096)
+        att = types.SimpleNamespace(n_heads=heads[0], n_kv_heads=heads[1], head_dim=heads[2], hidden=4096, window=0)
         decoder = types.SimpleNamespace(att=att)
         for rows in range(1, 17):
             for width in (1, 3, 8, 9, 16, 17, 257, 291, 292, 512, 580, 582, 583, 1000, 1024, 1025):
@@ -184,3 +184,44 @@ def test_resident_steps_go_the_same_way_launched_and_replayed(monkeypatch):
                 assert not launched or K.decode_layers_takes(rows, heads[1], width, None)
                 seen.add(launched)
     assert seen == {True, False}
+
+
+# (rows, pages of the table, kv heads, head size, width, heads * size): what was measured on 148 SMs, us part by part / resident
+MEASURED_STEPS = [
+    ((1, 4, 8, 64, 2048, 2048), True),        # 856 / 639
+    ((8, 16, 8, 64, 2048, 2048), True),       # 965 / 810
+    ((8, 128, 8, 64, 2048, 2048), True),      # 1,261 / 1,128
+    ((8, 512, 8, 64, 2048, 2048), False),     # 2,185 / 2,209
+    ((16, 4, 8, 64, 2048, 2048), True),       # 968 / 908
+    ((16, 16, 8, 64, 2048, 2048), True),      # 1,059 / 1,032
+    ((16, 512, 8, 64, 2048, 2048), False),    # 3,465 / 3,608
+    ((8, 64, 8, 128, 4096, 4096), True),      # 1,902 / 1,773
+    ((8, 512, 8, 128, 4096, 4096), True),     # 4,048 / 3,918
+    ((16, 4, 8, 128, 4096, 4096), False),     # 1,772 / 1,825
+    ((16, 64, 8, 128, 4096, 4096), False),    # 2,137 / 2,187
+    ((8, 128, 32, 128, 4096, 4096), True),    # 3,805 / 3,660
+    ((16, 8, 32, 128, 4096, 4096), False),    # 1,880 / 1,970
+    ((8, 64, 32, 64, 2048, 2048), True),      # 1,258 / 1,132
+    ((8, 512, 32, 64, 2048, 2048), False),    # 5,754 / 6,466
+    ((1, 128, 4, 64, 2048, 2048), False),     # 875 / 892
+    ((4, 128, 4, 64, 2048, 2048), True),      # 907 / 802
+    ((1, 16, 1, 128, 2048, 1024), True),      # 1,013 / 685
+    ((1, 128, 1, 128, 2048, 1024), False),    # 1,122 / 1,849
+    ((4, 128, 1, 128, 2048, 1024), False),    # 881 / 1,087
+    ((2, 128, 2, 128, 1536, 1536), False),    # 926 / 1,145
+    ((8, 64, 12, 64, 768, 768), False),       # 417 / 452
+    ((8, 8, 12, 64, 768, 768), True),         # 322 / 292
+    ((8, 16, 2, 64, 512, 512), False),        # 106 / 119
+    ((1, 512, 2, 64, 512, 512), False),       # 157 / 221
+]
+
+
+@pytest.mark.parametrize("sizes,pays", MEASURED_STEPS, ids=lambda v: str(v))
+def test_resident_steps_where_they_are_shorter(monkeypatch, sizes, pays):
+    from stratum_b200 import kernels as K
+    from stratum_b200.engine.resident import ResidentSteps
+    monkeypatch.setattr(K, "sm_count", lambda device: 148)
+    rows, width, n_kv, head_dim, hidden, heads_width = sizes
+    att = types.SimpleNamespace(n_heads=heads_width // head_dim, n_kv_heads=n_kv, head_dim=head_dim, hidden=hidden,
+                                window=0)
+    assert ResidentSteps.takes(types.SimpleNamespace(att=att), _step_of(rows, width)) == pays
