@@ -8,6 +8,8 @@ there is no CPU or library-op fallback.
 from __future__ import annotations
 
 import ctypes
+import threading
+from collections import OrderedDict
 from ctypes import c_float, c_int, c_size_t, c_uint64, c_void_p
 from typing import Optional, Tuple
 
@@ -1820,18 +1822,21 @@ def _sample_scratch_for(rows: int, device):
     at zero, a mark for the one-block kernel)."""
     global _sample_scratch
     if _sample_scratch is None or _sample_scratch[6].numel() < rows:
-        n = max(rows, 64)
-        f32, i32 = torch.float32, torch.int32
-        _sample_scratch = (torch.empty(n * SAMPLE_SPLITS, dtype=f32, device=device),
-                           torch.empty(n * SAMPLE_SPLITS, dtype=i32, device=device),
-                           torch.empty(n * SAMPLE_SPLITS * 8, dtype=f32, device=device),
-                           torch.empty(n * SAMPLE_SPLITS, dtype=i32, device=device),
-                           torch.empty(n * SAMPLE_SPLITS * SAMPLE_LIST, dtype=f32, device=device),
-                           torch.empty(n * SAMPLE_SPLITS * SAMPLE_LIST, dtype=i32, device=device),
-                           torch.zeros(n, dtype=i32, device=device),
-                           torch.zeros(n, dtype=i32, device=device))
+        _sample_scratch = _new_sample_scratch(max(rows, 64), device)
         scratch_regrown()
     return _sample_scratch
+
+
+def _new_sample_scratch(n: int, device):
+    f32, i32 = torch.float32, torch.int32
+    return (torch.empty(n * SAMPLE_SPLITS, dtype=f32, device=device),
+            torch.empty(n * SAMPLE_SPLITS, dtype=i32, device=device),
+            torch.empty(n * SAMPLE_SPLITS * 8, dtype=f32, device=device),
+            torch.empty(n * SAMPLE_SPLITS, dtype=i32, device=device),
+            torch.empty(n * SAMPLE_SPLITS * SAMPLE_LIST, dtype=f32, device=device),
+            torch.empty(n * SAMPLE_SPLITS * SAMPLE_LIST, dtype=i32, device=device),
+            torch.zeros(n, dtype=i32, device=device),
+            torch.zeros(n, dtype=i32, device=device))
 
 
 def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor, top_p: torch.Tensor,
@@ -1854,6 +1859,24 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
 
 
 SAMPLE_GIVEN_MAX = 256
+SAMPLE_GIVEN_STREAMS = 8
+_given_scratch: "OrderedDict[tuple, tuple]" = OrderedDict()      # (device, stream) -> scratch, the latest used last
+_given_lock = threading.Lock()
+
+
+def _given_scratch_for(rows: int, device):
+    """The same for picks that nothing holds up: one for each stream that picks, since picks on two streams may run at the same
+    time.  (A scratch is allocated on the stream it serves, so one that is given back is not reused ahead of the picks on
+    that stream.)"""
+    key = (device.index, _stream().value)
+    with _given_lock:
+        s = _given_scratch.pop(key, None)
+        if s is None or s[6].numel() < rows:
+            s = _new_sample_scratch(max(rows, 64), device)
+        _given_scratch[key] = s
+        if len(_given_scratch) > SAMPLE_GIVEN_STREAMS:
+            _given_scratch.popitem(last=False)
+    return s
 
 
 def sample_given(logits: torch.Tensor, temperature: float, top_k: int, top_p: float, uniforms, ids: torch.Tensor,
@@ -1864,7 +1887,7 @@ def sample_given(logits: torch.Tensor, temperature: float, top_k: int, top_p: fl
     n = logits.shape[0]
     if len(uniforms) != n or n > SAMPLE_GIVEN_MAX:
         raise KernelError(f"sample_given: one uniform per row, at most {SAMPLE_GIVEN_MAX}")
-    scratch = (None,) * 8 if one_block_per_row else _sample_scratch_for(n, logits.device)
+    scratch = (None,) * 8 if one_block_per_row else _given_scratch_for(n, logits.device)
     f = _fn("sampling", "stratum_sample_given",
             [c_void_p, c_int, c_int, c_int, c_float, c_int, c_float, c_void_p, c_void_p, c_void_p] + [c_void_p] * 9)
     _check(f(logits.data_ptr(), logits.stride(0), n, logits.shape[1], temperature, top_k, top_p, (c_float * n)(*uniforms),

@@ -226,3 +226,48 @@ def test_numbers_given_with_the_launch(vocab, n, temp, top_k, top_p):
     assert out[0] == out[1]
     with pytest.raises(K.KernelError):
         K.sample_given(L, temp, top_k, top_p, us + [0.5], ids, vals)
+
+
+def test_picks_on_two_streams_share_no_scratch(monkeypatch):
+    """Nothing holds a pick up any more, so picks on two streams may run at the same time: the scratch each is launched with
+    (whose counters begin and end at zero) is its stream's own, and is kept for the stream's next pick.  (Nothing is launched
+    here: the launches' arguments are compared.)"""
+    from stratum_b200 import kernels as K
+    seen = []
+    monkeypatch.setattr(K, "_fn", lambda lib, name, types: lambda *a: seen.append([getattr(p, "value", p) for p in a[10:18]]) or 0)
+    L = torch.zeros((4, 9000), dtype=torch.float32, device="cuda")
+    ids = torch.empty(4, dtype=torch.int32, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(3)] + [torch.cuda.current_stream()]
+    for _ in range(2):
+        for s in streams:
+            with torch.cuda.stream(s):
+                K.sample_given(L, 0.7, 20, 0.9, [0.5] * 4, ids)
+    first, second = seen[:4], seen[4:]
+    assert first == second
+    assert len({p for row in first for p in row}) == 4 * 8 and all(p for row in first for p in row)
+
+
+def test_picks_in_turn_on_two_streams():
+    """Picks that follow one another without a wait, on two streams in turn, are the picks of one stream."""
+    from stratum_b200 import kernels as K
+    rng = np.random.default_rng(5)
+    rows, vocab, turns = 24, 40000, 12
+    L = [_dev(rng.standard_normal((rows, vocab)) * 2.0, torch.float32) for _ in range(2)]
+    us = [float(np.float32(u)) for u in rng.random(rows)]
+
+    def pick(i):
+        ids = torch.empty(rows, dtype=torch.int32, device="cuda")
+        vals = torch.empty(rows, dtype=torch.float32, device="cuda")
+        K.sample_given(L[i], 0.8, 50, 0.95, us, ids, vals)
+        return ids, vals
+
+    want = [tuple(t.tolist() for t in pick(i)) for i in range(2)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(turns):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got.append((i, pick(i)))
+    torch.cuda.synchronize()
+    assert all(tuple(t.tolist() for t in out) == want[i] for i, out in got)
