@@ -1678,6 +1678,21 @@ class _DecodeLayers(ctypes.Structure):
                [("eps", c_float), ("scale", c_float), ("layer", _DecodeLayer * DECODE_LAYERS_MAX)]
 
 
+def _decode_layers_fn():
+    """The launcher, once the struct's two descriptions are seen to agree in size (a field on one side only would shift every
+    pointer behind it)."""
+    global _decode_layers_checked
+    if not _decode_layers_checked:
+        there = _fn("decode_layers", "stratum_decode_layers_params", [])()
+        if there != ctypes.sizeof(_DecodeLayers):
+            raise KernelError(f"decode_layers: its parameters are {there} bytes, described here as {ctypes.sizeof(_DecodeLayers)}")
+        _decode_layers_checked = True
+    return _fn("decode_layers", "stratum_decode_layers", [c_void_p, c_int, c_void_p])
+
+
+_decode_layers_checked = False
+
+
 def sm_count(device) -> int:
     return torch.cuda.get_device_properties(device).multi_processor_count
 
@@ -1757,8 +1772,7 @@ def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: tor
     p.bt_stride, p.n_layers, p.M, p.H, p.F = block_table.stride(0), len(layers), rows, H, F
     p.n_q, p.n_kv, p.D, p.window = n_q, n_kv, head_dim, int(window)
     p.eps, p.scale = float(eps), float(scale)
-    f = _fn("decode_layers", "stratum_decode_layers", [c_void_p, c_int, c_void_p])
-    status = f(ctypes.addressof(p), blocks, _stream())
+    status = _decode_layers_fn()(ctypes.addressof(p), blocks, _stream())
     if status == -6:
         return False
     _check(status, "decode_layers")

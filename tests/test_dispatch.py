@@ -225,3 +225,15 @@ def test_resident_steps_where_they_are_shorter(monkeypatch, sizes, pays):
     att = types.SimpleNamespace(n_heads=heads_width // head_dim, n_kv_heads=n_kv, head_dim=head_dim, hidden=hidden,
                                 window=0)
     assert ResidentSteps.takes(types.SimpleNamespace(att=att), _step_of(rows, width)) == pays
+
+
+def test_resident_parameters_are_described_alike(monkeypatch):
+    """The struct and its mirror are of one size, and a launch with another is refused."""
+    import ctypes
+    from stratum_b200 import kernels as K
+    monkeypatch.setattr(K, "_decode_layers_checked", False)
+    assert K._decode_layers_fn() is not None and K._decode_layers_checked
+    monkeypatch.setattr(K, "_decode_layers_checked", False)
+    monkeypatch.setattr(K, "_DecodeLayers", ctypes.c_char * 64)
+    with pytest.raises(K.KernelError):
+        K._decode_layers_fn()
