@@ -50,7 +50,6 @@
 #define DL_MAX_PAGES 1024             // pages a block attends to
 #define DL_WHOLE 8                    // up to this many pages a pair is not cut
 #define DL_STRIDE 20                  // floats from one row of x to the next among the partial sums: no bank conflicts
-#define DL_SPIN_LIMIT (1u << 21)      // polls of half a microsecond: a second
 
 struct DlLayer {
   const bf16 *w_qkv, *w_o, *w_gu, *w_down;
@@ -70,6 +69,7 @@ struct DlParams {
   const int *pos, *seq, *block_table;
   int* status;
   int bt_stride, n_layers, M, H, F, n_q, n_kv, D, n_pairs, window, vocab;
+  unsigned spin_limit;                // polls of a meeting, half a microsecond each
   float eps, scale;
   DlLayer layer[DL_MAX_LAYERS];
 };
@@ -181,8 +181,14 @@ struct DlFeeder {
       ok = matrix(PH_QKV, L.w_qkv) && pages(L) && matrix(PH_O, L.w_o) && matrix(PH_GU, L.w_gu) && matrix(PH_DOWN, L.w_down);
     }
     if (ok) ok = matrix(PH_HEAD, P.w_head);
+    // the block stays until everything that was asked for has landed: until all of it has been taken, or, where the warps that
+    // compute gave up (the last copies may then be on their way still), for a while
+    for (int s = 0; s < DL_STAGES && ok; s++) {
+      ok = free_stage();
+      next();
+    }
     if (!ok)
-      for (int i = 0; i < 2000; i++) __nanosleep(1000);      // copies already under way land
+      for (int i = 0; i < 2000; i++) __nanosleep(1000);
   }
 };
 
@@ -195,7 +201,7 @@ __device__ __forceinline__ void dl_arrive(const DlParams& P) {
 __device__ __forceinline__ bool dl_meet(const DlParams& P, DlSmem& S, unsigned target, int code) {
   if (threadIdx.x == 0) {
     bool ok = false;
-    for (unsigned i = 0; i < DL_SPIN_LIMIT; i++) {
+    for (unsigned i = 0; i < P.spin_limit; i++) {
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(P.counters) : "memory");
       if ((int)(v - target) >= 0) { ok = true; break; }

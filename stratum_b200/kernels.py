@@ -10,7 +10,7 @@ from __future__ import annotations
 import ctypes
 import threading
 from collections import OrderedDict
-from ctypes import c_float, c_int, c_size_t, c_uint64, c_void_p
+from ctypes import c_float, c_int, c_size_t, c_uint32, c_uint64, c_void_p
 from typing import Optional, Tuple
 
 import torch
@@ -1662,6 +1662,7 @@ def attention_stream(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
 
 # ------------------------------------------------------------------ a decode step's layers as one kernel
 DECODE_LAYERS_MAX, DECODE_LAYERS_MAX_ROWS, DECODE_LAYERS_MAX_BLOCKS = 96, 16, 160
+DECODE_LAYERS_SPIN_LIMIT = 1 << 21    # polls of a grid-wide meeting, half a microsecond each: a second
 
 
 class _DecodeLayer(ctypes.Structure):
@@ -1675,7 +1676,7 @@ class _DecodeLayers(ctypes.Structure):
                                         "part_ml", "counters", "rope", "pos", "seq", "block_table", "status")] + \
                [(n, c_int) for n in ("bt_stride", "n_layers", "M", "H", "F", "n_q", "n_kv", "D", "n_pairs", "window",
                                      "vocab")] + \
-               [("eps", c_float), ("scale", c_float), ("layer", _DecodeLayer * DECODE_LAYERS_MAX)]
+               [("spin_limit", c_uint32)] + [("eps", c_float), ("scale", c_float), ("layer", _DecodeLayer * DECODE_LAYERS_MAX)]
 
 
 def _decode_layers_fn():
@@ -1771,7 +1772,7 @@ def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: tor
     p.status = status_word().data_ptr()
     p.bt_stride, p.n_layers, p.M, p.H, p.F = block_table.stride(0), len(layers), rows, H, F
     p.n_q, p.n_kv, p.D, p.window = n_q, n_kv, head_dim, int(window)
-    p.eps, p.scale = float(eps), float(scale)
+    p.eps, p.scale, p.spin_limit = float(eps), float(scale), DECODE_LAYERS_SPIN_LIMIT
     status = _decode_layers_fn()(ctypes.addressof(p), blocks, _stream())
     if status == -6:
         return False
