@@ -42,17 +42,17 @@ def pays(rows: int, width: int, n_kv: int, head_dim: int, hidden: int, heads_wid
     Up to 8 rows, cut pairs: the block that merges a pair reads its pieces four at a time, behind an atomic (5 to 8 us a layer),
     and what that is taken from must be there.
     * Narrow models have too little to stream in the meantime: width 768, 12 layers, 8 rows behind 2,500 417 / 452; width
-      1,024, 8 rows behind 8,000 816 / 857; 2,048 wide (1B) 1,261 / 1,128.
+      1,024 behind 2,500 605 / 593, behind 8,000 816 / 857; 2,048 wide (1B) 1,261 / 1,128.
     * Few kv heads make many pieces of a pair: up to one a page, and to all blocks over the kv heads.  1 row: one kv head of
-      128 behind 1,000 (16 pieces) 1,013 / 685, behind 8,000 (125) 1,122 / 1,849; four kv heads behind 8,000 (32) 875 / 892;
-      eight (18) 928 / 858.  From four rows on 37 pieces are still covered: four kv heads, 4 rows behind 8,000 907 / 802.
+      128 behind 1,000 (16 pieces) 1,013 / 685, behind 8,000 (125) 1,122 / 1,849; four kv heads (up to 37) behind 2,500
+      856 / 753 and 1,567 / 1,372, behind 8,000, the worst, 875 / 892 and 1,590 / 1,579; eight (18) 928 / 858.
     * Heads of 64 in quarter pages draw less than attention_stream.cu's whole pages: 32 kv heads, 8 rows, 111 pages a block
       (behind 2,500) 1,258 / 1,132, 221 (behind 8,000) 2,087 / 2,124; 8 kv heads, 8 rows behind 32,000 2,185 / 2,209."""
     if rows > 8:
         return max(hidden, heads_width) <= 3072 and width <= (16 if n_kv >= 8 else WHOLE_PAGES)
     if width <= WHOLE_PAGES:
         return True
-    if hidden < 2048 or min(width, blocks // n_kv) > (40 if rows >= 4 else 20):
+    if hidden < (1024 if n_kv >= 8 and width <= 64 else 2048) or min(width, blocks // n_kv) > 40:
         return False
     return head_dim != 64 or rows * n_kv * width <= 111 * blocks
 

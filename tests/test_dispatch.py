@@ -203,7 +203,10 @@ MEASURED_STEPS = [
     ((16, 8, 32, 128, 4096, 4096), False),    # 1,880 / 1,970
     ((8, 64, 32, 64, 2048, 2048), True),      # 1,258 / 1,132
     ((8, 512, 32, 64, 2048, 2048), False),    # 5,754 / 6,466
-    ((1, 128, 4, 64, 2048, 2048), False),     # 875 / 892
+    ((1, 64, 4, 64, 2048, 2048), True),       # 856 / 753
+    ((8, 64, 8, 64, 1024, 1024), True),       # 605 / 593
+    ((8, 128, 8, 64, 1024, 1024), False),     # 816 / 857
+    ((8, 16, 2, 128, 1536, 1536), False),     # 4 rows: 829 / 854
     ((4, 128, 4, 64, 2048, 2048), True),      # 907 / 802
     ((1, 16, 1, 128, 2048, 1024), True),      # 1,013 / 685
     ((1, 128, 1, 128, 2048, 1024), False),    # 1,122 / 1,849
