@@ -1662,7 +1662,7 @@ def attention_stream(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
 
 # ------------------------------------------------------------------ a decode step's layers as one kernel
 DECODE_LAYERS_MAX, DECODE_LAYERS_MAX_ROWS, DECODE_LAYERS_MAX_BLOCKS = 96, 16, 160
-DECODE_LAYERS_SPIN_LIMIT = 1 << 21    # polls of a grid-wide meeting, half a microsecond each: a second
+DECODE_LAYERS_ABSENT = 0              # arrivals its meetings wait for in vain (for a test of the bounded wait)
 
 
 class _DecodeLayer(ctypes.Structure):
@@ -1676,7 +1676,7 @@ class _DecodeLayers(ctypes.Structure):
                                         "part_ml", "counters", "rope", "pos", "seq", "block_table", "status")] + \
                [(n, c_int) for n in ("bt_stride", "n_layers", "M", "H", "F", "n_q", "n_kv", "D", "n_pairs", "window",
                                      "vocab")] + \
-               [("spin_limit", c_uint32)] + [("eps", c_float), ("scale", c_float), ("layer", _DecodeLayer * DECODE_LAYERS_MAX)]
+               [("absent", c_uint32)] + [("eps", c_float), ("scale", c_float), ("layer", _DecodeLayer * DECODE_LAYERS_MAX)]
 
 
 def _decode_layers_fn():
@@ -1772,7 +1772,7 @@ def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: tor
     p.status = status_word().data_ptr()
     p.bt_stride, p.n_layers, p.M, p.H, p.F = block_table.stride(0), len(layers), rows, H, F
     p.n_q, p.n_kv, p.D, p.window = n_q, n_kv, head_dim, int(window)
-    p.eps, p.scale, p.spin_limit = float(eps), float(scale), DECODE_LAYERS_SPIN_LIMIT
+    p.eps, p.scale, p.absent = float(eps), float(scale), DECODE_LAYERS_ABSENT
     status = _decode_layers_fn()(ctypes.addressof(p), blocks, _stream())
     if status == -6:
         return False

@@ -247,7 +247,7 @@ def test_weights_that_no_16_byte_copy_can_read(model, which):
 
 
 def test_a_meeting_that_runs_out(model, monkeypatch):
-    """Blocks that may not wait for the others leave at their first meeting: the step ends with an error, no sequence is longer,
+    """Blocks that wait for one more than there are give up after a second: the step ends with an error, no sequence is longer,
     and the next step is right."""
     from stratum_b200 import StepEntry
     from stratum_b200 import kernels as K
@@ -255,13 +255,11 @@ def test_a_meeting_that_runs_out(model, monkeypatch):
     llm = _stratum(path, 1024)
     t = rand_tokens(np.random.default_rng(10), 151, cfg["vocab_size"])
     slots = _fill(llm, [t[:150]])
-    limit = K.DECODE_LAYERS_SPIN_LIMIT
-    monkeypatch.setattr(K, "DECODE_LAYERS_SPIN_LIMIT", 0)
-    for _ in range(2):
-        with pytest.raises(K.KernelError, match="waiting for the others"):
-            llm.engine.step([StepEntry(slots[0], t[150:], [0])])
-        assert llm.engine.length(slots[0]) == 150
-    monkeypatch.setattr(K, "DECODE_LAYERS_SPIN_LIMIT", limit)
+    monkeypatch.setattr(K, "DECODE_LAYERS_ABSENT", 1)
+    with pytest.raises(K.KernelError, match="resident decode step"):
+        llm.engine.step([StepEntry(slots[0], t[150:], [0])])
+    assert llm.engine.length(slots[0]) == 150
+    monkeypatch.setattr(K, "DECODE_LAYERS_ABSENT", 0)
     got = llm.engine.step([StepEntry(slots[0], t[150:], [0])]).cpu().numpy()
     assert_close(got, plain_logits(cfg, w, t)[-1:], "bfloat16", "the step behind one that gave up")
 
