@@ -27,10 +27,20 @@ BATCHES = [(30,), (1,), (64, 63, 65), (16, 17, 128, 15, 1, 2, 127, 300), (700, 5
 
 
 @pytest.fixture(autouse=True)
-def wherever_it_can(monkeypatch):
-    """These tests are of the kernel: it takes every step it can run, not only those that are shorter in it."""
+def launches(monkeypatch):
+    """These tests are of the kernel: it takes every step it can run, not only those that are shorter in it.  The rows of its
+    launches, in their order (a step that is captured is launched twice: once to warm up)."""
+    from stratum_b200 import kernels as K
     from stratum_b200.engine import resident
     monkeypatch.setattr(resident, "pays", lambda *a: True)
+    seen, real = [], K.decode_layers
+
+    def counted(x, *args):
+        seen.append(x.shape[0])
+        return real(x, *args)
+
+    monkeypatch.setattr(K, "decode_layers", counted)
+    return seen
 
 
 @pytest.fixture(scope="module", params=sorted(MODELS))
@@ -58,21 +68,24 @@ def _decode(llm, slots, tokens):
 
 
 @pytest.mark.parametrize("lens", BATCHES, ids=lambda b: f"{len(b)} rows, {max(b)}")
-def test_against_the_oracle(model, lens):
+def test_against_the_oracle(model, lens, launches):
     path, cfg, w = model
     llm = _stratum(path, sum(n + 128 for n in lens))
     rng = np.random.default_rng(len(lens))
     steps = 3
     toks = [rand_tokens(rng, n + steps, cfg["vocab_size"]) for n in lens]
     slots = _fill(llm, [t[:n] for t, n in zip(toks, lens)])
+    del launches[:]                                          # (a prompt of one token is a step of its own)
     got = [_decode(llm, slots, [t[n + i] for t, n in zip(toks, lens)]) for i in range(steps)]
     assert llm.model.resident_steps() is not None
+    rows = len(lens) if len(lens) <= 8 else 16
+    assert launches and set(launches) == {rows}
     for j, (t, n) in enumerate(zip(toks, lens)):
         ref = plain_logits(cfg, w, t)
         assert_close(np.stack([g[j] for g in got]), ref[n:], "bfloat16", f"row {j} of {n} tokens")
 
 
-def test_window_and_rows_alone(model):
+def test_window_and_rows_alone(model, launches):
     """A sliding window (the same attribute both paths read) against the part-by-part path, and a row's bits in another batch."""
     path, cfg, _ = model
     lens = [200, 64, 10, 130]
@@ -88,6 +101,7 @@ def test_window_and_rows_alone(model):
             layer.part("mixer").window = 70
         out.append(_decode(llm, slots, [t[-1] for t in toks]))
         assert (llm.model.resident_steps() is not None) == on
+        assert launches == [4, 4]                            # (none by the second model)
     assert_close(out[0], out[1], "bfloat16", "window")
     llm = _stratum(path, 2048)
     alone = []
@@ -99,9 +113,17 @@ def test_window_and_rows_alone(model):
     both = _decode(llm, slots, [t[-1] for t in toks])
     # (pairs of up to eight pages are never cut, so the order of every sum is the same)
     assert np.array_equal(both, np.stack(alone))
+    # and among twelve rows, of which the kernel takes sixteen with a second accumulator
+    more = _fill(llm, [rand_tokens(rng, n, cfg["vocab_size"]) for n in (1, 63, 90, 17, 40, 128, 33, 7)])
+    for s in slots:
+        llm.release(s)
+    slots = _fill(llm, [t[:-1] for t in toks])
+    order = more[:5] + slots + more[5:]
+    twelve = _decode(llm, order, [9] * 5 + [t[-1] for t in toks] + [9] * 3)
+    assert launches[-1] == 16 and np.array_equal(twelve[5:9], np.stack(alone))
 
 
-def test_steps_it_leaves_alone(model):
+def test_steps_it_leaves_alone(model, launches):
     """Some rows' logits only; more rows than sixteen run part by part; a step launched from the host gives a replayed one's
     bits."""
     from stratum_b200 import StepEntry
@@ -113,15 +135,19 @@ def test_steps_it_leaves_alone(model):
     slots = _fill(llm, [t[:19] for t in toks])
     got = llm.engine.step([StepEntry(s, [t[19]], [0] if i != 1 else []) for i, (s, t) in enumerate(zip(slots, toks[:3]))])
     assert_close(got.cpu().numpy(), np.stack([ref[0][19], ref[2][19]]), "bfloat16", "wanted rows")
+    assert launches == [3]
     _decode(llm, slots[3:], [t[19] for t in toks[3:]])
+    assert set(launches[1:]) == {16}
+    del launches[:]
     got = _decode(llm, slots, [t[20] for t in toks])
+    assert not launches
     assert_close(got[:3], np.stack([r[20] for r in ref]), "bfloat16", "seventeen rows")
     for s in slots:
         llm.release(s)
     a, b = _fill(llm, [t[:19] for t in toks[:2]]), _fill(llm, [t[:19] for t in toks[:2]])
     replayed = _decode(llm, a, [t[19] for t in toks[:2]])
     launched = llm.engine.step([StepEntry(s, [t[19]], [0]) for s, t in zip(b, toks)]).cpu().numpy()
-    assert np.array_equal(replayed, launched)
+    assert np.array_equal(replayed, launched) and launches == [2, 2, 2]
 
 
 def test_the_cache_does_not_follow_from_the_wanted_rows(model):
@@ -192,6 +218,94 @@ def test_a_launch_that_is_refused(model, monkeypatch):
     assert asked == ["stratum_decode_layers"]             # asked once, and not inside a capture
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+# The widths the kernel serves, four layers of them.  On 148 SMs: two tiles of the stream a block (widths above 2,368), three and
+# four chunks of k, 5 to 9 tiles of the head (several groups of the partial sums' tiles), a k of the down product that ends
+# inside a chunk, 3, 4 and 1 query heads a kv head.
+WIDE = {
+    "8B": dict(BASE, hidden_size=4096, intermediate_size=14336, num_attention_heads=32, num_key_value_heads=8, head_dim=128,
+               vocab_size=10000, max_position_embeddings=16384),
+    "7B": dict(BASE, hidden_size=4096, intermediate_size=11008, num_attention_heads=32, num_key_value_heads=32, head_dim=128,
+               vocab_size=3000, max_position_embeddings=16384),
+    "3B": dict(BASE, hidden_size=3072, intermediate_size=8192, num_attention_heads=24, num_key_value_heads=8, head_dim=128,
+               vocab_size=12800, max_position_embeddings=16384),
+    "1B": dict(BASE, hidden_size=2048, intermediate_size=8192, num_attention_heads=32, num_key_value_heads=8, head_dim=64,
+               vocab_size=20000, max_position_embeddings=16384),
+}
+# rows; lengths.  The long ones: a block's share of 3 to 60 pages, cuts at odd pages, blocks that end one cut pair, take whole
+# ones and begin another, pairs of eight and nine pages beside each other
+WIDE_BATCHES = [(201,), (3700,) * 8, (64, 63, 65, 1, 512, 513, 577, 130, 30), tuple(range(20, 500, 30)),
+                (9000,), (3705, 1000, 64, 2050, 513), (520, 8000, 449, 2, 575, 1090, 300, 5)]
+
+
+@pytest.fixture(scope="module", params=sorted(WIDE))
+def wide(request):
+    from stratum_b200 import Stratum
+    from stratum_b200.config import LlamaConfig
+    llm = Stratum.from_random(LlamaConfig.from_dict(WIDE[request.param]), seed=5, max_tokens=64000, max_seqs=40)
+    for layer in llm.model.layers:         # the attention's share of the stream, the mean of many values, is not to drown beside
+        layer.part("feed_forward").down.weight.mul_(0.1)       # the feed-forward's: a page left out would not be seen then
+    return llm
+
+
+@pytest.mark.parametrize("lens", WIDE_BATCHES, ids=lambda b: f"{len(b)} rows, {max(b)}")
+def test_served_widths(wide, lens, launches):
+    """Logits of two steps, and the keys and values they leave, against the part-by-part path over the same prompts."""
+    from stratum_b200 import StepEntry
+    llm, cache = wide, wide.engine.cache
+    rng = np.random.default_rng(len(lens) + max(lens))
+    toks = [rand_tokens(rng, n + 2, llm.model.vocab) for n in lens]
+    out, plan = [], llm.model.resident_steps()
+    assert plan is not None
+    for on in (True, False):
+        llm.model._resident = plan if on else None
+        del launches[:]
+        slots = _fill(llm, [t[:-2] for t in toks])
+        del launches[:]                                      # (a prompt of one token is a step of its own)
+        logits = [llm.engine.step([StepEntry(s, [t[i]], [0]) for s, t in zip(slots, toks)]).cpu().numpy() for i in (-2, -1)]
+        assert launches == ([len(lens)] * 2 if on else [])
+        group, rows = cache.groups[0], cache.page_table_rows(slots, 0)
+        kv = [[x[:, row[n // 64], :, n % 64].float().cpu().numpy() for row, n in zip(rows, lens)] for x in (group.k, group.v)]
+        out.append((logits, kv))
+        for s in slots:
+            llm.release(s)
+    llm.model._resident = plan
+    # Both round the same rows to bfloat16, each sum in its own order: 0.003 to 0.007 of the row's largest logit.  One page left
+    # out of the longest row moves it by 0.3 (201 keys) to 0.009 (8,000).
+    for a, b in zip(out[0][0], out[1][0]):
+        for j in range(len(lens)):
+            err = np.max(np.abs(a[j] - b[j])) / np.max(np.abs(b[j]))
+            assert err <= 0.01, f"row {j} of {lens[j]} tokens: {err:.4f}"
+    for what, a, b in zip("kv", out[0][1], out[1][1]):
+        assert_close(np.stack(a), np.stack(b), "bfloat16", what)
+
+
+def test_steps_on_two_streams(launches):
+    """Two models stepped on streams of their own, nothing between the steps that waits: each gives what it gives alone.  (All
+    blocks of a launch are resident together or none are, so the two kernels take turns.)"""
+    from stratum_b200 import StepEntry, Stratum
+    from stratum_b200 import kernels as K
+    from stratum_b200.config import LlamaConfig
+    rng = np.random.default_rng(12)
+    streams, steps, want = [torch.cuda.Stream() for _ in range(2)], [], []
+    for seed in (1, 2):
+        llm = Stratum.from_random(LlamaConfig.from_dict(WIDE["8B"]), seed=seed, max_tokens=2048, max_seqs=4)
+        slots = _fill(llm, [rand_tokens(rng, n, 10000) for n in (300, 700)])
+        llm.engine.cache.reserve(slots, [1, 1])
+        batch = llm.engine.build_batch([StepEntry(s, [7], [0]) for s in slots])
+        want.append(llm.model.forward(batch, llm.engine.cache))
+        steps.append((llm, batch))
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(12):
+        for i, (llm, batch) in enumerate(steps):
+            with torch.cuda.stream(streams[i]):
+                got.append((i, llm.model.forward(batch, llm.engine.cache)))
+    torch.cuda.synchronize()
+    K.check_status()
+    assert len(launches) == 26
+    assert all(torch.equal(logits, want[i]) for i, logits in got)
 
 
 EDITS = {
@@ -265,7 +379,7 @@ def test_a_meeting_that_runs_out(model, monkeypatch):
 
 
 def test_sizes_it_refuses():
-    """The launcher refuses what its shares and registers do not hold; the plan asks the same questions."""
+    """The plan refuses what the launcher's shares and registers do not hold."""
     from stratum_b200 import kernels as K
     dev = torch.device("cuda")
     ok = dict(H=2048, F=8192, vocab=128256, n_q=32, n_kv=8, head_dim=64, device=dev)

@@ -240,3 +240,43 @@ def test_resident_parameters_are_described_alike(monkeypatch):
     monkeypatch.setattr(K, "_DecodeLayers", ctypes.c_char * 64)
     with pytest.raises(K.KernelError):
         K._decode_layers_fn()
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="the parameters name no memory: only a machine that cannot launch asks this")
+def test_resident_launcher_refuses():
+    """The launcher's own questions, one broken at a time, before it calls CUDA at all."""
+    import ctypes
+    from stratum_b200 import kernels as K
+    SHAPE, ALIGN, LIMIT = -2, -3, -4
+    f = K._decode_layers_fn()
+
+    def status(blocks=148, layer=None, **over):
+        p = K._DecodeLayers()
+        for name, kind in p._fields_:
+            if kind is ctypes.c_void_p:
+                setattr(p, name, 4096)
+        for n in range(4):
+            for name, _ in K._DecodeLayer._fields_:
+                setattr(p.layer[n], name, 4096)
+        sizes = dict(bt_stride=64, n_layers=4, M=8, H=4096, F=14336, n_q=32, n_kv=8, D=128, n_pairs=64, vocab=128256,
+                     eps=1e-5, scale=0.1)
+        for name, v in dict(sizes, **over).items():
+            setattr(p, name, v)
+        for name, v in (layer or {}).items():
+            setattr(p.layer[3], name, v)
+        return f(ctypes.addressof(p), blocks, None)
+
+    assert status() > 0                                    # (no device: a CUDA error, not a refusal)
+    assert status(M=0) == 0
+    for want, cases in ((LIMIT, [dict(M=17), dict(n_layers=97), dict(blocks=161), dict(bt_stride=0), dict(bt_stride=3000), dict(M=1, bt_stride=20000)]),
+                        (SHAPE, [dict(n_layers=0), dict(blocks=0), dict(D=80), dict(n_kv=5), dict(n_kv=0), dict(n_q=72), dict(n_pairs=65),
+                                 dict(n_pairs=-1), dict(H=4160), dict(H=8192), dict(H=256), dict(F=14400), dict(F=128), dict(n_q=64),
+                                 dict(vocab=1001), dict(vocab=200), dict(vocab=-2), dict(x=None), dict(w_head=None),
+                                 dict(logits=None), dict(rope=None), dict(status=None), dict(counters=None), dict(part_ml=None),
+                                 dict(layer=dict(w_o=None)), dict(layer=dict(v=None))]),
+                        (ALIGN, [dict(x=4104), dict(w_head=4098), dict(rope=4104), dict(layer=dict(k=4098)),
+                                 dict(layer=dict(gain_next=4100))])):
+        for c in cases:
+            assert status(**c) == want, c
+    assert status(vocab=0, w_head=None, logits=None) > 0   # a step that wants no logits
+    assert status(n_pairs=0, rope=None) > 0

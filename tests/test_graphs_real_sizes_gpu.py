@@ -1,6 +1,7 @@
 """Decode steps as replayed CUDA graphs at the layer sizes of Llama-3.1-8B, Llama-3.2-1B and Llama-2-7B.
 
-This is the schedule that generation uses by default and that the benchmark times: the stream-K and
+This is the schedule of decode steps that run part by part (models of fewer than four layers, as here, more rows than
+the resident kernel takes, float32): the stream-K and
 cluster forms of the matrix product with their second pass, the TMA-fed decode attention with its late
 launch trigger, padded rows and page tables of a bucketed width, all overlapping through programmatic
 dependent launch.  Every replayed step's logits are compared with the launch-by-launch engine's (the same
