@@ -540,7 +540,8 @@ def main() -> int:
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--batch", type=int, default=8)
     ap.add_argument("--context", type=int, default=4096)
-    ap.add_argument("--layers", type=int, default=0, help="fewer layers than the configuration has (0 = all)")
+    ap.add_argument("--layers", type=int, default=0, help="fewer layers than the configuration has (0 = all; decode steps of fewer than four run part by part "
+                         "where the whole model's run as one resident kernel)")
     ap.add_argument("--no-points", action="store_true", help="skip the batch-1 and batch-64 points")
     ap.add_argument("--decode-only", action="store_true",
                     help="time the decode steps only and print a short line (for profiler runs)")

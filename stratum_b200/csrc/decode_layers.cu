@@ -16,8 +16,8 @@
 //
 // Split.  A block takes an equal share of the rows of every matrix, to a pair of rows, with all of k, so nothing has to be
 // added across blocks; its eight warps cut every 1,024 values of k, and their partial sums meet in shared memory in the order
-// of the warps.  A sum's order follows from k alone: a row gives the same bits in any batch.  Weights are the A operand of
-// mma.sync.m16n8k16 (16 rows a tile), rows of x the B operand, straight from L2 into registers, k visited in an order of its
+// of the warps.  A product's order of sums follows from k alone: its rows give the same bits in any batch.  Weights are the A
+// operand of mma.sync.m16n8k16 (16 rows a tile), rows of x the B operand, straight from L2 into registers, k visited in an order of its
 // own that both share (a lane takes the 8 contiguous values 8t..8t+7 of 32, see gemm_skinny.cu).  tcgen05 would add its trips
 // through tensor memory to every phase, and mma.sync has three times the rate at which the weights arrive.
 //
@@ -25,9 +25,10 @@
 // the product behind the norm multiplies its sums by 1 / sqrt(sum / size + eps).  The stream itself stays in the registers of
 // the threads that add to it, in float32.
 //
-// Attention.  The pages of all (sequence, kv head) pairs form one list, cut evenly over the blocks (pairs of few pages are not
-// cut: a row's bits then do not depend on its batch); four warps take 16 keys of a page each, two pages at a time; scores and
-// values as in attention_mma.cu (keys along M).
+// Attention.  The pages of all (sequence, kv head) pairs form one list, cut evenly over the blocks.  Pairs of few pages are not
+// cut, so a row of up to 512 visible keys gives the same bits in any batch of the kernel's; where a longer one is cut follows
+// from the batch.  Four warps take 16 keys of a page each, two pages at a time; scores and values as in attention_mma.cu (keys
+// along M).
 // A pair seen by several blocks is merged by whichever of them comes last, in the order of its keys.  The new token's key and
 // value, which another block may have written a phase ago, do not come through the ring: one warp takes them from L2.
 #include "common.cuh"
