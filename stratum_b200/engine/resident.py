@@ -66,16 +66,7 @@ class Decoder(NamedTuple):
 
 def _is(part, kind) -> bool:
     """Exactly that part, run as it was written (not a subclass, no `forward` of the object's own)."""
-    return type(part) is kind and "forward" not in vars(part)
-
-
-def _copies(t) -> bool:
-    """Whether the kernel's 16-byte copies can read it (the parts have kernels for what they cannot)."""
-    return t.is_contiguous() and t.data_ptr() % 16 == 0
-
-
-def _plain(linear) -> bool:
-    return type(linear) is Linear and linear.bias is None and _copies(linear.weight)
+    return type(part) is kind and "forward" not in part.__dict__
 
 
 class ResidentSteps:
@@ -94,11 +85,14 @@ class ResidentSteps:
         rt = model.runtime
         if rt is None or rt.dtype != torch.bfloat16 or rt.device.type != "cuda" or PAGE_TOKENS != 64:
             return None
-        if not _is(model.final_norm, RMSNorm) or not _is(model.head, LinearHead) or model.spec.keep_embedded:
+        head = model.head
+        if not _is(model.final_norm, RMSNorm) or not _is(head, LinearHead) or model.spec.keep_embedded:
+            return None
+        if type(head.proj) is not Linear or head.proj.bias is not None:
             return None
         if any(e.cache_of is not None for e in model.schedule) or not MIN_LAYERS <= len(model.schedule) <= K.DECODE_LAYERS_MAX:
             return None
-        eps, shapes, stops = model.final_norm.eps, set(), []
+        eps, hidden, sizes, stops = model.final_norm.eps, model.hidden, None, []
         for e in model.schedule:
             layer = model.layers[e.layer]
             norm_a, att = layer.part("mixer_norm"), layer.part("mixer")
@@ -108,18 +102,22 @@ class ResidentSteps:
                 return None
             if norm_a.eps != eps or norm_b.eps != eps or att.bias or att.q_norm is not None or att.k_norm is not None:
                 return None
-            if ff.bias or ff.act != K.ACT_NONE or att.hidden != model.hidden:
+            if ff.bias or ff.act != K.ACT_NONE or att.hidden != hidden:
                 return None
-            if not (_plain(att.qkv) and _plain(att.o) and _plain(ff.gate_up) and _plain(ff.down)
-                    and _copies(norm_a.gain) and _copies(norm_b.gain)):
+            qkv, o, gate_up, down = att.qkv, att.o, ff.gate_up, ff.down
+            if not type(qkv) is type(o) is type(gate_up) is type(down) is Linear:
+                return None
+            if not qkv.bias is o.bias is gate_up.bias is down.bias is None:
                 return None
             rot = att.position.rotary() if att.position is not None else None
-            shapes.add((att.n_heads, att.n_kv_heads, att.head_dim, att.window, att.scale, ff.intermediate,
-                        None if rot is None else rot.key))
+            these = (att.n_heads, att.n_kv_heads, att.head_dim, att.window, att.scale, ff.intermediate,
+                     None if rot is None else rot.key)
+            if sizes is None:
+                sizes = these
+            elif these != sizes:
+                return None
             stops.append((norm_a, att, norm_b, ff))
-        if len(shapes) != 1 or not _plain(model.head.proj) or not _copies(model.final_norm.gain):
-            return None
-        if not K.decode_layers_sizes_ok(model.hidden, ff.intermediate, model.vocab, att.n_heads, att.n_kv_heads, att.head_dim,
+        if not K.decode_layers_sizes_ok(hidden, ff.intermediate, model.vocab, att.n_heads, att.n_kv_heads, att.head_dim,
                                         rt.device):
             return None
         return Decoder(att, rot, stops)
@@ -137,7 +135,8 @@ class ResidentSteps:
 
     def run(self, model, x: torch.Tensor, step, cache) -> Optional[torch.Tensor]:
         """Float32 logits of the step's wanted rows; x: the embedded tokens.  None where the step is not one the kernel takes, or
-        the launch was refused because not all of its blocks can be resident (`refused` is then set); x is as it was."""
+        the launch was refused, because not all of its blocks can be resident or its copies cannot read a weight (`refused` is then
+        set); x is as it was."""
         # (not by whose logits are wanted: what a step leaves in the cache does not depend on that)
         if not (step.all_single and 0 < step.n_tokens <= K.DECODE_LAYERS_MAX_ROWS and step.n_seqs == step.n_tokens
                 and len(step.block_tables) == 1):

@@ -1721,7 +1721,8 @@ def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: tor
     every SM: x float32 [rows, H] (embedded), layers a list of (w_qkv, w_o, w_gate_up, w_down, gain of the feed-forward's
     norm, gain of the norm behind the layer, k_cache, v_cache), logits float32 [rows, vocab] (None: no head).  Weights bfloat16, gate and up
     rows alternating, rotated pairs neighbours; rope: (cos, sin) [rows, pairs, 2] or None.  At most 16 rows.
-    False where the device or the context cannot hold one block per SM at a time: nothing was launched."""
+    False, and nothing launched, where the device or the context cannot hold one block per SM at a time, or a pointer is not on
+    the 16-byte boundary that the kernel's copies need."""
     H, rows = x.shape[1], x.shape[0]
     _need(x, "x", torch.float32); _need(gain_first, "gain_first", torch.float32)
     _need(w_head, "w_head", torch.bfloat16)
@@ -1737,10 +1738,11 @@ def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: tor
         raise KernelError("decode_layers: the step's description has another number of rows")
     F, KO = layers[0][3].shape[1], n_q * head_dim
     p = _DecodeLayers()
+    s_qkv, s_o, s_gu, s_down, s_page = (KO + 2 * n_kv * head_dim, H), (H, KO), (2 * F, H), (H, F), (n_kv, 64, head_dim)
     for q, (w_qkv, w_o, w_gu, w_down, gain_ff, gain_next, k, v) in zip(p.layer, layers):
-        for t, shape in ((w_qkv, (KO + 2 * n_kv * head_dim, H)), (w_o, (H, KO)), (w_gu, (2 * F, H)), (w_down, (H, F))):
+        for t, shape in ((w_qkv, s_qkv), (w_o, s_o), (w_gu, s_gu), (w_down, s_down)):
             _need(t, "a layer's matrix", torch.bfloat16)
-            if tuple(t.shape) != shape:
+            if t.shape != shape:
                 raise KernelError("decode_layers: a layer's matrix has another shape")
         for t in (gain_ff, gain_next):
             _need(t, "a layer's gain", torch.float32)
@@ -1748,21 +1750,24 @@ def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: tor
                 raise KernelError("decode_layers: a layer's gain has another size")
         for t in (k, v):
             _need(t, "a layer's cache", torch.bfloat16)
-            if tuple(t.shape[1:]) != (n_kv, 64, head_dim):
+            if t.shape[1:] != s_page:
                 raise KernelError("decode_layers: a layer's cache has another shape")
         q.w_qkv, q.w_o, q.w_gu, q.w_down = w_qkv.data_ptr(), w_o.data_ptr(), w_gu.data_ptr(), w_down.data_ptr()
         q.gain_ff, q.gain_next, q.k, q.v = gain_ff.data_ptr(), gain_next.data_ptr(), k.data_ptr(), v.data_ptr()
     blocks, dev = sm_count(x.device), x.device
-    bf = lambda n: torch.empty(rows * n, dtype=torch.bfloat16, device=dev)          # noqa: E731
-    f32 = lambda n: torch.empty(n, dtype=torch.float32, device=dev)                 # noqa: E731
-    xb, qb, ob, ab = bf(H), bf(KO), bf(KO), bf(F)
-    ss, part_o, part_ml = f32(2 * blocks * 16), f32(2 * blocks * 8 * head_dim), f32(2 * blocks * 8 * 2)
+    # one buffer for what the blocks hand one another: bfloat16 rows of x, q, o and a; float32 sums of squares and pieces
+    parts = {"xb": 2 * rows * H, "qb": 2 * rows * KO, "ob": 2 * rows * KO, "ab": 2 * rows * F, "ss": 4 * 2 * blocks * 16,
+             "part_o": 4 * 2 * blocks * 8 * head_dim, "part_ml": 4 * 2 * blocks * 8 * 2}
+    buffer = torch.empty(sum(parts.values()) + 256 * len(parts), dtype=torch.uint8, device=dev)
+    at = buffer.data_ptr()
+    for name, n in parts.items():
+        setattr(p, name, at)
+        at += (n + 255) // 256 * 256
     counters = torch.zeros(1 + rows * n_kv, dtype=torch.int32, device=dev)          # (a step begins with zeros whatever came before)
-    p.x, p.gain_first = x.data_ptr(), gain_first.data_ptr()
+    p.x, p.gain_first, p.w_head = x.data_ptr(), gain_first.data_ptr(), w_head.data_ptr()
     if logits is not None:
-        p.w_head, p.logits, p.vocab = w_head.data_ptr(), logits.data_ptr(), w_head.shape[0]
-    p.xb, p.qb, p.ob, p.ab = xb.data_ptr(), qb.data_ptr(), ob.data_ptr(), ab.data_ptr()
-    p.ss, p.part_o, p.part_ml, p.counters = ss.data_ptr(), part_o.data_ptr(), part_ml.data_ptr(), counters.data_ptr()
+        p.logits, p.vocab = logits.data_ptr(), w_head.shape[0]
+    p.counters = counters.data_ptr()
     if rope is not None:
         _need(rope, "rope", torch.float32)
         if rope.shape[0] != rows:
@@ -1774,7 +1779,7 @@ def decode_layers(x: torch.Tensor, layers, gain_first: torch.Tensor, w_head: tor
     p.n_q, p.n_kv, p.D, p.window = n_q, n_kv, head_dim, int(window)
     p.eps, p.scale, p.absent = float(eps), float(scale), DECODE_LAYERS_ABSENT
     status = _decode_layers_fn()(ctypes.addressof(p), blocks, _stream())
-    if status == -6:
+    if status in (-3, -6):
         return False
     _check(status, "decode_layers")
     return True
